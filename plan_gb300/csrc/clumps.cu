@@ -43,8 +43,7 @@ namespace {
 
 constexpr uint32_t kNone = 0xffffffffu;
 constexpr int kSmallSort = 2048;
-constexpr uint32_t kBigKinematics = 4096;  // larger clumps sum with warp_ordered_sum
-constexpr int kKinTile = 512;
+constexpr uint32_t kBigKinematics = 4096;  // larger clumps sum with ordered_sum_chunk
 
 struct CP {
     double G, shear, Omega;
@@ -171,32 +170,42 @@ __global__ void __launch_bounds__(128) k_kinematics(const uint32_t *list, uint32
     }
 }
 
-// The same sums for clumps of more than kBigKinematics members: the block stages the terms
-// of kKinTile members in shared memory and warp c runs sum c with warp_ordered_sum.
+// The same sums for clumps of more than kBigKinematics members: the block stages the terms of
+// 256 members in shared memory (one member per thread, the next ones on their way meanwhile)
+// and warp c < 7 runs sum c (ordered_sum_chunk).
 __global__ void __launch_bounds__(256) k_kinematics_big(const uint32_t *list, CT ct, Pool P, const double4_32a *pos, const double4_32a *vel,
                                                         int with_hill, double G, double Omega) {
-    __shared__ double term[7][kKinTile];
+    static_assert(kSumChunk == 256, "one member per thread");
+    __shared__ __align__(16) double term[7 * kSumStage];
+    __shared__ uint2 steps[7 * kSumChunk];
     __shared__ double res[7];
     const uint32_t s = list[blockIdx.x];
     const uint32_t o = ct.moff[s], m = ct.mn[s];
     if (m <= kBigKinematics) return;
     const int w = threadIdx.x >> 5;
+    const uint32_t at = sum_slot(threadIdx.x);
     double acc = 0.0;
-    for (uint32_t base = 0; base < m; base += kKinTile) {
-        const uint32_t cnt = min((uint32_t)kKinTile, m - base);
-        for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) {
-            const uint32_t id = P.idx[o + base + i];
-            const double4_32a p = pos[id], v = vel[id];
-            term[0][i] = p.w;
-            term[1][i] = p.x * p.w;
-            term[2][i] = p.y * p.w;
-            term[3][i] = p.z * p.w;
-            term[4][i] = v.x * p.w;
-            term[5][i] = v.y * p.w;
-            term[6][i] = v.z * p.w;
+    double4_32a p = make_double4_32a(0, 0, 0, 0), v = p;
+    auto fetch = [&](uint32_t k) {
+        p = v = make_double4_32a(0, 0, 0, 0);
+        if (k < m) {
+            const uint32_t id = P.idx[o + k];
+            p = pos[id];
+            v = vel[id];
         }
+    };
+    fetch(threadIdx.x);
+    for (uint32_t base = 0; base < m; base += kSumChunk) {
+        term[at] = p.w;
+        term[kSumStage + at] = p.x * p.w;
+        term[2 * kSumStage + at] = p.y * p.w;
+        term[3 * kSumStage + at] = p.z * p.w;
+        term[4 * kSumStage + at] = v.x * p.w;
+        term[5 * kSumStage + at] = v.y * p.w;
+        term[6 * kSumStage + at] = v.z * p.w;
         __syncthreads();
-        if (w < 7) acc = warp_ordered_sum(term[w], cnt, acc);
+        fetch(base + kSumChunk + threadIdx.x);
+        if (w < 7) ordered_sum_chunk(term + w * kSumStage, acc, steps + w * kSumChunk);
         __syncthreads();
     }
     if (w < 7 && (threadIdx.x & 31) == 0) res[w] = acc;

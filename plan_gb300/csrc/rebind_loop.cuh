@@ -23,9 +23,9 @@
 //    applies the reference's FP64 update to the state. Its division is a reciprocal product
 //    with Markstein's correction; the reciprocals of the next masses are taken 32 at a time
 //    off the dependent chain while the accepted particles have equal masses;
-//  * SortParticles: the seven member sums in member order (warp_ordered_sum_window over
-//    per-point products m, m x, ..., m vz formed once per snapshot, 128 terms per step with
-//    the next terms prefetched into registers), the centre of mass and the Hill radius,
+//  * SortParticles: the seven member sums in member order (ordered_sum_chunk over per-point
+//    products m, m x, ..., m vz formed once per snapshot, 256 members at a time, the next
+//    ones staged meanwhile), the centre of mass and the Hill radius,
 //    squared distances, and a stable sort by squared distance (in shared memory up to
 //    kRbSmall members, else a block radix sort on the top 32 bits and an exact fix-up of
 //    equal prefixes). Squared distances order members as distances do, except that two
@@ -689,67 +689,66 @@ __device__ bool rb_sort_particles(const RbArgs &a, uint32_t slot, RbShared &sh, 
     uint32_t *idx = a.P.idx + o;
     double *dist = a.P.dist + o;
     // 1) the seven sums in member order (CalculateKinematicProperties): warp w < 7 runs sum w
-    // over the per-point products, 64 terms per step, from a shared-memory stage that the
-    // other nine warps fill: 256 members at a time (one per loading thread), double-buffered,
-    // the member indices of a chunk read one chunk ahead, so the sums never wait on a gather
-    // from memory
+    // over the per-point products from a shared-memory stage that the other nine warps fill:
+    // 256 members at a time (one per loading thread), double-buffered, the products of a chunk
+    // on their way to registers a whole chunk before they are staged, their indices one more
     double acc = 0.0;
     uint32_t its = 0;
     long long tsum = 0;
     {
-        constexpr uint32_t kCh = 256;            // members per chunk
+        constexpr uint32_t kCh = kSumChunk;      // members per chunk
         constexpr uint32_t kLd = kRB - 7 * 32;   // loading threads (warps 7..15)
-        constexpr int kK = 2;                    // terms per lane and step
-        static_assert(2 * 7 * kCh * sizeof(double) <= kRbSmem, "sum stage");
-        static_assert(kCh <= kLd && kCh % (32 * kK) == 0, "sum chunk");
-        double *stg = reinterpret_cast<double *>(sh.buf);  // [2][7][kCh]
-        auto put = [&](double *d, uint32_t k, const double4_32a &p, const double4_32a &v) {
-            d[k] = p.x;
-            d[kCh + k] = p.y;
-            d[2 * kCh + k] = p.z;
-            d[3 * kCh + k] = p.w;
-            d[4 * kCh + k] = v.x;
-            d[5 * kCh + k] = v.y;
-            d[6 * kCh + k] = v.z;
-        };
+        constexpr uint32_t kBuf = 7 * kSumStage; // doubles per buffer
+        static_assert(2 * kBuf * sizeof(double) + 7 * kSumChunk * sizeof(uint2) <= kRbSmem, "sum stage and lists");
+        static_assert(kCh <= kLd, "sum chunk");
+        double *stg = reinterpret_cast<double *>(sh.buf);  // [2][7][kSumStage]
+        uint2 *list = reinterpret_cast<uint2 *>(stg + 2 * kBuf) + (size_t)kSumChunk * (wid < 7 ? wid : 0);
         const uint32_t nch = (m + kCh - 1) / kCh;
-        if ((uint32_t)tid < min(m, kCh)) {  // chunk 0: every thread
-            const uint32_t q = idx[tid];
-            put(stg, (uint32_t)tid, a.tm0[q], a.tm1[q]);
-        }
         const uint32_t k0 = (uint32_t)tid - 7u * 32u;  // loading threads: their member of a chunk
-        uint32_t q0 = 0;                              // and its index in the next chunk
-        if (wid >= 7 && k0 < kCh && kCh + k0 < m) q0 = idx[kCh + k0];
+        const bool loads = wid >= 7 && k0 < kCh;
+        const uint32_t at = sum_slot(k0 < kCh ? k0 : 0u);
+        uint32_t qn = 0;  // a loading thread's member index, one chunk ahead of the products
+        double4_32a p = make_double4_32a(0, 0, 0, 0), v = p;
+        auto fetch = [&](uint32_t g) {  // the products of member g, whose index is in qn; then the next index
+            p = v = make_double4_32a(0, 0, 0, 0);
+            if (g < m) {
+                p = a.tm0[qn];
+                v = a.tm1[qn];
+            }
+            if (g + kCh < m) qn = idx[g + kCh];
+        };
+        auto put = [&](uint32_t b) {
+            double *d = stg + (size_t)b * kBuf + at;
+            d[0] = p.x;
+            d[kSumStage] = p.y;
+            d[2 * kSumStage] = p.z;
+            d[3 * kSumStage] = p.w;
+            d[4 * kSumStage] = v.x;
+            d[5 * kSumStage] = v.y;
+            d[6 * kSumStage] = v.z;
+        };
+        if (loads) {
+            if (k0 < m) qn = idx[k0];
+            fetch(k0);
+            put(0);
+            fetch(kCh + k0);
+        }
         __syncthreads();
         const long long ts = clock64();
         for (uint32_t c = 0; c < nch; ++c) {
             const uint32_t b = c & 1u;
             if (wid < 7) {
-                const double *src = stg + ((size_t)b * 7 + wid) * kCh;
-                const uint32_t cnt = min(kCh, m - c * kCh);
-                for (uint32_t w0 = 0; w0 < cnt; w0 += 32 * kK) {
-                    const uint32_t k = w0 + (uint32_t)lane * kK;
-                    double x[kK];
-                    const double2 v2 = k < cnt ? *reinterpret_cast<const double2 *>(src + k) : make_double2(0.0, 0.0);
-                    x[0] = v2.x;
-                    x[1] = k + 1 < cnt ? v2.y : 0.0;
-                    acc = warp_ordered_sum_window<kK>(x, min(32u * kK, cnt - w0), acc, &its);
-                }
-            } else if (c + 1 < nch && k0 < kCh) {
-                // chunk c + 1 into the other buffer, and the index of chunk c + 2
-                const uint32_t g1 = (c + 1) * kCh, g2 = g1 + kCh;
-                if (g1 + k0 < m) {
-                    const double4_32a p0 = a.tm0[q0], u0 = a.tm1[q0];
-                    q0 = g2 + k0 < m ? idx[g2 + k0] : 0u;
-                    put(stg + (size_t)(b ^ 1u) * 7 * kCh, k0, p0, u0);
-                }
+                ordered_sum_chunk(stg + (size_t)b * kBuf + (size_t)wid * kSumStage, acc, list, &its);
+            } else if (loads && c + 1 < nch) {
+                put(b ^ 1u);
+                fetch((c + 2) * kCh + k0);
             }
             __syncthreads();
         }
         tsum = clock64() - ts;
     }
     if (wid < 7 && lane == 0) sh.tabM[wid] = acc;  // the table is free between calls
-    if (wid < 7 && lane == 0 && stat) {  // each sum: its time and its steps
+    if (wid < 7 && lane == 0 && stat) {  // each sum: its time and the chunks it took term by term
         atomicAdd(&stat[17 + wid], (unsigned long long)its);
         atomicAdd(&stat[24 + wid], (unsigned long long)tsum);
     }
