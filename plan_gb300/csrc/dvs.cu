@@ -1,8 +1,10 @@
 // --Density_Vs_Scale on the GPU: every (cell centre, radius, sub-centre) query of
 // BasicAnalysesWithTree is one thread walking the particle tree with the reference's sheared
 // node tests (dvs.cuh, the same code the CPU tests run on the oracle's tree); the largest
-// count per radius is an atomic maximum. The host sets up the grid with the reference's own
+// count per radius is an atomic maximum, and queries that cannot reach it stop early. The host sets up the grid with the reference's own
 // arithmetic and turns the counts into densities.
+#include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -10,6 +12,7 @@
 #include "dvs.cuh"
 #include "pipeline.h"
 #include "tree_walk.cuh"
+#include "knn_f32.cuh"
 
 namespace plan {
 
@@ -36,16 +39,145 @@ struct DevTreeView {
     }
 };
 
-__global__ void k_dvs(DevTreeView tv, const double *xs, const double *ys, const double *zs, DvsGeom g, uint32_t *maxc, unsigned *err) {
-    const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (tid >= (uint64_t)g.nx * g.ny * g.nz * g.nvar) return;
-    double x, y, z;
+// Query tid in the order they are taken: variant by variant, the largest radius first (the
+// longest walks start first), the cells of a variant side by side (neighbours meet the same nodes).
+__device__ __forceinline__ uint64_t dvs_order(const DvsGeom &g, uint64_t tid) {
+    const uint64_t cells = (uint64_t)g.nx * g.ny * g.nz;
+    const uint32_t v = (uint32_t)(tid / cells);
+    return (tid % cells) * g.nvar + (v < (uint32_t)g.nlev ? g.nlev - 1 - v : v);
+}
+
+// A node's class in FP32, in FP64 where that cannot tell.
+struct NodeClass {
+    const DevTreeView &tv;
+    const FTree &ft;
+    const DvsGeom &g;
+    const DvsGeomF &gf;
+    double c[3];
+    float cf[3];
     int lev;
-    dvs_query(g, xs, ys, zs, tid, x, y, z, lev);
-    bool overflow = false;
-    const uint32_t n = dvs_count(tv, x, y, z, g.radius[lev], g.maxd[lev], g, &overflow);
-    if (overflow) atomicOr(err, (unsigned)kDevErrCapacity);
-    atomicMax(&maxc[lev], n);
+    __device__ int operator()(uint32_t n) const {
+        const float4 h = ft.nhi[n];
+        const float nf[3] = {h.x, h.y, h.z};
+        const int cls = dvs_class_f(cf, nf, h.w, lev, gf);
+        if (cls >= 0) return cls;
+        double nc[3], hw;
+        tv.node(n, nc[0], nc[1], nc[2], hw);
+        return dvs_class(c, nc, hw, g.radius[lev], g.maxd[lev], g);
+    }
+};
+
+// Only the largest count of each radius is wanted, so most queries end without a look at a
+// point: the points of contained nodes bound a query's count from below, those of the met
+// leaves on top bound it from above, and a query whose upper bound does not exceed the largest
+// count known is done. k_dvs<0> finds the largest lower bound over the cell centres (a seed for
+// k_dvs<1>, whose first queries would otherwise have nothing to compare with); k_dvs<1> bounds
+// every query and counts the points of the met leaves, in FP32 with the exact FP64 test where
+// that is too close, for those left, until the bound drops to the largest count.
+//
+// A warp takes one query: its lanes classify up to 32 nodes of a last-in first-out list at a
+// time, append the children of the met ones, and later share the points of the met leaves.
+// Measured with the tree's build, 150,000 particles, 32 cells a side, 1.2 M queries: 12.8 ms. A
+// thread per query took 87 ms (the few thousand node tests and tens of thousands of points of
+// each large ball one at a time), FP64 throughout with every point counted 1,075 ms. What
+// bounds it: the node tests of the large radii, whose bounds are too loose to stop before the
+// points.
+constexpr uint32_t kDvsList = 1024;    // nodes to classify, per warp
+constexpr uint32_t kDvsLeaves = 1024;  // met leaves, per warp
+constexpr int kDvsWarps = 4;
+
+template <int kCount>
+__global__ void __launch_bounds__(32 * kDvsWarps) k_dvs(DevTreeView tv, FTree ft, const double *xs, const double *ys, const double *zs,
+                                                        const __grid_constant__ DvsGeom g, const __grid_constant__ DvsGeomF gf, uint64_t n,
+                                                        unsigned long long *next, uint32_t *maxc, unsigned *err) {
+    __shared__ uint32_t s_list[kDvsWarps][kDvsList], s_leaf[kDvsWarps][kDvsLeaves];
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, below = (1u << lane) - 1u;
+    const unsigned full = 0xffffffffu;
+    uint32_t *list = s_list[w], *leaves = s_leaf[w];
+    for (;;) {
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(next, 1ull);
+        at = __shfl_sync(full, at, 0);
+        if (at >= n) return;
+        double x, y, z;
+        int lev;
+        dvs_query(g, xs, ys, zs, dvs_order(g, at), x, y, z, lev);
+        const NodeClass classify{tv, ft, g, gf, {x, y, z}, {(float)x, (float)y, (float)z}, lev};
+        uint32_t inside = 0, partial = 0;  // of the whole warp, the same in every lane
+        uint32_t top = 1, nleaf = 0;
+        // the listed leaves' points: true when the count cannot exceed the largest known
+        auto count_leaves = [&](bool stop) {
+            const double r = g.radius[lev], rr = r * r;
+            const float rr32 = (float)rr;
+            const float4 qh = make_float4(classify.cf[0], classify.cf[1], classify.cf[2], 0.f);
+            const float4 ql = make_float4((float)(x - (double)qh.x), (float)(y - (double)qh.y), (float)(z - (double)qh.z), 0.f);
+            for (uint32_t k = 0; k < nleaf; ++k) {
+                if (stop && inside + partial <= *(volatile uint32_t *)&maxc[lev]) return;
+                const uint32_t b = tv.begin(leaves[k]), e = tv.end(leaves[k]);
+                uint32_t in = 0;
+                for (uint32_t p = b + lane; p < e; p += 32) {
+                    const float v = f_dr2(qh, ql, ft.phi[p], ft.plo[p]);
+                    if (f_hi(v) < rr32 * (1.f - kRel)) {
+                        ++in;
+                    } else if (!(f_lo(v) > rr32 * (1.f + kRel))) {
+                        double px, py, pz;
+                        tv.point(p, px, py, pz);
+                        const double dx = x - px, dy = y - py, dz = z - pz;
+                        if (dx * dx + dy * dy + dz * dz <= rr) ++in;
+                    }
+                }
+                inside += __reduce_add_sync(full, in);
+                partial -= e - b;
+            }
+        };
+        if (lane == 0) list[0] = 0;
+        __syncwarp();
+        while (top) {
+            // near the end of the list one node at a time: each of the tree's levels then adds at
+            // most seven more
+            const uint32_t take = min(top, top > kDvsList / 2 ? 1u : 32u);
+            const bool mine = lane < take;
+            const uint32_t node = mine ? list[top - 1 - lane] : 0u;
+            const int cls = mine ? classify(node) : 0;
+            top -= take;
+            const uint32_t nd = cls == 2 ? tv.daughters(node) : 0u;
+            const bool leaf = cls == 2 && nd == 0;
+            const uint32_t size = cls == 1 || leaf ? tv.end(node) - tv.begin(node) : 0u;
+            inside += __reduce_add_sync(full, cls == 1 ? size : 0u);
+            const unsigned lm = __ballot_sync(full, leaf);
+            uint32_t incl = nd;
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t o = __shfl_up_sync(full, incl, d);
+                if (lane >= (uint32_t)d) incl += o;
+            }
+            const uint32_t add = __shfl_sync(full, incl, 31);
+            if (top + add > kDvsList) {  // a tree deeper than an octree of 32 levels can be
+                if (lane == 0) atomicOr(err, (unsigned)kDevErrCapacity);
+                return;
+            }
+            __syncwarp();
+            for (uint32_t c = 0; c < nd; ++c) list[top + incl - nd + c] = tv.first(node) + c;
+            top += add;
+            if (lm) {
+                partial += __reduce_add_sync(full, leaf ? size : 0u);
+                if (kCount) {
+                    if (nleaf + __popc(lm) > kDvsLeaves) {
+                        count_leaves(false);
+                        nleaf = 0;
+                        __syncwarp();
+                        // the leaves of this step stay in partial: they are listed now
+                    }
+                    if (leaf) leaves[nleaf + __popc(lm & below)] = node;
+                    nleaf += __popc(lm);
+                }
+            }
+            __syncwarp();
+        }
+        if (kCount) count_leaves(true);
+        // a query that stopped early is not above the largest count: what it counted is a lower bound
+        if (lane == 0 && inside > *(volatile uint32_t *)&maxc[lev]) atomicMax(&maxc[lev], inside);
+        __syncwarp();
+    }
 }
 
 __global__ void k_z_extent(const double4_32a *pos, uint32_t n, unsigned long long *ext) {
@@ -115,8 +247,26 @@ int density_vs_scale(Context &c, const plan_params &p, double time, std::vector<
         PLAN_CUDA(cudaMemcpyAsync(d_y.p, ys.data(), ys.size() * 8, cudaMemcpyHostToDevice, s));
         PLAN_CUDA(cudaMemcpyAsync(d_z.p, zs.data(), zs.size() * 8, cudaMemcpyHostToDevice, s));
         PLAN_CUDA(cudaMemsetAsync(d_max.p, 0, (size_t)g.nlev * 4, s));
-        k_dvs<<<(unsigned)((nthreads + 127) / 128), 128, 0, s>>>(DevTreeView{ktree_of(tr)}, d_x.p, d_y.p, d_z.p, g, d_max.p, c.d_err);
-        c.launches++;
+        // the largest magnitude of a coordinate: the root box holds every node, the centres are their own
+        double coord = 0;
+        for (int d = 0; d < 3; ++d) coord = std::fmax(coord, std::fabs(tr.box.root_center[d]) + tr.box.half_width);
+        for (const std::vector<double> *v : {&xs, &ys, &zs})
+            if (!v->empty()) coord = std::fmax(coord, std::fmax(std::fabs(v->front()), std::fabs(v->back())) + g.sub1[0] + g.sub1[1] + g.sub1[2]);
+        const DvsGeomF gf = dvs_geom_f(g, coord);
+        int rc = ensure_split(c, s);
+        if (rc) return rc;
+        const FTree ft{tr.phi, tr.plo, tr.nhi, tr.nlo};
+        const DevTreeView tv{ktree_of(tr)};
+        const uint64_t ncentre = (uint64_t)g.nx * g.ny * g.nz * g.nlev;
+        int sms = 152;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
+        auto blocks = [&](uint64_t queries) { return (unsigned)std::min<uint64_t>((queries + kDvsWarps - 1) / kDvsWarps, (uint64_t)sms * 6); };
+        StreamBuf<unsigned long long> d_next(s);
+        PLAN_CUDA(d_next.alloc(2));
+        PLAN_CUDA(cudaMemsetAsync(d_next.p, 0, 16, s));
+        k_dvs<0><<<blocks(ncentre), 32 * kDvsWarps, 0, s>>>(tv, ft, d_x.p, d_y.p, d_z.p, g, gf, ncentre, d_next.p, d_max.p, c.d_err);
+        k_dvs<1><<<blocks(nthreads), 32 * kDvsWarps, 0, s>>>(tv, ft, d_x.p, d_y.p, d_z.p, g, gf, nthreads, d_next.p + 1, d_max.p, c.d_err);
+        c.launches += 2;
         PLAN_CUDA(cudaGetLastError());
         PLAN_CUDA(cudaMemcpyAsync(maxc.data(), d_max.p, (size_t)g.nlev * 4, cudaMemcpyDeviceToHost, s));
         PLAN_CUDA(cudaStreamSynchronize(s));

@@ -1,5 +1,6 @@
-// The arithmetic of --Density_Vs_Scale, host+device (dvs.cu runs it on the GPU; the parity
-// tests also compile it for the CPU and run it on the oracle's tree).
+// The arithmetic of --Density_Vs_Scale, host+device (dvs.cu runs the set-up, the queries and the
+// node classes on the GPU; the parity tests compile them for the CPU and run them, with the
+// plain count dvs_count, on the oracle's tree).
 //
 // BasicAnalysesWithTree (src/analyses.hpp:196-333) counts the tree points within a ball
 // around every cell centre of the grid (z from the cell centre at the box centre down past
@@ -25,7 +26,7 @@
 namespace plan {
 
 constexpr int kDvsMaxLevels = 24;
-constexpr int kDvsStack = 256;
+constexpr int kDvsDepth = 34;  // the root and 32 levels below it
 
 struct DvsGeom {
     double box_length[3], box_min[3], box_max[3];
@@ -130,77 +131,189 @@ PLAN_DVS_HD inline void dvs_query(const DvsGeom &g, const double *xs, const doub
     }
 }
 
-// RecursiveBallSearchCountWithShear from the root, depth first on an explicit stack. Tree
-// provides node(n, cx, cy, cz, hw), begin(n), end(n), first(n), daughters(n) and point(q, x,
-// y, z). Returns the count; *overflow is set (and the walk stops) if the stack would overrun,
-// which a 32-level octree cannot make happen.
-template <class Tree>
-PLAN_DVS_HD inline uint32_t dvs_count(const Tree &t, double cx, double cy, double cz, double r, const double *maxd, const DvsGeom &g,
-                                      bool *overflow) {
-    uint32_t stack[kDvsStack];
-    int top = 0;
-    stack[top++] = 0;
-    uint32_t count = 0;
-    const double c[3] = {cx, cy, cz};
-    while (top > 0) {
-        const uint32_t node = stack[--top];
-        double nc[3], c2c[3], hw;
-        t.node(node, nc[0], nc[1], nc[2], hw);
-        // ShearedCenter2Center (src/tree.hpp:3308-3331)
-        for (int i = 0; i < 3; ++i) {
-            c2c[i] = c[i] - nc[i];
-            if (std::fabs(c2c[i]) > maxd[i]) {
-                if (c2c[i] > 0) c2c[i] -= g.box_length[i];
-                else c2c[i] += g.box_length[i];
-                if (i == 0) {
-                    if (c[0] < 0) {
-                        nc[1] -= g.shear;
-                        nc[1] += (double)(int)((g.box_max[1] - nc[1]) / g.box_length[1]) * g.box_length[1];
-                    } else {
-                        nc[1] += g.shear;
-                        nc[1] -= (double)(int)((nc[1] - g.box_min[1]) / g.box_length[1]) * g.box_length[1];
-                    }
+// Where a node lies for the ball of radius r around c: 0 outside, 1 contained, 2 met
+// (src/tree.hpp:3308-3380). nc: the node's centre, hw its half width.
+PLAN_DVS_HD inline int dvs_class(const double c[3], const double node[3], double hw, double r, const double *maxd, const DvsGeom &g) {
+    double nc[3] = {node[0], node[1], node[2]}, c2c[3];
+    // ShearedCenter2Center (src/tree.hpp:3308-3331)
+    for (int i = 0; i < 3; ++i) {
+        c2c[i] = c[i] - nc[i];
+        if (std::fabs(c2c[i]) > maxd[i]) {
+            if (c2c[i] > 0) c2c[i] -= g.box_length[i];
+            else c2c[i] += g.box_length[i];
+            if (i == 0) {
+                if (c[0] < 0) {
+                    nc[1] -= g.shear;
+                    nc[1] += (double)(int)((g.box_max[1] - nc[1]) / g.box_length[1]) * g.box_length[1];
+                } else {
+                    nc[1] += g.shear;
+                    nc[1] -= (double)(int)((nc[1] - g.box_min[1]) / g.box_length[1]) * g.box_length[1];
                 }
             }
         }
-        // SphereContainNodeWithShear (src/tree.hpp:3335-3346)
-        const double tmp = hw * g.diag;
-        const double t0 = std::fabs(c2c[0]) + tmp, t1 = std::fabs(c2c[1]) + tmp, t2 = std::fabs(c2c[2]) + tmp;
-        if (t0 * t0 + t1 * t1 + t2 * t2 < r * r) {
-            count += t.end(node) - t.begin(node);
+    }
+    // SphereContainNodeWithShear (src/tree.hpp:3335-3346)
+    const double tmp = hw * g.diag;
+    const double t0 = std::fabs(c2c[0]) + tmp, t1 = std::fabs(c2c[1]) + tmp, t2 = std::fabs(c2c[2]) + tmp;
+    if (t0 * t0 + t1 * t1 + t2 * t2 < r * r) return 1;
+    // SphereNodeIntersectWithShear (src/tree.hpp:3350-3380)
+    const double cd = c2c[0] * c2c[0] + c2c[1] * c2c[1] + c2c[2] * c2c[2];
+    const double tr = tmp + r;
+    if (cd > tr * tr) return 0;
+    if (cd < r || cd < hw) return 2;
+    double m2 = 0;
+    for (int d = 0; d < 3; ++d) {
+        const double lo = (c[d] - c2c[d]) - hw, hi = (c[d] - c2c[d]) + hw;
+        if (c[d] < lo) m2 += (c[d] - lo) * (c[d] - lo);
+        else if (c[d] > hi) m2 += (c[d] - hi) * (c[d] - hi);
+    }
+    return m2 <= r * r ? 2 : 0;
+}
+
+// dvs_class in FP32: the same class, or -1 when a comparison is too close to call (or not
+// finite). The single-precision geometry: every coordinate, length and shear rounded once, and
+// eps, an absolute bound on the error of any difference formed from them: 2^-20 of the largest
+// magnitude among them (their roundings and the few operations on them stay below half of it).
+struct DvsGeomF {
+    float box_length[3], box_min1, box_max1, shear, eps;
+    float radius[kDvsMaxLevels];
+    float maxd[kDvsMaxLevels][3];
+};
+
+// coord: the largest magnitude of a node's or a query's coordinate
+inline DvsGeomF dvs_geom_f(const DvsGeom &g, double coord) {
+    DvsGeomF f{};
+    double big = coord + std::fabs(g.shear);
+    for (int d = 0; d < 3; ++d) {
+        f.box_length[d] = (float)g.box_length[d];
+        big += std::fabs(g.box_length[d]) + std::fabs(g.box_min[d]) + std::fabs(g.box_max[d]);
+    }
+    f.box_min1 = (float)g.box_min[1];
+    f.box_max1 = (float)g.box_max[1];
+    f.shear = (float)g.shear;
+    f.eps = (float)(big * 9.5367431640625e-07);
+    for (int i = 0; i < g.nlev; ++i) {
+        f.radius[i] = (float)g.radius[i];
+        for (int d = 0; d < 3; ++d) f.maxd[i][d] = (float)g.maxd[i][d];
+    }
+    return f;
+}
+
+// a < b for values within ea and eb of the exact ones: 1 yes, 0 no, -1 too close or not finite
+PLAN_DVS_HD inline int dvs_less(float a, float ea, float b, float eb) {
+    if (a + ea < b - eb) return 1;
+    if (a - ea > b + eb) return 0;
+    return -1;
+}
+
+PLAN_DVS_HD inline int dvs_class_f(const float c[3], const float node[3], float hw, int lev, const DvsGeomF &g) {
+    constexpr float kRel = 1.9073486328125e-06f;  // 2^-19: the roundings of the squares and sums below
+    const float r = g.radius[lev];
+    float n1 = node[1], d[3];
+    for (int i = 0; i < 3; ++i) {
+        d[i] = c[i] - (i == 1 ? n1 : node[i]);
+        // z is never periodic: its limit is a hundred boxes (maxd[2]), which a tree inside it keeps
+        const int far = dvs_less(g.maxd[lev][i], g.eps, std::fabs(d[i]), g.eps);
+        if (far < 0) return -1;
+        if (far) {
+            d[i] = d[i] > 0 ? d[i] - g.box_length[i] : d[i] + g.box_length[i];
+            if (i == 0) {
+                if (std::fabs(c[0]) <= g.eps) return -1;
+                float q;
+                if (c[0] < 0) {
+                    n1 = n1 - g.shear;
+                    q = (g.box_max1 - n1) / g.box_length[1];
+                } else {
+                    n1 = n1 + g.shear;
+                    q = (n1 - g.box_min1) / g.box_length[1];
+                }
+                const float k = std::trunc(q), e = 4.0f * g.eps / g.box_length[1];  // whole boxes moved
+                const float f = std::fabs(q - k);
+                if (!(e < 0.25f && std::fabs(q) < 4096.0f) || (f < e && std::fabs(q) > 0.5f) || f > 1.0f - e) return -1;
+                n1 = c[0] < 0 ? n1 + k * g.box_length[1] : n1 - k * g.box_length[1];
+            }
+        }
+    }
+    const float e = 8.0f * g.eps + hw * kRel;  // of a difference, moved by boxes or not, and of what hw adds
+    const float a0 = std::fabs(d[0]), a1 = std::fabs(d[1]), a2 = std::fabs(d[2]);
+    const float tmp = hw * 1.7320508f, rr = r * r, erR = rr * kRel;
+    const float t0 = a0 + tmp, t1 = a1 + tmp, t2 = a2 + tmp;
+    const float s = t0 * t0 + t1 * t1 + t2 * t2;
+    const int in = dvs_less(s, s * kRel + e * (2.0f * (t0 + t1 + t2) + 3.0f * e), rr, erR);
+    if (in != 0) return in;
+    const float cd = a0 * a0 + a1 * a1 + a2 * a2, ecd = cd * kRel + e * (2.0f * (a0 + a1 + a2) + 3.0f * e);
+    const float tr = tmp + r, tt = tr * tr;
+    const int out = dvs_less(tt, tt * kRel, cd, ecd);
+    if (out != 0) return out < 0 ? -1 : 0;
+    const int near_r = dvs_less(cd, ecd, r, r * kRel), near_h = dvs_less(cd, ecd, hw, hw * kRel);
+    if (near_r == 1 || near_h == 1) return 2;
+    if (near_r < 0 || near_h < 0) return -1;
+    const float b0 = a0 > hw ? a0 - hw : 0.0f, b1 = a1 > hw ? a1 - hw : 0.0f, b2 = a2 > hw ? a2 - hw : 0.0f;
+    const float m2 = b0 * b0 + b1 * b1 + b2 * b2;
+    const int gap = dvs_less(rr, erR, m2, m2 * kRel + e * (2.0f * (b0 + b1 + b2) + 3.0f * e));
+    return gap < 0 ? -1 : (gap ? 0 : 2);
+}
+
+// Walks the nodes the ball meets from the root, depth first: contained(n) for every contained
+// node, leaf(n) for every leaf that is met. classify(n) gives dvs_class. The siblings still to
+// visit are kept per level. *overflow is set (and the walk stops) if they would overrun the
+// stack, which a 32-level octree cannot make happen.
+template <class Tree, class Class, class Contained, class Leaf>
+PLAN_DVS_HD inline void dvs_walk(const Tree &t, Class classify, Contained contained, Leaf leaf, bool *overflow) {
+    uint32_t next[kDvsDepth], end[kDvsDepth];
+    int top = 0;
+    next[0] = 0;
+    end[0] = 1;
+    while (top >= 0) {
+        if (next[top] == end[top]) {
+            --top;
             continue;
         }
-        // SphereNodeIntersectWithShear (src/tree.hpp:3350-3380)
-        const double cd = c2c[0] * c2c[0] + c2c[1] * c2c[1] + c2c[2] * c2c[2];
-        const double tr = tmp + r;
-        if (cd > tr * tr) continue;
-        bool hit = cd < r || cd < hw;
-        if (!hit) {
-            double m2 = 0;
-            for (int d = 0; d < 3; ++d) {
-                const double lo = (c[d] - c2c[d]) - hw, hi = (c[d] - c2c[d]) + hw;
-                if (c[d] < lo) m2 += (c[d] - lo) * (c[d] - lo);
-                else if (c[d] > hi) m2 += (c[d] - hi) * (c[d] - hi);
+        const uint32_t n = next[top]++;
+        const int cls = classify(n);
+        if (cls == 1) {
+            contained(n);
+        } else if (cls == 2) {
+            const uint32_t nd = t.daughters(n);
+            if (nd == 0) {
+                leaf(n);
+            } else if (top + 1 == kDvsDepth) {
+                *overflow = true;
+                return;
+            } else {
+                ++top;
+                next[top] = t.first(n);
+                end[top] = next[top] + nd;
             }
-            hit = m2 <= r * r;
         }
-        if (!hit) continue;
-        const uint32_t nd = t.daughters(node);
-        if (nd == 0) {  // the points themselves are compared without the image
-            for (uint32_t q = t.begin(node); q != t.end(node); ++q) {
+    }
+}
+
+// RecursiveBallSearchCountWithShear (src/tree.hpp:3382-3402): the points of the contained nodes
+// and those of the met leaves within r, compared without the image. Tree provides node(n, cx,
+// cy, cz, hw), begin(n), end(n), first(n), daughters(n) and point(q, x, y, z).
+template <class Tree>
+PLAN_DVS_HD inline uint32_t dvs_count(const Tree &t, double cx, double cy, double cz, double r, const double *maxd, const DvsGeom &g,
+                                      bool *overflow) {
+    uint32_t count = 0;
+    const double c[3] = {cx, cy, cz};
+    dvs_walk(
+        t,
+        [&](uint32_t n) {
+            double nc[3], hw;
+            t.node(n, nc[0], nc[1], nc[2], hw);
+            return dvs_class(c, nc, hw, r, maxd, g);
+        },
+        [&](uint32_t n) { count += t.end(n) - t.begin(n); },
+        [&](uint32_t n) {
+            for (uint32_t q = t.begin(n); q != t.end(n); ++q) {
                 double px, py, pz;
                 t.point(q, px, py, pz);
                 const double dx = c[0] - px, dy = c[1] - py, dz = c[2] - pz;
                 if (dx * dx + dy * dy + dz * dz <= r * r) ++count;
             }
-        } else {
-            if (top + (int)nd > kDvsStack) {
-                *overflow = true;
-                return count;
-            }
-            for (int d = (int)nd - 1; d >= 0; --d) stack[top++] = t.first(node) + (uint32_t)d;
-        }
-    }
+        },
+        overflow);
     return count;
 }
 

@@ -396,7 +396,7 @@ int launch_by_k(uint32_t k, F f) {
 }  // namespace
 
 // FP32 hi/lo copies of points and node centres for the filtered kernels
-static int ensure_split(Context &c, cudaStream_t s) {
+int ensure_split(Context &c, cudaStream_t s) {
     DevTree &tr = c.tree;
     if (tr.phi) return kOk;
     tr.phi = c.arena.get<float4>(tr.Tu);
