@@ -2863,10 +2863,10 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
                         const unsigned long long *w = &rs[(size_t)kRbStats * worst];
                         std::fprintf(stderr,
                                      "[plan]   loop pass %u: %zu clumps, %llu calls, %llu accepted; worst clump: calls %llu scanned %llu cand %llu acc %llu "
-                                     "rounds %llu unsure %llu | kcycles search %llu accept %llu (warp-0 updates %llu: table %llu chain %llu) sort %llu (sums %llu; dist %llu "
-                                     "order %llu) sorts %llu members %llu | sum steps/kcycles:",
+                                     "rounds %llu unsure %llu | kcycles search %llu accept %llu (warp-0 windows %llu in %llu, updates %llu) sort %llu (sums %llu; dist %llu "
+                                     "order %llu) sorts %llu members %llu | chunks term by term/sum kcycles:",
                                      (unsigned)pass, active_all.size(), calls, acc, w[0], w[13], w[1], w[2], w[12], w[10], w[3] / 1000, w[4] / 1000,
-                                     w[14] / 1000, w[15] / 1000, w[16] / 1000, w[5] / 1000, w[6] / 1000, w[8] / 1000, w[9] / 1000, w[7], w[11]);
+                                     w[14] / 1000, w[15], w[16] / 1000, w[5] / 1000, w[6] / 1000, w[8] / 1000, w[9] / 1000, w[7], w[11]);
                         for (int q = 0; q < 7; ++q) std::fprintf(stderr, " %llu/%llu", w[17 + q], w[24 + q] / 1000);
                         std::fprintf(stderr, " | tiles %llu set-up kcycles %llu; predicted %llu held %llu taken %llu\n", w[32], w[31] / 1000, w[33],
                                      w[34], w[35]);

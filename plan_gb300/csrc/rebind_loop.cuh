@@ -20,15 +20,15 @@
 //  * acceptance: 512 candidates at a time, one per thread in registers (the next 512
 //    prefetched meanwhile). Every thread tests its candidate against the current state in
 //    FP32 (FP64 when too close to call), the block finds the first bound one, and warp 0
-//    applies the reference's FP64 update to the state. Its division is a reciprocal product
-//    with Markstein's correction; the reciprocals of the next masses are taken 32 at a time
-//    off the dependent chain while the accepted particles have equal masses;
+//    applies the reference's FP64 updates from it on, 32 candidates at a time: the updates of
+//    those bound on entry back to back, then all tests at once. The division of an update is a
+//    reciprocal product with Markstein's correction, the reciprocals taken off the chain;
 //  * SortParticles: the seven member sums in member order (ordered_sum_chunk over per-point
 //    products m, m x, ..., m vz formed once per snapshot, 256 members at a time, the next
 //    ones staged meanwhile), the centre of mass and the Hill radius,
 //    squared distances, and a stable sort by squared distance (in shared memory up to
-//    kRbSmall members, else a block radix sort on the top 32 bits and an exact fix-up of
-//    equal prefixes). Squared distances order members as distances do, except that two
+//    kRbSmall members, else a block radix sort on the leading bits and an exact fix-up of
+//    equal keys). Squared distances order members as distances do, except that two
 //    squared distances may round to one distance: neighbours within a few ulps are compared
 //    through their square roots, and a tie goes to the library-order replay exactly as in
 //    the round kernels. The square roots of the last sort are taken when the loop ends.
@@ -43,14 +43,19 @@ constexpr uint32_t kCallLimit = 1u << 20;     // calls of one clump in one launc
 constexpr int kRbStats = 40;                  // counters per slot
 constexpr int kCk = 24;                       // checkpoints per clump and run
 // dynamic shared memory: the largest of the frontier, the small sort and the acceptance
-// tile (per candidate: FP64 position and velocity, index, FP32 form, taken flag)
-constexpr size_t kRbTileBytes = (size_t)kRB * (64 + 4 + sizeof(CandF) + 1);
+// tile (per candidate: FP64 position and velocity, index, FP32 form)
+constexpr size_t kRbTileBytes = (size_t)kRB * (64 + 4 + sizeof(CandF));
 constexpr size_t kRbSmem14 = 14 * (kRbFront > kRbSmall ? kRbFront : kRbSmall);
-constexpr size_t kRbSmem = kRbSmem14 > kRbTileBytes ? kRbSmem14 : kRbTileBytes;
+// digit of the member sort: two passes order 22 bits of the squared distances' range, which
+// leaves runs of one or two members to the insertion sort; the counters are the largest use of
+// the dynamic shared memory
+constexpr uint32_t kRbDigit = 11;
+constexpr size_t kRbRadixBytes = ((size_t)kRbWarps << kRbDigit) * 4;
+constexpr size_t kRbSmemMost = kRbSmem14 > kRbTileBytes ? kRbSmem14 : kRbTileBytes;
+constexpr size_t kRbSmem = kRbRadixBytes > kRbSmemMost ? kRbRadixBytes : kRbSmemMost;
 static_assert(kRbFront * 14 <= kRbSmem, "frontier");
 static_assert(kRbTileBytes <= kRbSmem, "acceptance tile");
 static_assert(kRbSmall * 14 <= kRbSmem, "small sort");
-static_assert((256 + 256 * kRbWarps + 1) * 4 <= kRbSmem, "radix counters");
 
 // Checkpoints of the clumps' runs, by key rank: after the calls ck_after() selects, the
 // sorted member list (index, squared distance) and the state (M, centre, velocity, Hill
@@ -168,8 +173,9 @@ struct RbShared {
     uint32_t *warp_tot;
     uint32_t *u;         // scalars
     double *st;          // M, com x y z, vcom x y z, hill (the call's starting state)
-    double *tabM, *tabY; // reciprocal table (warp 0)
-    float *tabF;
+    double *sums;        // the member sums
+    double *tk;          // a window's updates: per acceptance m x .. m vz, M', 1 / M'
+    double *hist;        // the states of a window: x y z vx vy vz M, before it and after each update
     float *sf;           // acceptance state for every thread: hi[6], lo[6], Mf
     double *sd;          // acceptance state in FP64: x y z vx vy vz M
 };
@@ -306,22 +312,27 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
     const uint32_t nel = s_nel;
     const long long t1 = clock64();
     // 4) the reference's sequential acceptance (src/tree.hpp:4686-4706), 512 candidates at a
-    // time. Every thread holds one candidate (its FP32 form in registers; the FP64 position
-    // and velocity, the index, the FP32 form and the taken flag also in shared memory). The
-    // block finds the first bound candidate; warp 0 takes it and then goes on alone through
-    // the next candidates, 32 at a time, as long as each 32 holds a bound one (no block
-    // barrier per acceptance where acceptances are dense); the block search resumes after a
-    // 32 without any.
+    // time, those held by earlier clumps left out. Every thread holds one candidate (its FP32
+    // form; the FP64 position and velocity, the index and the FP32 form are in shared memory).
+    // The block finds the first bound candidate; warp 0 goes on from it alone, 32 candidates
+    // (a window) at a time, until none of a window's is bound; the block search then resumes.
+    //
+    // An update depends on all before it (RN(RN(RN(c M') + RN(m q)) / M') for every component,
+    // five dependent FP64 instructions of 64 cycles), the test of the next candidate on its
+    // result. A window therefore supposes that exactly the candidates bound to the state on
+    // entry (or too close to call) will be accepted: their masses M', the reciprocals and the
+    // products m q are formed by all lanes at once, the updates run back to back, and then
+    // every lane tests its candidate against the state just before it. What precedes the first
+    // candidate that came out otherwise is as the reference has it; the window ends there.
+    // Measured per accepted particle where they are dense: 550 cycles (27 to a window), against 1,790 with one
+    // test and one update at a time.
     double4_32a *tpos = reinterpret_cast<double4_32a *>(sh.buf), *tvel = tpos + kRB;
     uint32_t *tq = reinterpret_cast<uint32_t *>(tvel + kRB);
     CandF *tf = reinterpret_cast<CandF *>(tq + kRB);
-    uint8_t *ttk = reinterpret_cast<uint8_t *>(tf + kRB);
     uint32_t &s_pos = sh.u[8];
     const float G32 = (float)a.cp.G, shear32 = (float)a.cp.shear;
     double comp = 0.0;      // warp 0, lane c < 6: component c of the state (x y z vx vy vz)
     double M = sh.st[0];    // warp 0: the mass
-    double tab_m = -1.0;    // warp 0: the mass the reciprocal table was built for
-    int tab_n = 0, tab_i = 0;
     uint32_t nacc = 0, rounds = 0;
     if (tid == 0) {
         sh.u[12] = 0;
@@ -348,90 +359,140 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
             sh.sd[6] = M;
         }
     }
-    // warp 0 takes candidate j of the tile: the reference's update (src/tree.hpp:4696-4701,
-    // the new mass multiplies the old centre), lane c < 6 updating component c as
-    // RN(RN(RN(c M') + RN(m q_c)) / M'); the new state is published in shared memory
-    auto take = [&](uint32_t j) {
-        const unsigned full = 0xffffffffu;
-        const long long tu0 = clock64();
-        const double m = tpos[j].w;
-        if (!(tab_i < tab_n && dbits(m) == dbits(tab_m))) {
-            // the next masses M_{l+1} = RN(M_l + m) on the grid of M's binade (exact while
-            // they stay inside it), and their correctly rounded reciprocals
-            tab_m = m;
-            tab_i = 0;
-            tab_n = 0;
-            const uint64_t mb = dbits(M);
-            const uint32_t ex = (uint32_t)(mb >> 52) & 0x7ffu;
-            long long dn = 0;
-            if ((mb >> 63) == 0 && ex > 60u && ex < 2000u && grid_term(m, ex, dn) && dn > 0) {
-                const long long n0 = (long long)((mb & 0xfffffffffffffull) | (1ull << 52));
-                const long long nl = n0 + (long long)(lane + 1) * dn;
-                const bool ok = nl > (1LL << 52) && nl <= (1LL << 53);
-                const unsigned okm = __ballot_sync(full, ok);
-                const unsigned edge = __ballot_sync(full, ok && nl == (1LL << 53));
-                int cnt = (~okm) ? __ffs(~okm) - 1 : 32;
-                if (edge) cnt = min(cnt, __ffs(edge));
-                if (lane < cnt) {
-                    const double Ml = grid_value(nl, ex);
-                    float fh, fl;
-                    split_any(Ml, fh, fl);
-                    sh.tabM[lane] = Ml;
-                    sh.tabY[lane] = __drcp_rn(Ml);
-                    sh.tabF[lane] = fh;
-                }
-                tab_n = cnt;
-                __syncwarp();
-            }
-        }
-        const long long tu1 = clock64();
-        double Mn, y;
-        float Mnf;
-        if (tab_i < tab_n) {
-            Mn = sh.tabM[tab_i];
-            y = sh.tabY[tab_i];
-            Mnf = sh.tabF[tab_i];
-            ++tab_i;
-        } else {
-            Mn = M + m;
-            y = __drcp_rn(Mn);
-            float fl;
-            split_any(Mn, Mnf, fl);
-            tab_n = 0;
-        }
+    // the clump's state as the FP32 tests read it
+    auto publish = [&](double c, double mass) {
         if (lane < 6) {
-            // each lane loads its own component (one shared-memory load; a select over the
-            // whole position and velocity costs several hundred cycles here)
-            const double qc = reinterpret_cast<const double *>(lane < 3 ? &tpos[j] : &tvel[j])[lane < 3 ? lane : lane - 3];
-            const double num = comp * Mn + m * qc;
-            if ((dbits(num) << 1) == 0) {
-                comp = num;  // the quotient keeps the numerator's zero
-            } else {
-                const double q0 = num * y;
-                comp = fma(fma(-q0, Mn, num), y, q0);
-            }
             float h, l;
-            if (stat && lane == 0) sh.u[15] += (uint32_t)(clock64() - tu1);
-            split_f(comp, h, l);  // the FP64 pipe is idle here: its conversions beat the integer split
+            split_f(c, h, l);
             sh.sf[lane] = h;
             sh.sf[6 + lane] = l;
-            sh.sd[lane] = comp;
+            sh.sd[lane] = c;
         }
-        M = Mn;
         if (lane == 0) {
-            sh.sf[12] = Mnf;
-            sh.sd[6] = Mn;
-            const uint32_t q2 = tq[j];
+            sh.sf[12] = (float)mass;
+            sh.sd[6] = mass;
+        }
+        __syncwarp();
+    };
+    // warp 0: candidate k against the state in FP32
+    auto test = [&](const CandF &cf) { return bound_hilo_fast(cf, sh.sf[12], sh.sf, sh.sf + 6, G32, shear32); };
+    // warp 0 takes the window of the tile's candidates from at on; returns where the next one
+    // starts, and whether any candidate was bound (or too close to call) on entry
+    auto window = [&](uint32_t at, uint32_t tlen, bool &any) -> uint32_t {
+        const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
+        const uint32_t k = at + (uint32_t)lane;
+        const bool has = k < tlen;
+        CandF cf = tf[has ? k : at];
+        const unsigned P = __ballot_sync(full, has && test(cf) != 0);
+        any = P != 0;
+        if (!any) return min(at + 32u, tlen);
+        const long long tw0 = clock64();
+        // the masses after each supposed acceptance: integers on the grid of M's binade, up to
+        // the first lane where that does not hold (then one update with an ordinary addition)
+        const double m = has ? tpos[k].w : 0.0;
+        const bool sup = (P >> lane) & 1u;
+        const uint64_t mb = dbits(M);
+        const uint32_t ex = (uint32_t)(mb >> 52) & 0x7ffu;
+        long long dn = 0;
+        bool ok = true;
+        if (sup) ok = (mb >> 63) == 0 && ex > 60u && ex < 2000u && grid_term(m, ex, dn) && dn > 0;
+        long long nl = ok ? dn : 0;
+        for (int d = 1; d < 32; d <<= 1) {
+            const long long o = __shfl_up_sync(full, nl, d);
+            if (lane >= d) nl += o;
+        }
+        nl += (long long)((mb & 0xfffffffffffffull) | (1ull << 52));
+        ok = ok && (!sup || (nl > (1LL << 52) && nl < (1LL << 53)));
+        const unsigned okm = __ballot_sync(full, ok);
+        uint32_t lim = ~okm ? (uint32_t)__ffs(~okm) - 1u : 32u;  // lanes of this window
+        unsigned use = lim < 32 ? P & ((1u << lim) - 1u) : P;
+        double Ml = grid_value(nl, ex);
+        if (!use) {
+            const uint32_t j = (uint32_t)__ffs(P) - 1u;
+            use = 1u << j;
+            lim = j + 1;
+            Ml = M + m;
+        }
+        const uint32_t rank = __popc(use & below), cnt = __popc(use);
+        if ((use >> lane) & 1u) {
+            const double4_32a p = tpos[k], v = tvel[k];
+            double *t = sh.tk + 8 * rank;
+            t[0] = m * p.x;
+            t[1] = m * p.y;
+            t[2] = m * p.z;
+            t[3] = m * v.x;
+            t[4] = m * v.y;
+            t[5] = m * v.z;
+            t[6] = Ml;
+            t[7] = __drcp_rn(Ml);
+        }
+        if (lane < 6) sh.hist[lane] = comp;
+        if (lane == 6) sh.hist[6] = M;
+        __syncwarp();
+        // the updates, lane c < 6 component c, the state after each one kept. With a correctly
+        // rounded reciprocal Markstein's correction gives the correctly rounded quotient, but
+        // makes +0 of a numerator -0, which only a component that is -0 already can lead to.
+        auto updates = [&](auto zero) {
+            const int c = lane < 6 ? lane : 6;
+            double x = lane < 6 ? comp : 0.0;
+            const double *t = sh.tk;
+            double add = lane < 6 ? t[c] : 0.0, Mn = t[6], y = t[7];
+            for (uint32_t a = 0; a < cnt; ++a) {
+                t += a + 1 < cnt ? 8 : 0;
+                const double add1 = lane < 6 ? t[c] : 0.0, Mn1 = t[6], y1 = t[7];
+                const double num = x * Mn + add;
+                const double q0 = num * y;
+                x = fma(fma(-q0, Mn, num), y, q0);
+                if constexpr (decltype(zero)::value)
+                    if ((dbits(num) << 1) == 0) x = num;
+                if (lane < 7) sh.hist[8 * (a + 1) + lane] = lane < 6 ? x : Mn;
+                add = add1;
+                Mn = Mn1;
+                y = y1;
+            }
+        };
+        if (__any_sync(full, dbits(comp) == 1ull << 63)) updates(std::true_type());
+        else updates(std::false_type());
+        __syncwarp();
+        const long long tw1 = clock64();
+        // every candidate against the state before it
+        bool bound = false, unsure = false;
+        const double *S = sh.hist + 8 * rank;
+        if (has && (uint32_t)lane < lim) {
+            float h[6], l[6], mh, ml;
+            for (int c = 0; c < 6; ++c) split_any(S[c], h[c], l[c]);
+            split_any(S[6], mh, ml);
+            const int r = bound_hilo_fast(cf, mh, h, l, G32, shear32);
+            bound = r == 1;
+            unsure = r < 0;
+        }
+        if (unsure) {
+            bound = bound_fp64(tpos[k], tvel[k], S[6], S[0], S[1], S[2], S[3], S[4], S[5], a.cp);
+            if (stat) atomicAdd(&sh.u[12], 1u);
+        }
+        const unsigned B = __ballot_sync(full, bound);
+        unsigned diff = B ^ use;
+        if (lim < 32) diff &= (1u << lim) - 1u;
+        uint32_t end = diff ? (uint32_t)__ffs(diff) - 1u : lim;  // lanes before it came out as supposed
+        const unsigned acc = end < 32 ? use & ((1u << end) - 1u) : use;
+        if (diff && ((use >> end) & 1u)) ++end;  // supposed to be bound and is not: settled too
+        const uint32_t n = __popc(acc);
+        if ((acc >> lane) & 1u) {
+            const uint32_t q2 = tq[k];
             // the lowest rank keeps the particle; who lost one is found after the pass
             atomicMin(&a.owner[q2], myrank);
-            elig[nacc] = q2;  // accepted ones overwrite candidates already consumed
-            if (stat) {
-                sh.u[13] += (uint32_t)(clock64() - tu0);
-                sh.u[14] += (uint32_t)(tu1 - tu0);
-            }
+            elig[nacc + rank] = q2;  // accepted ones overwrite candidates already consumed
         }
-        ++nacc;
-        __syncwarp();
+        nacc += n;
+        comp = lane < 6 ? sh.hist[8 * n + lane] : 0.0;
+        M = sh.hist[8 * n + 6];
+        publish(comp, M);
+        if (stat && lane == 0) {
+            sh.u[13] += (uint32_t)(clock64() - tw0);
+            sh.u[14] += 1;
+            sh.u[15] += (uint32_t)(tw1 - tw0);
+        }
+        return min(at + end, tlen);
     };
     // the prefetched candidate of the next tile
     uint32_t nq = kNone, now_ = kNone, ntn = kNone;
@@ -451,7 +512,6 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
     for (uint32_t base = 0; base < nel; base += kRB) {
         const long long tt0 = clock64();
         const uint32_t q = nq;
-        const uint32_t tlen = min((uint32_t)kRB, nel - base);
         const bool valid = q != kNone;
         bool taken = true;
         CandF cf;
@@ -475,9 +535,6 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
                           a.dfirst, call);
             else if (tn != kNone && tn < myrank)
                 defer_add(a.dset, a.dover, a.dmax, slot, tn, true, a.dcall, a.dfirst, call);
-            tpos[tid] = np;
-            tvel[tid] = nv;
-            tq[tid] = q;
             cf.ph[0] = nph.x; cf.ph[1] = nph.y; cf.ph[2] = nph.z;
             cf.pl[0] = npl.x; cf.pl[1] = npl.y; cf.pl[2] = npl.z;
             split_any(nv.x, cf.vh[0], cf.vl[0]);
@@ -485,9 +542,15 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
             split_any(nv.z, cf.vh[2], cf.vl[2]);
             float wl;
             split_any(np.w, cf.w, wl);
-            tf[tid] = cf;
         }
-        ttk[tid] = taken ? 1 : 0;
+        uint32_t place;  // the candidates left, side by side in the tile
+        const uint32_t tlen = rb_block_rank(!taken, place, sh.warp_tot);
+        if (!taken) {
+            tpos[place] = np;
+            tvel[place] = nv;
+            tq[place] = q;
+            tf[place] = cf;
+        }
         nq = kNone;
         if (base + kRB + tid < nel) {  // prefetch (accepted ones are written below base + kRB only)
             nq = elig[base + kRB + tid];
@@ -501,16 +564,12 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
         __syncthreads();
         t_setup += clock64() - tt0;
         ++n_tiles;
-        for (uint32_t pos = 0;;) {
+        if ((uint32_t)tid < tlen) cf = tf[tid];
+        for (uint32_t pos = 0; pos < tlen;) {
             ++rounds;
             bool bound = false, unsure = false;
-            if (valid && !taken && (uint32_t)tid >= pos) {
-                float shv[6], slv[6];
-                for (int c = 0; c < 6; ++c) {
-                    shv[c] = sh.sf[c];
-                    slv[c] = sh.sf[6 + c];
-                }
-                const int r = bound_hilo_fast(cf, sh.sf[12], shv, slv, G32, shear32);
+            if ((uint32_t)tid < tlen && (uint32_t)tid >= pos) {
+                const int r = bound_hilo_fast(cf, sh.sf[12], sh.sf, sh.sf + 6, G32, shear32);
                 if (r >= 0) bound = r == 1;
                 else unsure = true;
             }
@@ -529,41 +588,12 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
             }
             if (f == kNone) break;  // the rest of the tile is not bound
             if (tid < 32) {
-                const unsigned full = 0xffffffffu;
-                take(f);
-                // warp 0 alone through the next candidates while acceptances are dense
-                uint32_t at = f + 1;
-                while (at < tlen) {
-                    const uint32_t k = at + lane;
-                    bool bd = false, un = false;
-                    if (k < tlen && !ttk[k]) {
-                        float shv[6], slv[6];
-                        for (int c = 0; c < 6; ++c) {
-                            shv[c] = sh.sf[c];
-                            slv[c] = sh.sf[6 + c];
-                        }
-                        const int r = bound_hilo_fast(tf[k], sh.sf[12], shv, slv, G32, shear32);
-                        if (r >= 0) bd = r == 1;
-                        else un = true;
-                    }
-                    if (un) {
-                        bd = bound_fp64(tpos[k], tvel[k], sh.sd[6], sh.sd[0], sh.sd[1], sh.sd[2], sh.sd[3], sh.sd[4], sh.sd[5], a.cp);
-                        if (stat) atomicAdd(&sh.u[12], 1u);
-                    }
-                    const unsigned bb = __ballot_sync(full, bd);
-                    if (!bb) {  // none of these 32 is bound: leave them, back to the block search
-                        at = min(at + 32u, tlen);
-                        break;
-                    }
-                    const uint32_t j = at + (uint32_t)(__ffs(bb) - 1);
-                    take(j);
-                    at = j + 1;
-                }
+                uint32_t at = f;
+                for (bool any = true; any && at < tlen;) at = window(at, tlen, any);
                 if (lane == 0) s_pos = at;
             }
             __syncthreads();
             pos = s_pos;
-            if (pos >= tlen) break;
         }
         __syncthreads();
     }
@@ -581,9 +611,9 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
             stat[12] += rounds;
             stat[13] += S;
             stat[10] += sh.u[12];
-            stat[14] += sh.u[13];
-            stat[15] += sh.u[14];  // of which the table look-up / rebuild
-            stat[16] += sh.u[15];  // and the FP64 update chain
+            stat[14] += sh.u[13];  // warp 0's windows: cycles, number, and cycles up to the last update
+            stat[15] += sh.u[14];
+            stat[16] += sh.u[15];
             stat[31] += (unsigned long long)t_setup;  // tile set-up: loads arriving, filters, splits
             stat[32] += n_tiles;
             stat[33] += sh.u[16];  // candidates predicted for an earlier clump
@@ -602,64 +632,88 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
 }
 
 // ------------------------------------------------------------------ SortParticles
-// Block radix sort (stable, 8-bit digits) of n (key, value) pairs from (ki, vi) into the
-// other buffer pair; digits that are the same for every key are skipped. Returns 0 when
-// the result is in (ki, vi), 1 when in (ko, vo).
-__device__ int rb_radix32(uint32_t *ki, uint32_t *vi, uint32_t *ko, uint32_t *vo, uint32_t n, uint32_t *smem) {
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    uint32_t *hist = smem, *wcnt = smem + 256, *flag = smem + 256 + 256 * kRbWarps;
+// Stable block sort of n keys of `bits` bits with their positions, by digits of kRbDigit bits:
+// (ki, position) to (ko, vo) and back, as many passes as the keys need (bits <= 2 kRbDigit).
+// Returns 1 when the result is in (ko, vo), 0 when in (ki, vi). Every warp counts and then
+// places a segment of its own with counters of its own, so a pass takes four block barriers
+// however long the segments are (with one 512-wide step at a time and three barriers in each,
+// four passes over 50,000 members took 1.27 M cycles; see kRbDigit for the digits).
+__device__ int rb_radix(uint32_t *ki, uint32_t *vi, uint32_t *ko, uint32_t *vo, uint32_t n, uint32_t bits, uint32_t *smem, uint32_t *warp_tot) {
+    constexpr uint32_t kBins = 1u << kRbDigit, kPer = kBins / kRB;
+    static_assert(kPer == 4, "a thread scans four digits");
+    const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, full = 0xffffffffu;
+    const uint32_t seg = ((n + kRbWarps * 32 - 1) / (kRbWarps * 32)) * 32, b = min(n, wid * seg), e = min(n, b + seg);
+    uint32_t *cnt = smem + wid * kBins;
     int where = 0;
-    for (int pass = 0; pass < 4; ++pass) {
-        const int sh = 8 * pass;
-        uint32_t *kin = where ? ko : ki, *vin = where ? vo : vi, *kout = where ? ki : ko, *vout = where ? vi : vo;
-        for (int d = tid; d < 256; d += kRB) hist[d] = 0;
-        for (int d = tid; d < 256 * kRbWarps; d += kRB) wcnt[d] = 0;
-        if (tid == 0) flag[0] = 0;
+    for (uint32_t sh = 0; sh < bits; sh += kRbDigit) {
+        const uint32_t *kin = where ? ko : ki, *vin = where ? vo : vi;
+        uint32_t *kout = where ? ki : ko, *vout = where ? vi : vo;
+        uint4 *z = reinterpret_cast<uint4 *>(smem);
+        for (uint32_t d = tid; d < kBins * kRbWarps / 4; d += kRB) z[d] = make_uint4(0, 0, 0, 0);
         __syncthreads();
-        for (uint32_t i = tid; i < n; i += kRB) atomicAdd(&hist[(kin[i] >> sh) & 255u], 1u);
+        for (uint32_t i = b + lane; i < e; i += 128) {
+            uint32_t k[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) k[j] = i + 32 * j < e ? kin[i + 32 * j] : 0u;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (i + 32 * j < e) atomicAdd(&cnt[(k[j] >> sh) & (kBins - 1)], 1u);
+        }
         __syncthreads();
-        for (int d = tid; d < 256; d += kRB)
-            if (hist[d] == n) flag[0] = 1;
-        __syncthreads();
-        if (flag[0]) continue;  // every key has this digit
-        if (tid < 32) {  // exclusive scan of the 256 bins by warp 0, 8 per lane
-            uint32_t v[8], s = 0;
-            for (int q = 0; q < 8; ++q) { v[q] = hist[lane * 8 + q]; s += v[q]; }
-            uint32_t incl = s;
+        {  // exclusive prefix over (digit, warp): four digits per thread
+            uint32_t s4[4] = {0, 0, 0, 0};
+            for (int w = 0; w < kRbWarps; ++w) {
+                const uint4 c = z[w * (kBins / 4) + tid];
+                s4[0] += c.x;
+                s4[1] += c.y;
+                s4[2] += c.z;
+                s4[3] += c.w;
+            }
+            const uint32_t mine = s4[0] + s4[1] + s4[2] + s4[3];
+            uint32_t incl = mine;
             for (int d = 1; d < 32; d <<= 1) {
-                const uint32_t u = __shfl_up_sync(0xffffffffu, incl, d);
-                if (lane >= d) incl += u;
+                const uint32_t o = __shfl_up_sync(full, incl, d);
+                if ((int)lane >= d) incl += o;
             }
-            uint32_t run = incl - s;
-            for (int q = 0; q < 8; ++q) { hist[lane * 8 + q] = run; run += v[q]; }
+            if (lane == 31) warp_tot[wid] = incl;
+            __syncthreads();
+            uint32_t at = incl - mine;
+            for (uint32_t w = 0; w < wid; ++w) at += warp_tot[w];
+            uint4 run = make_uint4(at, at + s4[0], at + s4[0] + s4[1], at + s4[0] + s4[1] + s4[2]);
+            for (int w = 0; w < kRbWarps; ++w) {
+                const uint4 c = z[w * (kBins / 4) + tid];
+                z[w * (kBins / 4) + tid] = run;
+                run.x += c.x;
+                run.y += c.y;
+                run.z += c.z;
+                run.w += c.w;
+            }
         }
         __syncthreads();
-        for (uint32_t b = 0; b < n; b += kRB) {
-            const uint32_t i = b + tid;
-            const bool valid = i < n;
-            const uint32_t key = valid ? kin[i] : 0u, val = valid ? vin[i] : 0u;
-            const uint32_t dig = valid ? (key >> sh) & 255u : 256u;
-            const unsigned peers = __match_any_sync(0xffffffffu, dig);
-            const uint32_t rk = __popc(peers & ((1u << lane) - 1u));
-            if (valid && (uint32_t)(__ffs(peers) - 1) == (uint32_t)lane) wcnt[wid * 256 + dig] = __popc(peers);
-            __syncthreads();
-            if (valid) {
-                uint32_t off = hist[dig];
-                for (int w = 0; w < wid; ++w) off += wcnt[w * 256 + dig];
-                kout[off + rk] = key;
-                vout[off + rk] = val;
+        for (uint32_t i0 = b; i0 < e; i0 += 128) {
+            uint32_t k[4], v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t i = i0 + 32 * j + lane;
+                k[j] = i < e ? kin[i] : 0u;
+                v[j] = i < e ? (sh ? vin[i] : i) : 0u;
             }
-            __syncthreads();
-            for (int d = tid; d < 256; d += kRB) {
-                uint32_t tot = 0;
-                for (int w = 0; w < kRbWarps; ++w) {
-                    tot += wcnt[w * 256 + d];
-                    wcnt[w * 256 + d] = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const bool some = i0 + 32 * j + lane < e;
+                const uint32_t d = some ? (k[j] >> sh) & (kBins - 1) : kBins;
+                const uint32_t peers = __match_any_sync(full, d), rk = __popc(peers & ((1u << lane) - 1u));
+                const uint32_t off = some ? cnt[d] : 0u;
+                __syncwarp();
+                if (some && rk == 0) cnt[d] = off + __popc(peers);
+                __syncwarp();
+                if (some) {
+                    kout[off + rk] = k[j];
+                    vout[off + rk] = v[j];
                 }
-                hist[d] += tot;
             }
-            __syncthreads();
         }
+        __syncthreads();
         where ^= 1;
     }
     return where;
@@ -678,6 +732,7 @@ __device__ __forceinline__ bool rb_sqrt_tie(double s0, double s1) {
 __device__ bool rb_sort_particles(const RbArgs &a, uint32_t slot, RbShared &sh, unsigned long long *stat) {
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     uint32_t &s_o = sh.u[8], &s_m = sh.u[9], &s_tie = sh.u[10], &s_r = sh.u[11];
+    uint32_t *s_kmin = sh.u + 20, *s_kmax = s_kmin + kRbWarps;
     const long long t0 = clock64();
     if (tid == 0) {
         s_o = a.ct.moff[slot];
@@ -747,16 +802,16 @@ __device__ bool rb_sort_particles(const RbArgs &a, uint32_t slot, RbShared &sh, 
         }
         tsum = clock64() - ts;
     }
-    if (wid < 7 && lane == 0) sh.tabM[wid] = acc;  // the table is free between calls
+    if (wid < 7 && lane == 0) sh.sums[wid] = acc;
     if (wid < 7 && lane == 0 && stat) {  // each sum: its time and the chunks it took term by term
         atomicAdd(&stat[17 + wid], (unsigned long long)its);
         atomicAdd(&stat[24 + wid], (unsigned long long)tsum);
     }
     __syncthreads();
     if (tid < 32) {
-        const double Ms = sh.tabM[0];
+        const double Ms = sh.sums[0];
         double v = 0.0;
-        if (lane >= 1 && lane <= 6) v = sh.tabM[lane] / Ms;
+        if (lane >= 1 && lane <= 6) v = sh.sums[lane] / Ms;
         if (lane == 7) v = cr_pow_third(Ms * a.cp.G / 3. / a.cp.Omega / a.cp.Omega);  // src/tree.hpp:4715-4717
         if (lane >= 1 && lane <= 7) sh.st[lane] = v;
         if (lane == 0) sh.st[0] = Ms;
@@ -769,8 +824,10 @@ __device__ bool rb_sort_particles(const RbArgs &a, uint32_t slot, RbShared &sh, 
         a.ct.vcom[slot] = make_double4_32a(sh.st[4], sh.st[5], sh.st[6], 0);
         a.ct.hill[slot] = sh.st[7];
     }
-    // 2) squared distances to the new centre (src/tree.hpp:4448-4450: (pos - com).Norm())
+    // 2) squared distances to the new centre (src/tree.hpp:4448-4450: (pos - com).Norm()), and
+    // the range of their top 32 bits
     const double cx = sh.st[1], cy = sh.st[2], cz = sh.st[3];
+    uint32_t kmin = kNone, kmax = 0;
     for (uint32_t k = tid; k < m; k += kRB) {
         const double4_32a p = a.t.pos[idx[k]];
         const double dx = p.x - cx, dy = p.y - cy, dz = p.z - cz;
@@ -778,8 +835,21 @@ __device__ bool rb_sort_particles(const RbArgs &a, uint32_t slot, RbShared &sh, 
         s = s + dy * dy;
         s = s + dz * dz;
         dist[k] = s;
+        const uint32_t hi = (uint32_t)(dbits(s) >> 32);
+        kmin = min(kmin, hi);
+        kmax = max(kmax, hi);
+    }
+    kmin = __reduce_min_sync(0xffffffffu, kmin);
+    kmax = __reduce_max_sync(0xffffffffu, kmax);
+    if (lane == 0) {
+        s_kmin[wid] = kmin;
+        s_kmax[wid] = kmax;
     }
     __syncthreads();
+    for (int w = 0; w < kRbWarps; ++w) {
+        kmin = min(kmin, s_kmin[w]);
+        kmax = max(kmax, s_kmax[w]);
+    }
     const long long t_dist = clock64();
     bool ok = true;
     if (m <= kRbSmall) {
@@ -833,8 +903,9 @@ __device__ bool rb_sort_particles(const RbArgs &a, uint32_t slot, RbShared &sh, 
         }
         __syncthreads();
     } else {
-        // 3b) large: radix sort of the top 32 bits with the position as payload into three
-        // fresh pool areas (D: the sorted segment; X, Y: sort buffers, given back after)
+        // 3b) large: radix sort by the leading 2 kRbDigit bits of the range (above the smallest),
+        // with the position as payload, into three fresh pool areas (D: the sorted segment; X,
+        // Y: sort buffers, given back after)
         if (tid == 0) s_r = pool_try_alloc(a.P, 3 * m);
         __syncthreads();
         const uint32_t r = s_r;
@@ -843,12 +914,13 @@ __device__ bool rb_sort_particles(const RbArgs &a, uint32_t slot, RbShared &sh, 
         } else {
             uint32_t *kx = a.P.idx + r + m, *ky = a.P.idx + r + 2 * m;
             uint32_t *vx = reinterpret_cast<uint32_t *>(a.P.dist + r + m), *vy = reinterpret_cast<uint32_t *>(a.P.dist + r + 2 * m);
+            const uint32_t bits = 32u - (uint32_t)__clz((int)(kmax - kmin)), drop = bits > 2 * kRbDigit ? bits - 2 * kRbDigit : 0u;
             for (uint32_t k = tid; k < m; k += kRB) {
-                kx[k] = (uint32_t)((unsigned long long)__double_as_longlong(dist[k]) >> 32);
-                vx[k] = k;
+                kx[k] = ((uint32_t)(dbits(dist[k]) >> 32) - kmin) >> drop;
+                vx[k] = k;  // what a range of no bits keeps
             }
             __syncthreads();
-            const int where = rb_radix32(kx, vx, ky, vy, m, reinterpret_cast<uint32_t *>(sh.buf));
+            const int where = rb_radix(kx, vx, ky, vy, m, bits - drop, reinterpret_cast<uint32_t *>(sh.buf), sh.warp_tot);
             const uint32_t *ks = where ? ky : kx, *vs = where ? vy : vx;
             uint32_t *didx = a.P.idx + r;
             double *ddist = a.P.dist + r;
@@ -858,7 +930,7 @@ __device__ bool rb_sort_particles(const RbArgs &a, uint32_t slot, RbShared &sh, 
                 ddist[k] = dist[src];
             }
             __syncthreads();
-            // runs of equal top bits: insertion sort by the full squared distance (stable)
+            // runs of equal keys: insertion sort by the full squared distance (stable)
             for (uint32_t k = tid; k < m; k += kRB) {
                 if ((k == 0 || ks[k] != ks[k - 1]) && k + 1 < m && ks[k + 1] == ks[k]) {
                     uint32_t e = k + 1;
@@ -968,11 +1040,11 @@ __device__ void rb_checkpoint(const RbArgs &a, uint32_t slot, uint32_t rank, uin
 __global__ void __launch_bounds__(kRB, 1) k_rebind_loop(RbArgs a) {
     extern __shared__ __align__(16) unsigned char rb_dyn[];
     __shared__ uint32_t warp_tot[kRbWarps];
-    __shared__ uint32_t u[20];
-    __shared__ double st[8], tabM[32], tabY[32], sd[8];
-    __shared__ float tabF[32], sf[16];
+    __shared__ uint32_t u[20 + 2 * kRbWarps];
+    __shared__ double st[8], sums[8], sd[8], tk[32 * 8], hist[33 * 8];
+    __shared__ float sf[16];
     __shared__ uint32_t s_item;
-    RbShared sh{rb_dyn, warp_tot, u, st, tabM, tabY, tabF, sf, sd};
+    RbShared sh{rb_dyn, warp_tot, u, st, sums, tk, hist, sf, sd};
     const int tid = threadIdx.x;
     for (uint32_t guard = 0; guard <= a.n; ++guard) {
         if (tid == 0) s_item = atomicAdd(a.head, 1u);
