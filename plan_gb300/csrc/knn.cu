@@ -16,65 +16,20 @@
 #include "exact64.cuh"
 #include "pipeline.h"
 #include "tree_walk.cuh"
-#include "knn_f32.cuh"
+#include "knn_warp.cuh"
 
 namespace plan {
 
 namespace {
 
 template <int KMAX>
-__global__ void __launch_bounds__(128) k_density(KTree t, uint32_t n, uint32_t k, double four_pi_over_three, double *dens, unsigned *err) {
+__global__ void __launch_bounds__(128) k_knn_positions(KTree t, const double *q3, const uint32_t *list, const uint32_t *nlist, uint32_t k,
+                                                       double est, uint32_t *oidx, double *odr2, unsigned *err) {
     extern __shared__ unsigned char smem[];
     double *sd = reinterpret_cast<double *>(smem);
     uint32_t *si = reinterpret_cast<uint32_t *>(sd + KMAX * blockDim.x);
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    SlabHeap h{sd + threadIdx.x, si + threadIdx.x, (int)blockDim.x};
-    double4_32a q = t.pos[i];
-    double r = knn_first_radius(t, q.x, q.y, q.z, t.leaf_of[i], k, err);
-    int got = knn_query(t, q.x, q.y, q.z, r, k, h, err);
-    if (got < (int)k) {
-        atomicOr(err, (unsigned)kDevErrCapacity);
-        dens[i] = 0;
-        return;
-    }
-    dens[i] = knn_median_density(t, h, (int)k, four_pi_over_three);
-}
-
-template <int KMAX>
-__global__ void __launch_bounds__(128) k_densest(KTree t, uint32_t n, uint32_t k, double threshold, const double *dens,
-                                                 uint32_t *densest, unsigned *err) {
-    extern __shared__ unsigned char smem[];
-    double *sd = reinterpret_cast<double *>(smem);
-    uint32_t *si = reinterpret_cast<uint32_t *>(sd + KMAX * blockDim.x);
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double di = dens[i];
-    uint32_t best = i;
-    if (di >= threshold) {  // src/tree.hpp:3719-3735
-        SlabHeap h{sd + threadIdx.x, si + threadIdx.x, (int)blockDim.x};
-        double4_32a q = t.pos[i];
-        double r = knn_first_radius(t, q.x, q.y, q.z, t.leaf_of[i], k, err);
-        int got = knn_query(t, q.x, q.y, q.z, r, k, h, err);
-        double bd = di;
-        for (int j = 0; j < got; ++j) {
-            uint32_t c = h.iget(j);
-            double dc = dens[c];
-            if (bd < dc) { best = c; bd = dc; }
-            else if (bd == dc && best > c) best = c;
-        }
-    }
-    densest[i] = best;
-}
-
-template <int KMAX>
-__global__ void __launch_bounds__(128) k_knn_positions(KTree t, const double *q3, uint32_t nq, uint32_t k, double est, uint32_t *oidx,
-                                                       double *odr2, unsigned *err) {
-    extern __shared__ unsigned char smem[];
-    double *sd = reinterpret_cast<double *>(smem);
-    uint32_t *si = reinterpret_cast<uint32_t *>(sd + KMAX * blockDim.x);
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nq) return;
+    for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < *nlist; u += gridDim.x * blockDim.x) {
+    const uint32_t i = list[u];
     SlabHeap h{sd + threadIdx.x, si + threadIdx.x, (int)blockDim.x};
     double qx = q3[3 * i], qy = q3[3 * i + 1], qz = q3[3 * i + 2];
     double r = est != 0 ? est : knn_first_radius(t, qx, qy, qz, 0xffffffffu, k, err);
@@ -83,156 +38,33 @@ __global__ void __launch_bounds__(128) k_knn_positions(KTree t, const double *q3
         oidx[(size_t)i * k + j] = j < got ? h.iget(j) : 0xffffffffu;
         odr2[(size_t)i * k + j] = j < got ? h.dget(j) : -1.0;
     }
+    }
 }
 
 
-// exact heap path, thread per query; list: the queries to answer (null: all nq)
+// ---------------------------------------------------------------- exact heap path
+// Thread per query, FP64, over a list on the device: what the warp kernels hand on because two
+// distances tie, which the library's heap order decides.
 template <int KMAX, int SPL>
-__global__ void __launch_bounds__(128) k_density_at(KTree t, const double *q3, const double *est, const uint32_t *list, uint32_t nq, uint32_t k,
-                                                    double four_pi_over_three, SplineCells sc, double *out, unsigned *err) {
+__global__ void __launch_bounds__(128) k_density_at(KTree t, const double *q3, const double *est, const uint32_t *list, const uint32_t *nlist,
+                                                    uint32_t k, double four_pi_over_three, SplineCells sc, double *out, unsigned *err) {
     extern __shared__ unsigned char smem[];
     double *sd = reinterpret_cast<double *>(smem);
     uint32_t *si = reinterpret_cast<uint32_t *>(sd + KMAX * blockDim.x);
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nq) return;
-    if (list) i = list[i];
-    SlabHeap h{sd + threadIdx.x, si + threadIdx.x, (int)blockDim.x};
-    double qx = q3[3 * i], qy = q3[3 * i + 1], qz = q3[3 * i + 2];
-    double r = est[i] != 0 ? est[i] : knn_first_radius(t, qx, qy, qz, 0xffffffffu, k, err);
-    int got = knn_query(t, qx, qy, qz, r, k, h, err);
-    if (got != (int)k) {
-        out[i] = 0.0;
-    } else if constexpr (SPL) {
-        // the reference passes self_id = 0: offsets are taken from tree point 0 (src/tree.hpp:4889, 4905)
-        const double4_32a p0 = t.pos[0];
-        out[i] = spline_density(t.pos, [&](int j) { return h.iget(j); }, (int)k, p0.x, p0.y, p0.z, sc);
-    } else {
-        out[i] = knn_median_density(t, h, (int)k, four_pi_over_three);
-    }
-}
-
-// Ascending sort of (key, index) pairs [0, n) by one warp (bitonic, in shared memory; the
-// entries up to the next power of two are padded, so C, a power of two, bounds n).
-template <int C>
-__device__ inline void warp_sort_pairs(unsigned long long *key, uint32_t *ix, uint32_t n, int lane) {
-    uint32_t P = 1;
-    while (P < n) P <<= 1;
-    for (uint32_t j = n + lane; j < P; j += 32) {
-        key[j] = ~0ull;
-        ix[j] = 0xffffffffu;
-    }
-    __syncwarp();
-    for (uint32_t size = 2; size <= P; size <<= 1)
-        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-            for (uint32_t u = lane; u < P / 2; u += 32) {
-                const uint32_t a = 2 * u - (u & (stride - 1)), b = a + stride;
-                const bool up = (a & size) == 0;
-                const unsigned long long ka = key[a], kb = key[b];
-                const uint32_t ia = ix[a], ib = ix[b];
-                const bool gt = ka > kb || (ka == kb && ia > ib);
-                if (gt == up) {
-                    key[a] = kb;
-                    key[b] = ka;
-                    ix[a] = ib;
-                    ix[b] = ia;
-                }
-            }
-            __syncwarp();
-        }
-}
-
-// Warp-cooperative form of k_density_at for queries that visit many points (the saddle
-// tests of the merge sweeps reach 10^5 points and more): one warp per query walks the tree
-// exactly as the reference does (every lane on the same path), the lanes take 32 points of
-// a visited range at a time, and every point within the running k-th smallest squared
-// distance goes to a per-warp buffer that a warp sort compacts. A squared distance is
-// non-negative, so its bits order like its value. With no tie at the k-boundary or inside
-// the k-set, the k kept are the reference heap's contents in its sorted order; a query with
-// such a tie, or one whose ties overflow the buffer, is listed for the exact heap path.
-template <int KM, int SPL>
-__global__ void __launch_bounds__(128) k_density_at_w(KTree t, const double *q3, const double *est, uint32_t nq, uint32_t k, double fpo3,
-                                                      SplineCells sc, double *out, uint32_t *redo, uint32_t *nredo, unsigned *err) {
-    constexpr uint32_t C = 4 * KM;  // candidates per warp
-    __shared__ unsigned long long s_key[4][C];
-    __shared__ uint32_t s_ix[4][C];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t i = blockIdx.x * 4 + w;
-    if (i >= nq) return;
-    const unsigned full = 0xffffffffu;
-    unsigned long long *key = s_key[w];
-    uint32_t *ix = s_ix[w];
-    const double qx = q3[3 * i], qy = q3[3 * i + 1], qz = q3[3 * i + 2];
-    double r = est[i] != 0 ? est[i] : knn_first_radius(t, qx, qy, qz, 0xffffffffu, k, err);
-    r = knn_final_radius(t, qx, qy, qz, r, k, err);
-    uint32_t n = 0, visited = 0;     // buffered candidates, points visited (the same in every lane)
-    unsigned long long tau = ~0ull;  // the running k-th smallest (bits); a point above it is out
-    bool overflow = false;
-    auto compact = [&]() {
-        warp_sort_pairs<C>(key, ix, n, lane);
-        if (n >= k) {
-            tau = key[k - 1];
-            uint32_t m = k;
-            while (m < n && key[m] == tau) ++m;
-            n = m;
-        }
-    };
-    traverse(t, qx, qy, qz, r,
-             [&](uint32_t b, uint32_t e, bool) {
-                 for (uint32_t p0 = b; p0 < e; p0 += 32) {
-                     const uint32_t p = p0 + (uint32_t)lane;
-                     unsigned long long kb = ~0ull;
-                     if (p < e) kb = dbits(point_dr2(qx, qy, qz, t.pos[p]));
-                     unsigned m = __ballot_sync(full, p < e && kb <= tau);
-                     if (!m) continue;
-                     if (n + __popc(m) > C) {
-                         compact();
-                         m = __ballot_sync(full, p < e && kb <= tau);
-                         if (n + __popc(m) > C) {
-                             overflow = true;
-                             return false;
-                         }
-                     }
-                     if ((m >> lane) & 1u) {
-                         const uint32_t at = n + __popc(m & ((1u << lane) - 1u));
-                         key[at] = kb;
-                         ix[at] = p;
-                     }
-                     n += __popc(m);
-                     __syncwarp();
-                 }
-                 visited += e - b;
-                 return true;
-             },
-             err);
-    bool redo_it = overflow;
-    if (!redo_it) {
-        compact();
-        if (visited < k) {  // fewer points than neighbours: the reference's zero
-            if (lane == 0) out[i] = 0.0;
-            return;
-        }
-        bool tie = n > k;  // a point beyond the k-th at the same distance
-        for (uint32_t j = 1 + (uint32_t)lane; j < k; j += 32) tie = tie || key[j] == key[j - 1];
-        redo_it = __any_sync(full, tie);
-    }
-    if (redo_it) {
-        if (lane == 0) redo[atomicAdd(nredo, 1u)] = i;
-        return;
-    }
-    if (lane == 0) {
-        if constexpr (SPL) {
-            const double4_32a p0 = t.pos[0];  // self_id = 0, as in the exact path
-            out[i] = spline_density(t.pos, [&](int j) { return ix[j]; }, (int)k, p0.x, p0.y, p0.z, sc);
+    for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < *nlist; u += gridDim.x * blockDim.x) {
+        const uint32_t i = list[u];
+        SlabHeap h{sd + threadIdx.x, si + threadIdx.x, (int)blockDim.x};
+        double qx = q3[3 * i], qy = q3[3 * i + 1], qz = q3[3 * i + 2];
+        double r = est[i] != 0 ? est[i] : knn_first_radius(t, qx, qy, qz, 0xffffffffu, k, err);
+        int got = knn_query(t, qx, qy, qz, r, k, h, err);
+        if (got != (int)k) {
+            out[i] = 0.0;
+        } else if constexpr (SPL) {
+            // the reference passes self_id = 0: offsets are taken from tree point 0 (src/tree.hpp:4889, 4905)
+            const double4_32a p0 = t.pos[0];
+            out[i] = spline_density(t.pos, [&](int j) { return h.iget(j); }, (int)k, p0.x, p0.y, p0.z, sc);
         } else {
-            // MedianSphericalDensityKernel on the sorted k-set, as knn_median_density
-            int j = (int)k;
-            const double m2 = 4 * dfrom(key[j / 2]);
-            for (j = j - 1; j >= 0; j--)
-                if (!(dfrom(key[j]) > m2)) break;
-            const double r2 = dfrom(key[j]);
-            double dens = 0;
-            for (; j >= 0; j--) dens = dens + t.pos[ix[j]].w;
-            out[i] = dens / (fpo3 * cr_pow15(r2));
+            out[i] = knn_median_density(t, h, (int)k, four_pi_over_three);
         }
     }
 }
@@ -256,133 +88,284 @@ __global__ void k_split_nodes(const double4_32a *ncf, uint32_t n, float4 *hi, fl
     lo[i] = make_float4((float)(c.x - (double)hx), (float)(c.y - (double)hy), (float)(c.z - (double)hz), (float)(c.w - (double)hw));
 }
 
-__device__ __forceinline__ double f_median_density(const KTree &t, const double *d64, const uint32_t *i64, int k, double fpo3) {
-    int i = k;
-    double m2 = 4 * d64[i / 2];
-    for (i = i - 1; i >= 0; i--) {
-        if (d64[i] > m2) continue;
-        break;
-    }
-    double r2 = d64[i];
-    double dens = 0;
-    for (; i >= 0; i--) dens = dens + t.pos[i64[i]].w;
-    return dens / (fpo3 * cr_pow15(r2));
-}
-
-template <int CAP, int SPL>
-__global__ void __launch_bounds__(128) k_density_f(KTree t, FTree f, uint32_t n, uint32_t k, double fpo3, SplineCells sc, double *dens,
-                                                   uint32_t *redo, uint32_t *nredo, unsigned *err) {
+template <int KMAX, int SPL>
+__global__ void __launch_bounds__(128) k_density_list(KTree t, const uint32_t *list, const uint32_t *nlist, uint32_t k, double fpo3,
+                                                      SplineCells sc, double *dens, unsigned *err) {
     extern __shared__ unsigned char smem[];
-    float *sk = reinterpret_cast<float *>(smem);
-    uint32_t *si = reinterpret_cast<uint32_t *>(sk + CAP * blockDim.x);
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool act = i < n;  // every lane reaches the reconvergence point below
-    FHeap fh{sk + threadIdx.x, si + threadIdx.x, (int)blockDim.x};
-    double d64[CAP];
-    uint32_t i64[CAP];
-    double4_32a q = make_double4_32a(0, 0, 0, 0);
-    int z = -1;
-    if (act) {
-        q = t.pos[i];
-        const double r = knn_first_radius(t, q.x, q.y, q.z, t.leaf_of[i], k, err);
-        z = knn_collect_f32(t, f, i, r, k, CAP, fh, err);
-    }
-    __syncwarp();  // the walks diverge; the FP64 part runs with the whole warp
-    const int got = z >= 0 ? knn_exact_f32(t, q.x, q.y, q.z, k, z, fh, d64, i64) : -1;
-    if (!act) return;
-    if (got < 0) {
-        redo[atomicAdd(nredo, 1u)] = i;
-        return;
-    }
-    if constexpr (SPL) dens[i] = spline_density(t.pos, [&](int j) { return i64[j]; }, (int)k, q.x, q.y, q.z, sc);
-    else dens[i] = f_median_density(t, d64, i64, (int)k, fpo3);
-}
-
-template <int CAP>
-__global__ void __launch_bounds__(128) k_densest_f(KTree t, FTree f, uint32_t n, uint32_t k, double threshold, const double *dens,
-                                                   uint32_t *densest, uint32_t *redo, uint32_t *nredo, unsigned *err) {
-    extern __shared__ unsigned char smem[];
-    float *sk = reinterpret_cast<float *>(smem);
-    uint32_t *si = reinterpret_cast<uint32_t *>(sk + CAP * blockDim.x);
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool act = i < n;  // every lane reaches the reconvergence point below
-    const double di = act ? dens[i] : 0.0;
-    uint32_t best = i;
-    const bool walk = act && di >= threshold;  // src/tree.hpp:3719-3735
-    FHeap fh{sk + threadIdx.x, si + threadIdx.x, (int)blockDim.x};
-    double d64[CAP];
-    uint32_t i64[CAP];
-    double4_32a q = make_double4_32a(0, 0, 0, 0);
-    int z = -1;
-    if (walk) {
-        q = t.pos[i];
-        const double r = knn_first_radius(t, q.x, q.y, q.z, t.leaf_of[i], k, err);
-        z = knn_collect_f32(t, f, i, r, k, CAP, fh, err);
-    }
-    __syncwarp();  // the walks diverge; the FP64 part runs with the whole warp
-    const int got = z >= 0 ? knn_exact_f32(t, q.x, q.y, q.z, k, z, fh, d64, i64) : -1;
-    if (!act) return;
-    if (walk) {
-        if (got < 0) {
-            redo[atomicAdd(nredo, 1u)] = i;
-            return;
+    double *sd = reinterpret_cast<double *>(smem);
+    uint32_t *si = reinterpret_cast<uint32_t *>(sd + KMAX * blockDim.x);
+    for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < *nlist; u += gridDim.x * blockDim.x) {
+        const uint32_t i = list[u];
+        SlabHeap h{sd + threadIdx.x, si + threadIdx.x, (int)blockDim.x};
+        double4_32a q = t.pos[i];
+        double r = knn_first_radius(t, q.x, q.y, q.z, t.leaf_of[i], k, err);
+        int got = knn_query(t, q.x, q.y, q.z, r, k, h, err);
+        if (got < (int)k) {
+            atomicOr(err, (unsigned)kDevErrCapacity);
+            dens[i] = 0;
+            continue;
         }
-        double bd = di;
-        for (int j = 0; j < got; ++j) {
-            uint32_t c = i64[j];
+        if constexpr (SPL) dens[i] = spline_density(t.pos, [&](int jj) { return h.iget(jj); }, (int)k, q.x, q.y, q.z, sc);
+        else dens[i] = knn_median_density(t, h, (int)k, fpo3);
+    }
+}
+
+template <int KMAX>
+__global__ void __launch_bounds__(128) k_densest_list(KTree t, const uint32_t *list, const uint32_t *nlist, uint32_t k, const double *dens,
+                                                      uint32_t *densest, unsigned *err) {
+    extern __shared__ unsigned char smem[];
+    double *sd = reinterpret_cast<double *>(smem);
+    uint32_t *si = reinterpret_cast<uint32_t *>(sd + KMAX * blockDim.x);
+    for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < *nlist; u += gridDim.x * blockDim.x) {
+        const uint32_t i = list[u];
+        SlabHeap h{sd + threadIdx.x, si + threadIdx.x, (int)blockDim.x};
+        double4_32a q = t.pos[i];
+        double r = knn_first_radius(t, q.x, q.y, q.z, t.leaf_of[i], k, err);
+        int got = knn_query(t, q.x, q.y, q.z, r, k, h, err);
+        uint32_t best = i;
+        double bd = dens[i];
+        for (int jj = 0; jj < got; ++jj) {
+            uint32_t c = h.iget(jj);
             double dc = dens[c];
             if (bd < dc) { best = c; bd = dc; }
             else if (bd == dc && best > c) best = c;
         }
+        densest[i] = best;
     }
-    densest[i] = best;
 }
 
-// exact FP64 path for a list of queries
-template <int KMAX, int SPL>
-__global__ void __launch_bounds__(128) k_density_list(KTree t, const uint32_t *list, uint32_t n, uint32_t k, double fpo3, SplineCells sc,
-                                                      double *dens, unsigned *err) {
-    extern __shared__ unsigned char smem[];
-    double *sd = reinterpret_cast<double *>(smem);
-    uint32_t *si = reinterpret_cast<uint32_t *>(sd + KMAX * blockDim.x);
-    uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    uint32_t i = list[j];
-    SlabHeap h{sd + threadIdx.x, si + threadIdx.x, (int)blockDim.x};
-    double4_32a q = t.pos[i];
-    double r = knn_first_radius(t, q.x, q.y, q.z, t.leaf_of[i], k, err);
-    int got = knn_query(t, q.x, q.y, q.z, r, k, h, err);
-    if (got < (int)k) {
-        atomicOr(err, (unsigned)kDevErrCapacity);
-        dens[i] = 0;
+// ---------------------------------------------------------------- warp per query
+// Densities of the tree points from the FP32 keys (median kernel). The density needs, of the
+// sorted k-set, the masses up to the last distance that is not beyond twice the median one
+// (MedianSphericalDensityKernel, src/tree.hpp:3473-3491) and that distance itself: the point
+// there and the number of masses go to at and cnt, and k_density_finish forms the density in
+// FP64, a thread per point. Where the tree's masses differ and those of a query do, their sum in
+// ascending order goes to dens and kMixed marks it. A query whose k-set, median cut, last point
+// or order is too close to tell in FP32 is listed for the exact warp kernel.
+constexpr uint32_t kMixed = 0x80000000u;
+
+__global__ void __launch_bounds__(32 * kWkWarps) k_density_w(KTree t, FTree f, uint32_t n, uint32_t k, bool uniform, uint32_t *at, uint32_t *cnt,
+                                                             double *dens, uint32_t *redo, uint32_t *nredo, unsigned *err) {
+    __shared__ WkBuf s_buf[kWkWarps];
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, full = 0xffffffffu;
+    const uint32_t i = blockIdx.x * kWkWarps + w;
+    if (i >= n) return;
+    WkBuf &s = s_buf[w];
+    const double4_32a p = t.pos[i];
+    WkQuery q{p.x, p.y, p.z, f.phi[i], f.plo[i]};
+    uint32_t m, visited, tau;
+    bool ok = wk_collect(t, f, q, wk_first_radius(t, q, t.leaf_of[i], k, err), k, s, m, visited, tau, err) && visited >= k && wk_kset(s, k, m, tau);
+    uint32_t last = 0, c = 0;
+    if (ok) {
+        __syncwarp();
+        // the median, and which members lie within twice its distance (four times its square)
+        uint32_t count, med = 0;
+        const uint32_t T = wk_select(s.key, k, k / 2 + 1, count);
+        for (uint32_t j = lane; j < k; j += 32)
+            if (s.key[j] <= T) med = max(med, s.key[j]);
+        med = __reduce_max_sync(full, med);
+        const float lo4 = 4.f * f_lo(__uint_as_float(med)), hi4 = 4.f * f_hi(__uint_as_float(med));
+        uint32_t far = 0, second = 0;
+        bool clear = true;
+        for (uint32_t j = lane; j < k; j += 32) {
+            const float v = __uint_as_float(s.key[j]);
+            const bool in = f_hi(v) <= lo4;
+            clear = clear && (in || f_lo(v) > hi4);
+            if (in) {
+                ++c;
+                second = max(second, min(far, s.key[j]));
+                far = max(far, s.key[j]);
+            }
+        }
+        c = __reduce_add_sync(full, c);
+        const uint32_t top = __reduce_max_sync(full, far);
+        const unsigned holders = __ballot_sync(full, far == top);
+        // the last point: no other as far, within the error bound
+        second = __reduce_max_sync(full, (far == top && lane == (uint32_t)(__ffs(holders) - 1)) ? second : far);
+        ok = __all_sync(full, clear) && c > 0 && f_hi(__uint_as_float(second)) < f_lo(__uint_as_float(top));
+        if (c == 1) ok = __all_sync(full, clear);
+        for (uint32_t j = lane; j < k; j += 32)
+            if (s.key[j] == top) last = s.ix[j];
+        last = __reduce_max_sync(full, last);
+        if (ok && !uniform) {
+            // all the summed masses the same? then k_density_finish adds them
+            const double m0 = t.pos[last].w;
+            bool same = true;
+            for (uint32_t j = lane; j < k; j += 32)
+                if (s.key[j] <= top) same = same && t.pos[s.ix[j]].w == m0;
+            if (!__all_sync(full, same)) {
+                // by rank, in ascending order; every neighbour in the order must be clear
+                double *ms = reinterpret_cast<double *>(s.xkey);
+                bool order = true;
+                for (uint32_t j = lane; j < k; j += 32) {
+                    const uint32_t v = s.key[j];
+                    if (v > top) continue;
+                    uint32_t rank = 0;
+                    for (uint32_t o = 0; o < k; ++o) {
+                        const uint32_t u = s.key[o];
+                        rank += u < v ? 1u : 0u;
+                        order = order && (o == j || u > top || f_hi(__uint_as_float(min(u, v))) < f_lo(__uint_as_float(max(u, v))));
+                    }
+                    ms[rank] = t.pos[s.ix[j]].w;
+                }
+                ok = __all_sync(full, order);
+                __syncwarp();
+                if (ok && lane == 0) {
+                    double sum = 0;
+                    for (int j = (int)c - 1; j >= 0; j--) sum = sum + ms[j];
+                    dens[i] = sum;
+                }
+                c |= kMixed;
+            }
+        }
+    }
+    if (lane == 0) {
+        at[i] = last;
+        cnt[i] = ok ? c : 0u;
+        if (!ok) redo[atomicAdd(nredo, 1u)] = i;
+    }
+}
+
+__global__ void k_density_finish(const double4_32a *pos, uint32_t n, double fpo3, const uint32_t *at, const uint32_t *cnt, double *dens) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const uint32_t c = cnt[i];
+    if (!c) return;  // listed
+    const double4_32a q = pos[i], p = pos[at[i]];
+    const double r2 = point_dr2(q.x, q.y, q.z, p);
+    double sum = 0;
+    if (c & kMixed) sum = dens[i];
+    else
+        for (uint32_t j = 0; j < c; ++j) sum = sum + p.w;
+    dens[i] = sum / (fpo3 * cr_pow15(r2));
+}
+
+// The densest of a point's k nearest and itself (src/tree.hpp:3719-3735): the largest density,
+// the smallest index among equal ones, whatever the order. Densities are positive (their bits
+// order like their values). At the points below the threshold, themselves.
+__device__ __forceinline__ void wk_densest(const uint32_t *ix, uint32_t k, uint32_t i, double di, const double *dens, uint32_t *densest) {
+    const uint32_t lane = threadIdx.x & 31, full = 0xffffffffu;
+    double bd = di;
+    uint32_t best = i;
+    for (uint32_t j = lane; j < k; j += 32) {
+        const uint32_t c = ix[j];
+        const double dc = dens[c];
+        if (dbits(bd) < dbits(dc)) { best = c; bd = dc; }
+        else if (dbits(bd) == dbits(dc) && best > c) best = c;
+    }
+    const uint32_t hi = __reduce_max_sync(full, (uint32_t)(dbits(bd) >> 32));
+    const uint32_t lo = __reduce_max_sync(full, (uint32_t)(dbits(bd) >> 32) == hi ? (uint32_t)dbits(bd) : 0u);
+    best = __reduce_min_sync(full, dbits(bd) == (((uint64_t)hi << 32) | lo) ? best : 0xffffffffu);
+    if (lane == 0) densest[i] = best;
+}
+
+__global__ void __launch_bounds__(32 * kWkWarps) k_densest_w(KTree t, FTree f, uint32_t n, uint32_t k, double threshold, const double *dens,
+                                                             uint32_t *densest, uint32_t *redo, uint32_t *nredo, unsigned *err) {
+    __shared__ WkBuf s_buf[kWkWarps];
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t i = blockIdx.x * kWkWarps + w;
+    if (i >= n) return;
+    WkBuf &s = s_buf[w];
+    const double di = dens[i];
+    if (!(di >= threshold)) {  // src/tree.hpp:3719-3735
+        if (lane == 0) densest[i] = i;
         return;
     }
-    if constexpr (SPL) dens[i] = spline_density(t.pos, [&](int jj) { return h.iget(jj); }, (int)k, q.x, q.y, q.z, sc);
-    else dens[i] = knn_median_density(t, h, (int)k, fpo3);
+    const double4_32a p = t.pos[i];
+    WkQuery q{p.x, p.y, p.z, f.phi[i], f.plo[i]};
+    uint32_t m, visited, tau;
+    if (wk_collect(t, f, q, wk_first_radius(t, q, t.leaf_of[i], k, err), k, s, m, visited, tau, err) && visited >= k && wk_kset(s, k, m, tau)) {
+        __syncwarp();
+        wk_densest(s.ix, k, i, di, dens, densest);
+    } else if (lane == 0) {
+        redo[atomicAdd(nredo, 1u)] = i;
+    }
 }
 
-template <int KMAX>
-__global__ void __launch_bounds__(128) k_densest_list(KTree t, const uint32_t *list, uint32_t n, uint32_t k, double threshold,
-                                                      const double *dens, uint32_t *densest, unsigned *err) {
-    extern __shared__ unsigned char smem[];
-    double *sd = reinterpret_cast<double *>(smem);
-    uint32_t *si = reinterpret_cast<uint32_t *>(sd + KMAX * blockDim.x);
-    uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    uint32_t i = list[j];
-    SlabHeap h{sd + threadIdx.x, si + threadIdx.x, (int)blockDim.x};
-    double4_32a q = t.pos[i];
-    double r = knn_first_radius(t, q.x, q.y, q.z, t.leaf_of[i], k, err);
-    int got = knn_query(t, q.x, q.y, q.z, r, k, h, err);
-    uint32_t best = i;
-    double bd = dens[i];
-    for (int jj = 0; jj < got; ++jj) {
-        uint32_t c = h.iget(jj);
-        double dc = dens[c];
-        if (bd < dc) { best = c; bd = dc; }
-        else if (bd == dc && best > c) best = c;
+// The exact k-set in FP64 order, for queries at given positions (q3; est: the first radius, 0
+// for the reference's own) or at the tree points of a list, counted on the device (nlist) or by
+// the host. What it makes of them:
+enum WkOp {
+    kOpMedian,   // the median density
+    kOpSpline,   // the spline density (offsets from tree point 0 at given positions: self_id = 0, as in the heap path)
+    kOpDensest,  // the densest neighbour
+    kOpKnn,      // indices and squared distances
+};
+struct WkOut {
+    double *dens;             // kOpMedian, kOpSpline: the result; kOpDensest: the densities
+    uint32_t *idx;            // kOpDensest: the result; kOpKnn: k per query
+    double *dr2;              // kOpKnn
+    uint32_t *redo, *nredo;   // queries for the heap path
+};
+
+template <int OP>
+__global__ void __launch_bounds__(32 * kWkWarps) k_exact_w(KTree t, FTree f, const double *q3, const double *est, double est0, const uint32_t *list,
+                                                           const uint32_t *nlist, uint32_t nq, uint32_t k, double fpo3, SplineCells sc, WkOut out,
+                                                           unsigned *err) {
+    __shared__ WkBuf s_buf[kWkWarps];
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    WkBuf &s = s_buf[w];
+    if (nlist) nq = *nlist;
+    for (uint32_t u = blockIdx.x * kWkWarps + w; u < nq; u += gridDim.x * kWkWarps) {
+        const uint32_t i = list ? list[u] : u;
+        double4_32a p;
+        if (q3) p = make_double4_32a(q3[3 * (size_t)i], q3[3 * (size_t)i + 1], q3[3 * (size_t)i + 2], 0.0);
+        else p = t.pos[i];
+        const WkQuery q = wk_query(p.x, p.y, p.z);
+        double r = q3 ? (est ? est[i] : est0) : 0.0;
+        if (q3) r = r != 0 ? r : knn_first_radius(t, p.x, p.y, p.z, 0xffffffffu, k, err);
+        else r = wk_first_radius(t, q, t.leaf_of[i], k, err);
+        uint32_t m, visited, tau;
+        __syncwarp();
+        bool ok = wk_collect(t, f, q, r, k, s, m, visited, tau, err);
+        if (ok && visited < k && (OP == kOpMedian || OP == kOpSpline) && q3) {  // fewer points than neighbours: the reference's zero
+            if (lane == 0) out.dens[i] = 0.0;
+            continue;
+        }
+        ok = ok && visited >= k && wk_sorted(t, q, s, k, m, tau);
+        if (!ok) {
+            if (lane == 0) out.redo[atomicAdd(out.nredo, 1u)] = i;
+            continue;
+        }
+        if constexpr (OP == kOpKnn) {
+            for (uint32_t j = lane; j < k; j += 32) {
+                out.idx[(size_t)i * k + j] = s.xix[j];
+                out.dr2[(size_t)i * k + j] = dfrom(s.xkey[j]);
+            }
+        } else if constexpr (OP == kOpDensest) {
+            wk_densest(s.xix, k, i, out.dens[i], out.dens, out.idx);
+        } else if constexpr (OP == kOpSpline) {
+            // the terms by the lanes, their sum in ascending order by one
+            const double4_32a o = q3 ? t.pos[0] : p;
+            double *term = reinterpret_cast<double *>(s.key);
+            static_assert(sizeof(s.key) + sizeof(s.ix) >= 128 * sizeof(double), "terms");
+            for (uint32_t j = lane; j < k; j += 32) {
+                const double4_32a c = t.pos[s.xix[j]];
+                term[j] = c.w / sc.volume * spline_weight(c.x - o.x, c.y - o.y, c.z - o.z, sc);
+            }
+            __syncwarp();
+            if (lane == 0) {
+                double dens = 0;
+                for (uint32_t j = 0; j < k; ++j) dens = dens + term[j];
+                out.dens[i] = dens;
+            }
+        } else {
+            double *ms = reinterpret_cast<double *>(s.key);
+            for (uint32_t j = lane; j < k; j += 32) ms[j] = t.pos[s.xix[j]].w;
+            __syncwarp();
+            if (lane == 0) {  // MedianSphericalDensityKernel on the sorted k-set, as knn_median_density
+                int j = (int)k;
+                const double m2 = 4 * dfrom(s.xkey[j / 2]);
+                for (j = j - 1; j >= 0; j--)
+                    if (!(dfrom(s.xkey[j]) > m2)) break;
+                const double r2 = dfrom(s.xkey[j]);
+                double dens = 0;
+                for (; j >= 0; j--) dens = dens + ms[j];
+                out.dens[i] = dens / (fpo3 * cr_pow15(r2));
+            }
+        }
+        __syncwarp();
     }
-    densest[i] = best;
 }
 
 template <class F>
@@ -411,95 +394,113 @@ int ensure_split(Context &c, cudaStream_t s) {
     return kOk;
 }
 
-template <class F>
-static int launch_by_cap(uint32_t k, F f) {
-    if (k <= 16) return f(std::integral_constant<int, 24>());
-    if (k <= 32) return f(std::integral_constant<int, 40>());
-    if (k <= 64) return f(std::integral_constant<int, 72>());
-    return kErrUnsupported;
+// Blocks for a list whose length only the device knows: enough to fill the GPU.
+static unsigned list_blocks(Context &c) {
+    int sms = 152;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
+    return (unsigned)sms * 4u;
 }
 
+// Two redo lists (for the exact warp kernel, then for the heap path) and their counts.
+struct RedoLists {
+    uint32_t *warp, *heap, *n;  // n[0], n[1]
+    int take(Context &c, size_t most, cudaStream_t s) {
+        warp = c.scratch.get<uint32_t>(most + 1);
+        heap = c.scratch.get<uint32_t>(most + 1);
+        n = c.scratch.get<uint32_t>(4);
+        if (!warp || !heap || !n) return kErrOutOfMemory;
+        PLAN_CUDA(cudaMemsetAsync(n, 0, 8, s));
+        return kOk;
+    }
+};
+
 int launch_density(Context &c, const plan_params &p, uint32_t k, cudaStream_t s) {
+    if (k > 64) return kErrUnsupported;
     KTree t = ktree_of(c.tree);
     const double fpo3 = 3.14159265358979323846 * 4. / 3.;
     int rc = ensure_split(c, s);
     if (rc) return rc;
     FTree f{c.tree.phi, c.tree.plo, c.tree.nhi, c.tree.nlo};
     const uint32_t n = c.tree.Tu;
-    uint32_t *redo = c.scratch.get<uint32_t>(n + 1), *nredo = c.scratch.get<uint32_t>(4);
-    if (!redo || !nredo) return kErrOutOfMemory;
-    PLAN_CUDA(cudaMemsetAsync(nredo, 0, 4, s));
-    const bool spl = !c.fs.median_kernel;
+    const size_t mark = c.scratch.used;
+    RedoLists redo;
+    rc = redo.take(c, n, s);
+    if (rc) return rc;
     const SplineCells sc = c.fs.spline;
-    rc = launch_by_cap(k, [&](auto capc) {
-        constexpr int CAP = decltype(capc)::value;
-        size_t sm = (size_t)CAP * 128 * 8;
-        auto kern = spl ? k_density_f<CAP, 1> : k_density_f<CAP, 0>;
-        if (sm > 48 * 1024) PLAN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        PLAN_CUDA(cudaEventRecord(c.kev[0], s));
-        kern<<<grid_for(n, 128), 128, sm, s>>>(t, f, n, k, fpo3, sc, c.tree.dens, redo, nredo, c.d_err);
-        PLAN_CUDA(cudaEventRecord(c.kev[1], s));
+    const unsigned lb = list_blocks(c);
+    WkOut out{c.tree.dens, nullptr, nullptr, redo.heap, redo.n + 1};
+    PLAN_CUDA(cudaEventRecord(c.kev[0], s));
+    if (c.fs.median_kernel) {
+        uint32_t *at = c.scratch.get<uint32_t>(n), *cnt = c.scratch.get<uint32_t>(n);
+        if (!at || !cnt) return kErrOutOfMemory;
+        const bool uniform = c.tree.nsinks == 0 && p.ntypes <= 1;
+        k_density_w<<<(n + kWkWarps - 1) / kWkWarps, 32 * kWkWarps, 0, s>>>(t, f, n, k, uniform, at, cnt, c.tree.dens, redo.warp, redo.n, c.d_err);
+        k_density_finish<<<grid_for(n, 256), 256, 0, s>>>(t.pos, n, fpo3, at, cnt, c.tree.dens);
+        k_exact_w<kOpMedian><<<lb, 32 * kWkWarps, 0, s>>>(t, f, nullptr, nullptr, 0.0, redo.warp, redo.n, 0, k, fpo3, sc, out, c.d_err);
+        c.launches += 3;
+    } else {
+        k_exact_w<kOpSpline><<<(n + kWkWarps - 1) / kWkWarps, 32 * kWkWarps, 0, s>>>(t, f, nullptr, nullptr, 0.0, nullptr, nullptr, n, k, fpo3, sc,
+                                                                                  out, c.d_err);
+        c.launches++;
+    }
+    rc = launch_by_k(k, [&](auto km, int threads) {
+        constexpr int KM = decltype(km)::value;
+        size_t sm = (size_t)KM * threads * 12;
+        auto kern = c.fs.median_kernel ? k_density_list<KM, 0> : k_density_list<KM, 1>;
+        kern<<<lb, threads, sm, s>>>(t, redo.heap, redo.n + 1, k, fpo3, sc, c.tree.dens, c.d_err);
         c.launches++;
         PLAN_CUDA(cudaGetLastError());
         return (int)kOk;
     });
     if (rc) return rc;
-    uint32_t h = 0;
-    PLAN_CUDA(cudaMemcpyAsync(&h, nredo, 4, cudaMemcpyDeviceToHost, s));
+    PLAN_CUDA(cudaEventRecord(c.kev[1], s));
+    uint32_t h[2] = {0, 0};
+    PLAN_CUDA(cudaMemcpyAsync(h, redo.n, 8, cudaMemcpyDeviceToHost, s));
     PLAN_CUDA(cudaStreamSynchronize(s));
     float kms = 0;
     cudaEventElapsedTime(&kms, c.kev[0], c.kev[1]);
-    c.stage_ms[20] = kms;  // the FP32-filtered density kernel alone
-    c.counters[17] = h;
-    if (!h) return kOk;
-    return launch_by_k(k, [&](auto km, int threads) {
-        constexpr int KM = decltype(km)::value;
-        size_t sm = (size_t)KM * threads * 12;
-        auto kern = spl ? k_density_list<KM, 1> : k_density_list<KM, 0>;
-        kern<<<grid_for(h, threads), threads, sm, s>>>(t, redo, h, k, fpo3, sc, c.tree.dens, c.d_err);
-        c.launches++;
-        PLAN_CUDA(cudaGetLastError());
-        return (int)kOk;
-    });
+    c.stage_ms[20] = kms;  // the density kernels
+    c.counters[17] = h[0] + h[1];
+    c.scratch.used = mark;
+    return kOk;
 }
 
 int launch_densest(Context &c, const plan_params &p, uint32_t k, double threshold, uint32_t *densest, cudaStream_t s) {
+    if (k > 64) return kErrUnsupported;
     KTree t = ktree_of(c.tree);
     int rc = ensure_split(c, s);
     if (rc) return rc;
     FTree f{c.tree.phi, c.tree.plo, c.tree.nhi, c.tree.nlo};
     const uint32_t n = c.tree.Tu;
-    uint32_t *redo = c.scratch.get<uint32_t>(n + 1), *nredo = c.scratch.get<uint32_t>(4);
-    if (!redo || !nredo) return kErrOutOfMemory;
-    PLAN_CUDA(cudaMemsetAsync(nredo, 0, 4, s));
-    rc = launch_by_cap(k, [&](auto capc) {
-        constexpr int CAP = decltype(capc)::value;
-        size_t sm = (size_t)CAP * 128 * 8;
-        if (sm > 48 * 1024) PLAN_CUDA(cudaFuncSetAttribute(k_densest_f<CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        PLAN_CUDA(cudaEventRecord(c.kev[0], s));
-        k_densest_f<CAP><<<grid_for(n, 128), 128, sm, s>>>(t, f, n, k, threshold, c.tree.dens, densest, redo, nredo, c.d_err);
-        PLAN_CUDA(cudaEventRecord(c.kev[1], s));
+    const size_t mark = c.scratch.used;
+    RedoLists redo;
+    rc = redo.take(c, n, s);
+    if (rc) return rc;
+    const unsigned lb = list_blocks(c);
+    PLAN_CUDA(cudaEventRecord(c.kev[0], s));
+    k_densest_w<<<(n + kWkWarps - 1) / kWkWarps, 32 * kWkWarps, 0, s>>>(t, f, n, k, threshold, c.tree.dens, densest, redo.warp, redo.n, c.d_err);
+    k_exact_w<kOpDensest><<<lb, 32 * kWkWarps, 0, s>>>(t, f, nullptr, nullptr, 0.0, redo.warp, redo.n, 0, k, 0.0, c.fs.spline,
+                                                       WkOut{c.tree.dens, densest, nullptr, redo.heap, redo.n + 1}, c.d_err);
+    c.launches += 2;
+    rc = launch_by_k(k, [&](auto km, int threads) {
+        constexpr int KM = decltype(km)::value;
+        size_t sm = (size_t)KM * threads * 12;
+        k_densest_list<KM><<<lb, threads, sm, s>>>(t, redo.heap, redo.n + 1, k, c.tree.dens, densest, c.d_err);
         c.launches++;
         PLAN_CUDA(cudaGetLastError());
         return (int)kOk;
     });
     if (rc) return rc;
-    uint32_t h = 0;
-    PLAN_CUDA(cudaMemcpyAsync(&h, nredo, 4, cudaMemcpyDeviceToHost, s));
+    PLAN_CUDA(cudaEventRecord(c.kev[1], s));
+    uint32_t h[2] = {0, 0};
+    PLAN_CUDA(cudaMemcpyAsync(h, redo.n, 8, cudaMemcpyDeviceToHost, s));
     PLAN_CUDA(cudaStreamSynchronize(s));
     float kms = 0;
     cudaEventElapsedTime(&kms, c.kev[0], c.kev[1]);
-    c.stage_ms[21] = kms;  // the FP32-filtered densest-neighbour kernel alone
-    c.counters[18] = h;
-    if (!h) return kOk;
-    return launch_by_k(k, [&](auto km, int threads) {
-        constexpr int KM = decltype(km)::value;
-        size_t sm = (size_t)KM * threads * 12;
-        k_densest_list<KM><<<grid_for(h, threads), threads, sm, s>>>(t, redo, h, k, threshold, c.tree.dens, densest, c.d_err);
-        c.launches++;
-        PLAN_CUDA(cudaGetLastError());
-        return (int)kOk;
-    });
+    c.stage_ms[21] = kms;  // the densest-neighbour kernels
+    c.counters[18] = h[0] + h[1];
+    c.scratch.used = mark;
+    return kOk;
 }
 
 int launch_density_at(Context &c, const double *d_q3, const double *d_est, uint32_t nq, uint32_t k, double *d_out, cudaStream_t s) {
@@ -507,67 +508,70 @@ int launch_density_at(Context &c, const double *d_q3, const double *d_est, uint3
     KTree t = ktree_of(c.tree);
     const double fpo3 = 3.14159265358979323846 * 4. / 3.;
     const bool spl = !c.fs.median_kernel;
+    int rc = ensure_split(c, s);
+    if (rc) return rc;
+    FTree f{c.tree.phi, c.tree.plo, c.tree.nhi, c.tree.nlo};
     const size_t mark = c.scratch.used;
-    uint32_t *redo = c.scratch.get<uint32_t>(nq + 1), *nredo = c.scratch.get<uint32_t>(4);
-    if (!redo || !nredo) {
+    uint32_t *heap = c.scratch.get<uint32_t>(nq + 1), *nheap = c.scratch.get<uint32_t>(4);
+    if (!heap || !nheap) {
         c.scratch.used = mark;
         return kErrOutOfMemory;
     }
-    PLAN_CUDA(cudaMemsetAsync(nredo, 0, 4, s));
+    PLAN_CUDA(cudaMemsetAsync(nheap, 0, 4, s));
     // a warp per query; the queries with distance ties go to the exact heap path
-    int rc = launch_by_k(k, [&](auto km, int) {
+    rc = launch_by_k(k, [&](auto km, int threads) {
         constexpr int KM = decltype(km)::value;
-        auto kern = spl ? k_density_at_w<KM, 1> : k_density_at_w<KM, 0>;
-        kern<<<(nq + 3) / 4, 128, 0, s>>>(t, d_q3, d_est, nq, k, fpo3, c.fs.spline, d_out, redo, nredo, c.d_err);
-        c.launches++;
+        auto kern = spl ? k_exact_w<kOpSpline> : k_exact_w<kOpMedian>;
+        kern<<<(nq + kWkWarps - 1) / kWkWarps, 32 * kWkWarps, 0, s>>>(t, f, d_q3, d_est, 0.0, nullptr, nullptr, nq, k, fpo3, c.fs.spline,
+                                                                    WkOut{d_out, nullptr, nullptr, heap, nheap}, c.d_err);
+        size_t sm = (size_t)KM * threads * 12;
+        auto list = spl ? k_density_at<KM, 1> : k_density_at<KM, 0>;
+        list<<<list_blocks(c), threads, sm, s>>>(t, d_q3, d_est, heap, nheap, k, fpo3, c.fs.spline, d_out, c.d_err);
+        c.launches += 2;
         PLAN_CUDA(cudaGetLastError());
         return (int)kOk;
     });
     uint32_t h = 0;
     if (!rc) {
-        PLAN_CUDA(cudaMemcpyAsync(&h, nredo, 4, cudaMemcpyDeviceToHost, s));
-        PLAN_CUDA(cudaStreamSynchronize(s));
+        PLAN_CUDA(cudaMemcpyAsync(&h, nheap, 4, cudaMemcpyDeviceToHost, s));
+        PLAN_CUDA(cudaStreamSynchronize(s));  // the list is scratch, released here
         c.counters[27] += h;
     }
-    if (!rc && h)
-        rc = launch_by_k(k, [&](auto km, int threads) {
-            constexpr int KM = decltype(km)::value;
-            size_t sm = (size_t)KM * threads * 12;
-            auto kern = spl ? k_density_at<KM, 1> : k_density_at<KM, 0>;
-            kern<<<grid_for(h, threads), threads, sm, s>>>(t, d_q3, d_est, redo, h, k, fpo3, c.fs.spline, d_out, c.d_err);
-            c.launches++;
-            PLAN_CUDA(cudaGetLastError());
-            return (int)kOk;
-        });
-    if (h) PLAN_CUDA(cudaStreamSynchronize(s));  // the redo list is scratch, released here
     c.scratch.used = mark;
     return rc;
 }
 
 int knn_positions(Context &c, const double *pos3, uint32_t nq, uint32_t k, double est, uint32_t *idx, double *dr2) {
     if (!c.tree.Tu || k == 0 || k > c.tree.Tu) return kErrArgument;
+    if (k > 128) return kErrUnsupported;
+    if (nq == 0) return kOk;
     cudaStream_t s = c.stream;
-    double *d_q = nullptr, *d_d = nullptr;
-    uint32_t *d_i = nullptr;
-    PLAN_CUDA(cudaMallocAsync(&d_q, (size_t)nq * 3 * 8, s));
-    PLAN_CUDA(cudaMallocAsync(&d_d, (size_t)nq * k * 8, s));
-    PLAN_CUDA(cudaMallocAsync(&d_i, (size_t)nq * k * 4, s));
-    PLAN_CUDA(cudaMemcpyAsync(d_q, pos3, (size_t)nq * 3 * 8, cudaMemcpyHostToDevice, s));
+    int rc = ensure_split(c, s);
+    if (rc) return rc;
+    StreamBuf<double> d_q(s), d_d(s);
+    StreamBuf<uint32_t> d_i(s), d_redo(s);
+    PLAN_CUDA(d_q.alloc((size_t)nq * 3));
+    PLAN_CUDA(d_d.alloc((size_t)nq * k));
+    PLAN_CUDA(d_i.alloc((size_t)nq * k));
+    PLAN_CUDA(d_redo.alloc((size_t)nq + 1));
+    PLAN_CUDA(cudaMemsetAsync(d_redo.p, 0, 4, s));
+    PLAN_CUDA(cudaMemcpyAsync(d_q.p, pos3, (size_t)nq * 3 * 8, cudaMemcpyHostToDevice, s));
     KTree t = ktree_of(c.tree);
-    int rc = launch_by_k(k, [&](auto km, int threads) {
+    FTree f{c.tree.phi, c.tree.plo, c.tree.nhi, c.tree.nlo};
+    rc = launch_by_k(k, [&](auto km, int threads) {
         constexpr int KM = decltype(km)::value;
+        k_exact_w<kOpKnn><<<(nq + kWkWarps - 1) / kWkWarps, 32 * kWkWarps, 0, s>>>(t, f, d_q.p, nullptr, est, nullptr, nullptr, nq, k, 0.0,
+                                                                                c.fs.spline, WkOut{nullptr, d_i.p, d_d.p, d_redo.p + 1, d_redo.p},
+                                                                                c.d_err);
         size_t sm = (size_t)KM * threads * 12;
-        k_knn_positions<KM><<<grid_for(nq, threads), threads, sm, s>>>(t, d_q, nq, k, est, d_i, d_d, c.d_err);
-        c.launches++;
+        k_knn_positions<KM><<<list_blocks(c), threads, sm, s>>>(t, d_q.p, d_redo.p + 1, d_redo.p, k, est, d_i.p, d_d.p, c.d_err);
+        c.launches += 2;
         PLAN_CUDA(cudaGetLastError());
         return (int)kOk;
     });
     if (rc) return rc;
-    PLAN_CUDA(cudaMemcpyAsync(idx, d_i, (size_t)nq * k * 4, cudaMemcpyDeviceToHost, s));
-    PLAN_CUDA(cudaMemcpyAsync(dr2, d_d, (size_t)nq * k * 8, cudaMemcpyDeviceToHost, s));
-    PLAN_CUDA(cudaFreeAsync(d_q, s));
-    PLAN_CUDA(cudaFreeAsync(d_d, s));
-    PLAN_CUDA(cudaFreeAsync(d_i, s));
+    PLAN_CUDA(cudaMemcpyAsync(idx, d_i.p, (size_t)nq * k * 4, cudaMemcpyDeviceToHost, s));
+    PLAN_CUDA(cudaMemcpyAsync(dr2, d_d.p, (size_t)nq * k * 8, cudaMemcpyDeviceToHost, s));
     PLAN_CUDA(cudaStreamSynchronize(s));
     return kOk;
 }

@@ -76,96 +76,6 @@ __device__ __forceinline__ int f_intersects(const float4 nh, const float4 nl, co
     return in == 1 ? 0 : 1;
 }
 
-// The reference's recursion with FP32 node classification; returns false if any
-// classification was unsure (the caller then takes the FP64 path).
-template <class Visit>
-__device__ __forceinline__ bool f_traverse(const KTree &t, const FTree &f, const float4 qh, const float4 ql, float r, Visit visit,
-                                           unsigned *err) {
-    uint32_t node = 0;
-    for (uint32_t guard = 0; guard < 4u * t.nodes + 8u; ++guard) {
-        if (node >= t.nodes) {
-            atomicOr(err, (unsigned)kDevErrBadNode);
-            return false;
-        }
-        const float4 nh = f.nhi[node], nl = f.nlo[node];
-        bool down = false;
-        int cont = f_contained(nh, nl, qh, ql, r);
-        if (cont < 0) return false;
-        if (cont) {
-            if (!visit(t.nbeg[node], t.nend[node])) return true;
-        } else {
-            int inter = f_intersects(nh, nl, qh, ql, r);
-            if (inter < 0) return false;
-            if (inter) {
-                if (t.nnd[node] == 0) {
-                    if (!visit(t.nbeg[node], t.nend[node])) return true;
-                } else {
-                    down = true;
-                }
-            }
-        }
-        if (down) {
-            node = t.nfd[node];
-            continue;
-        }
-        while (node != 0) {
-            uint32_t p = t.npar[node];
-            if (node + 1 < t.nfd[p] + t.nnd[p]) {
-                node = node + 1;
-                break;
-            }
-            node = p;
-        }
-        if (node == 0) return true;
-    }
-    atomicOr(err, (unsigned)kDevErrLoopLimit);
-    return false;
-}
-
-// Max-heap of FP32 keys (approximate distances) with candidate indices, strided slab.
-struct FHeap {
-    float *k;
-    uint32_t *ix;
-    int stride;
-    __device__ float kget(int j) const { return k[j * stride]; }
-    __device__ void put(int j, float v, uint32_t i) { k[j * stride] = v; ix[j * stride] = i; }
-    __device__ void sift_up(int j) {
-        float v = kget(j);
-        uint32_t vi = ix[j * stride];
-        while (j > 0) {
-            int p = (j - 1) / 2;
-            if (!(kget(p) < v)) break;
-            put(j, kget(p), ix[p * stride]);
-            j = p;
-        }
-        put(j, v, vi);
-    }
-    __device__ void sift_down(int j, int len) {
-        float v = kget(j);
-        uint32_t vi = ix[j * stride];
-        for (;;) {
-            int c = 2 * j + 1;
-            if (c >= len) break;
-            if (c + 1 < len && kget(c) < kget(c + 1)) ++c;
-            if (!(v < kget(c))) break;
-            put(j, kget(c), ix[c * stride]);
-            j = c;
-        }
-        put(j, v, vi);
-    }
-    // keep the `cap` smallest keys
-    __device__ void add(int &size, int cap, float v, uint32_t i) {
-        if (size < cap) {
-            put(size, v, i);
-            sift_up(size);
-            ++size;
-        } else if (v < kget(0)) {
-            put(0, v, i);
-            sift_down(0, size);
-        }
-    }
-};
-
 __device__ __forceinline__ float f_dr2(const float4 qh, const float4 ql, const float4 ph, const float4 pl) {
     float dx = f_diff(qh.x, ql.x, ph.x, pl.x), dy = f_diff(qh.y, ql.y, ph.y, pl.y), dz = f_diff(qh.z, ql.z, ph.z, pl.z);
     return dx * dx + dy * dy + dz * dz;
@@ -174,81 +84,5 @@ __device__ __forceinline__ float f_dr2(const float4 qh, const float4 ql, const f
 // Upper/lower bounds of the FP64 distance given the FP32 one.
 __device__ __forceinline__ float f_hi(float v) { return v * (1.f + kRel) + 1e-24f; }
 __device__ __forceinline__ float f_lo(float v) { return v * (1.f - kRel) - 1e-24f; }
-
-// Exact k-nearest of the reference for one query through the FP32 filter, in two parts.
-// knn_collect_f32 walks the tree in FP32 and leaves the candidates in ascending FP32 order in
-// the heap slab; it returns how many of them could belong to the k nearest (z), or -1 when
-// the query must take the exact FP64 path. knn_exact_f32 then takes their exact FP64
-// distances. The callers let the warp reconverge between the two (the walks of a warp's
-// queries diverge; the FP64 part, whose instructions cost the same for one lane as for 32,
-// then runs for all lanes at once).
-// Slab layout per thread: cap = k + slack entries of (float key, u32 idx) and of (double, u32).
-__device__ inline int knn_collect_f32(const KTree &t, const FTree &f, uint32_t qi, double r, uint32_t k, int cap, FHeap &fh, unsigned *err) {
-    const float4 qh = f.phi[qi], ql = f.plo[qi];
-    // radius doubling with count-only passes
-    for (int it = 0; it < 200; ++it) {
-        uint32_t cnt = 0;
-        bool ok = f_traverse(t, f, qh, ql, (float)r, [&](uint32_t b, uint32_t e) { cnt += e - b; return cnt < k; }, err);
-        if (!ok) return -1;
-        if ((float)r != (float)r || r > 1e30) return -1;
-        if (cnt >= k) break;
-        r = r * 2;
-        if (it == 199) return -1;
-    }
-    // the float radius must order exactly like the double one in every test above; tests
-    // carry their own margins, but a radius that is not representable to 2^-24 is fine
-    // because kRel covers its rounding
-    int size = 0;
-    uint32_t visited = 0;
-    bool ok = f_traverse(t, f, qh, ql, (float)r,
-                         [&](uint32_t b, uint32_t e) {
-                             for (uint32_t p = b; p < e; ++p) fh.add(size, cap, f_dr2(qh, ql, f.phi[p], f.plo[p]), p);
-                             visited += e - b;
-                             return true;
-                         },
-                         err);
-    if (!ok || visited < k) return -1;
-    // heap -> ascending FP32 order
-    for (int len = size; len > 1; --len) {
-        float v = fh.kget(0);
-        uint32_t vi = fh.ix[0];
-        fh.put(0, fh.kget(len - 1), fh.ix[(len - 1) * fh.stride]);
-        fh.put(len - 1, v, vi);
-        fh.sift_down(0, len - 1);
-    }
-    const float thr = f_hi(fh.kget(k - 1));  // >= the k-th smallest exact distance
-    if ((int)visited > size && !(f_lo(fh.kget(size - 1)) > thr)) return -1;  // buffer might miss candidates
-    int z = 0;
-    while (z < size && !(f_lo(fh.kget(z)) > thr)) ++z;
-    return z;
-}
-
-// The second part: fills d64/i64 (ascending exact dr2, the reference's k-set) from the z
-// candidates and returns k, or -1 on a tie the library heap order decides.
-__device__ inline int knn_exact_f32(const KTree &t, double qx, double qy, double qz, uint32_t k, int z, const FHeap &fh, double *d64,
-                                    uint32_t *i64) {
-    const int dstride = 1;
-    // exact FP64 distances for every possible member, insertion-sorted by (dr2, index)
-    for (int j = 0; j < z; ++j) {
-        uint32_t p = fh.ix[j * fh.stride];
-        double v = point_dr2(qx, qy, qz, t.pos[p]);
-        int m = j;
-        while (m > 0) {
-            double pv = d64[(m - 1) * dstride];
-            uint32_t pi = i64[(m - 1) * dstride];
-            if (pv < v || (pv == v && pi < p)) break;
-            d64[m * dstride] = pv;
-            i64[m * dstride] = pi;
-            --m;
-        }
-        d64[m * dstride] = v;
-        i64[m * dstride] = p;
-    }
-    // a tie at the k-boundary or inside the k-set is resolved by the library heap order of
-    // the reference: leave those queries to the exact path
-    for (int j = 1; j < (int)k + (z > (int)k ? 1 : 0); ++j)
-        if (d64[(j - 1) * dstride] == d64[j * dstride]) return -1;
-    return (int)k;
-}
 
 }  // namespace plan
