@@ -26,9 +26,8 @@
 //  * SortParticles: the seven member sums in member order (ordered_sum_chunk over per-point
 //    products m, m x, ..., m vz formed once per snapshot, 256 members at a time, the next
 //    ones staged meanwhile), the centre of mass and the Hill radius,
-//    squared distances, and a stable sort by squared distance (in shared memory up to
-//    kRbSmall members, else a block radix sort on the leading bits and an exact fix-up of
-//    equal keys). Squared distances order members as distances do, except that two
+//    squared distances, and a stable sort by squared distance (a block radix sort on the
+//    leading bits and an exact fix-up of equal keys; in shared memory up to kRbSmall members). Squared distances order members as distances do, except that two
 //    squared distances may round to one distance: neighbours within a few ulps are compared
 //    through their square roots, and a tie goes to the library-order replay exactly as in
 //    the round kernels. The square roots of the last sort are taken when the loop ends.
@@ -38,24 +37,23 @@ constexpr int kRB = 512;                      // threads of a rebinding block
 constexpr int kRbWarps = kRB / 32;
 constexpr uint32_t kRbFront = 4096;           // frontier entries of the ball search
 constexpr uint32_t kRbSmall = 4096;           // members sorted in shared memory
+constexpr uint32_t kRbOnePass = 512;          // members sorted by one digit
 constexpr uint32_t kWaitLimit = 1u << 25;     // bounded waits on blockers: sleeps of 1 us per 2^24 points
 constexpr uint32_t kCallLimit = 1u << 20;     // calls of one clump in one launch
 constexpr int kRbStats = 40;                  // counters per slot
 constexpr int kCk = 24;                       // checkpoints per clump and run
-// dynamic shared memory: the largest of the frontier, the small sort and the acceptance
-// tile (per candidate: FP64 position and velocity, index, FP32 form)
-constexpr size_t kRbTileBytes = (size_t)kRB * (64 + 4 + sizeof(CandF));
-constexpr size_t kRbSmem14 = 14 * (kRbFront > kRbSmall ? kRbFront : kRbSmall);
 // digit of the member sort: two passes order 22 bits of the squared distances' range, which
-// leaves runs of one or two members to the insertion sort; the counters are the largest use of
-// the dynamic shared memory
+// leaves runs of one or two members to the insertion sort
 constexpr uint32_t kRbDigit = 11;
-constexpr size_t kRbRadixBytes = ((size_t)kRbWarps << kRbDigit) * 4;
-constexpr size_t kRbSmemMost = kRbSmem14 > kRbTileBytes ? kRbSmem14 : kRbTileBytes;
-constexpr size_t kRbSmem = kRbRadixBytes > kRbSmemMost ? kRbRadixBytes : kRbSmemMost;
+constexpr size_t kRbRadixBytes = ((size_t)kRbWarps << kRbDigit) * 4;  // a counter per digit and warp
+// dynamic shared memory, reused by every phase: the frontier, the acceptance tile (per
+// candidate: FP64 position and velocity, index, FP32 form), the stage of the sums, and the
+// largest, the sort's counters with the keys and positions of a small clump
+constexpr size_t kRbTileBytes = (size_t)kRB * (64 + 4 + sizeof(CandF));
+constexpr size_t kRbSmem = kRbRadixBytes + (size_t)kRbSmall * 16;
 static_assert(kRbFront * 14 <= kRbSmem, "frontier");
 static_assert(kRbTileBytes <= kRbSmem, "acceptance tile");
-static_assert(kRbSmall * 14 <= kRbSmem, "small sort");
+static_assert(kRbSmall * 12 <= kRbRadixBytes, "the sorted members over the counters");
 
 // Checkpoints of the clumps' runs, by key rank: after the calls ck_after() selects, the
 // sorted member list (index, squared distance) and the state (M, centre, velocity, Hill
@@ -210,7 +208,51 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
     __syncthreads();
     const BallQ ball = make_ball(sh.st[1], sh.st[2], sh.st[3], sh.st[7]);
     const KTree &t = a.t;
-    // 1) breadth-first frontier (classes 1..4; 0 = not yet classified)
+    // 1) breadth-first frontier (classes 1..4; 0 = not yet classified): the levels of at most 32
+    // entries by warp 0 alone, without block barriers (a level costs it the latency of its node
+    // loads; a level of the whole block costs six barriers and a scan on top)
+    if (wid == 0) {
+        uint32_t nf = 1, node = 0;
+        int cls = 0;
+        for (int level = 0; level < 40; ++level) {
+            if ((uint32_t)lane < nf && cls == 0) {
+                if (node >= t.nodes) {
+                    atomicOr(a.err, (unsigned)kDevErrBadNode);
+                    cls = 3;
+                } else {
+                    uint32_t eb, ee;
+                    cls = ball_class(t, a.ft, a.epos, node, ball, eb, ee);
+                }
+            }
+            const bool down = (uint32_t)lane < nf && cls == 4;
+            if (!__any_sync(0xffffffffu, down)) break;
+            const uint32_t c0 = down ? t.nfd[node] : 0u, n = (uint32_t)lane >= nf || cls == 3 ? 0u : (down ? t.nnd[node] : 1u);
+            uint32_t incl = n;
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t o = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += o;
+            }
+            const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+            if (total > 32) break;
+            for (uint32_t c = 0; c < n; ++c) {
+                front2[incl - n + c] = down ? c0 + c : node;
+                fcls2[incl - n + c] = down ? 0 : (uint8_t)cls;
+            }
+            __syncwarp();
+            nf = total;
+            if ((uint32_t)lane < nf) {
+                node = front2[lane];
+                cls = fcls2[lane];
+            }
+            __syncwarp();
+        }
+        if ((uint32_t)lane < nf) {
+            front[lane] = node;
+            fcls[lane] = (uint8_t)cls;
+        }
+        if (lane == 0) s_nf = nf;
+    }
+    __syncthreads();
     for (int level = 0; level < 40; ++level) {
         const uint32_t nf = s_nf;
         if (tid == 0) s_expand = 0;
@@ -719,6 +761,28 @@ __device__ int rb_radix(uint32_t *ki, uint32_t *vi, uint32_t *ko, uint32_t *vo, 
     return where;
 }
 
+// runs of equal keys: insertion sort by the full squared distance (stable), a thread per run
+__device__ __forceinline__ void rb_fix_runs(const uint32_t *ks, double *dist, uint32_t *idx, uint32_t m) {
+    for (uint32_t k = threadIdx.x; k + 1 < m; k += kRB) {
+        if ((k == 0 || ks[k] != ks[k - 1]) && ks[k + 1] == ks[k]) {
+            uint32_t e = k + 1;
+            while (e < m && ks[e] == ks[k]) ++e;
+            for (uint32_t i = k + 1; i < e; ++i) {
+                const double dv = dist[i];
+                const uint32_t iv = idx[i];
+                uint32_t j = i;
+                while (j > k && dist[j - 1] > dv) {
+                    dist[j] = dist[j - 1];
+                    idx[j] = idx[j - 1];
+                    --j;
+                }
+                dist[j] = dv;
+                idx[j] = iv;
+            }
+        }
+    }
+}
+
 // any two neighbours of a sorted run of squared distances whose square roots are equal
 __device__ __forceinline__ bool rb_sqrt_tie(double s0, double s1) {
     if (s0 == s1) return true;
@@ -852,53 +916,41 @@ __device__ bool rb_sort_particles(const RbArgs &a, uint32_t slot, RbShared &sh, 
     }
     const long long t_dist = clock64();
     bool ok = true;
+    // the keys of the sort: the leading bits of the range above the smallest
+    const uint32_t range = 32u - (uint32_t)__clz((int)(kmax - kmin));
     if (m <= kRbSmall) {
-        // 3a) in shared memory: bitonic sort by (squared distance, position)
-        unsigned long long *sk = reinterpret_cast<unsigned long long *>(sh.buf);
-        uint32_t *si = reinterpret_cast<uint32_t *>(sk + kRbSmall);
-        uint16_t *sp = reinterpret_cast<uint16_t *>(si + kRbSmall);
-        uint32_t n2 = 1;
-        while (n2 < m) n2 <<= 1;
-        for (uint32_t k = tid; k < n2; k += kRB) {
-            if (k < m) {
-                sk[k] = (unsigned long long)__double_as_longlong(dist[k]);
-                si[k] = idx[k];
-                sp[k] = (uint16_t)k;
-            } else {
-                sk[k] = ~0ull;
-                si[k] = kNone;
-                sp[k] = 0xffff;
-            }
+        // 3a) in shared memory, behind the counters: the keys and positions, then (over the
+        // counters) the members in order. Up to kRbOnePass members one digit is enough: over some
+        // 64 octaves it leaves runs of a few equal keys to the insertion sort.
+        const uint32_t most = m <= kRbOnePass && range <= 26 ? kRbDigit : 2 * kRbDigit, drop = range > most ? range - most : 0u;
+        uint32_t *kx = reinterpret_cast<uint32_t *>(sh.buf + kRbRadixBytes), *ky = kx + kRbSmall, *vx = ky + kRbSmall, *vy = vx + kRbSmall;
+        for (uint32_t k = tid; k < m; k += kRB) {
+            kx[k] = ((uint32_t)(dbits(dist[k]) >> 32) - kmin) >> drop;
+            vx[k] = k;  // what a range of no bits keeps
         }
         __syncthreads();
-        for (uint32_t size = 2; size <= n2; size <<= 1) {
-            for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-                for (uint32_t k = tid; k < n2; k += kRB) {
-                    const uint32_t j = k ^ stride;
-                    if (j > k) {
-                        const bool up = (k & size) == 0;
-                        const bool gt = sk[k] > sk[j] || (sk[k] == sk[j] && sp[k] > sp[j]);
-                        if (gt == up) {
-                            const unsigned long long tk = sk[k]; sk[k] = sk[j]; sk[j] = tk;
-                            const uint32_t ti = si[k]; si[k] = si[j]; si[j] = ti;
-                            const uint16_t tp = sp[k]; sp[k] = sp[j]; sp[j] = tp;
-                        }
-                    }
-                }
-                __syncthreads();
-            }
+        const int where = rb_radix(kx, vx, ky, vy, m, range - drop, reinterpret_cast<uint32_t *>(sh.buf), sh.warp_tot);
+        const uint32_t *ks = where ? ky : kx, *vs = where ? vy : vx;
+        double *sd = reinterpret_cast<double *>(sh.buf);
+        uint32_t *si = reinterpret_cast<uint32_t *>(sd + kRbSmall);
+        for (uint32_t k = tid; k < m; k += kRB) {
+            const uint32_t src = vs[k];
+            si[k] = idx[src];
+            sd[k] = dist[src];
         }
+        __syncthreads();
+        rb_fix_runs(ks, sd, si, m);
+        __syncthreads();
         // (every size: below 17 members the library's insertion sort is stable by distance,
         // which an order by squared distance only equals when no two roots tie)
         int tie = 0;
-        for (uint32_t k = tid + 1; k < m; k += kRB)
-            tie |= rb_sqrt_tie(__longlong_as_double((long long)sk[k - 1]), __longlong_as_double((long long)sk[k]));
+        for (uint32_t k = tid + 1; k < m; k += kRB) tie |= rb_sqrt_tie(sd[k - 1], sd[k]);
         if (__syncthreads_or(tie)) {
             if (tid == 0) s_tie = 1;
         } else {
             for (uint32_t k = tid; k < m; k += kRB) {
                 idx[k] = si[k];
-                dist[k] = __longlong_as_double((long long)sk[k]);
+                dist[k] = sd[k];
             }
         }
         __syncthreads();
@@ -914,13 +966,13 @@ __device__ bool rb_sort_particles(const RbArgs &a, uint32_t slot, RbShared &sh, 
         } else {
             uint32_t *kx = a.P.idx + r + m, *ky = a.P.idx + r + 2 * m;
             uint32_t *vx = reinterpret_cast<uint32_t *>(a.P.dist + r + m), *vy = reinterpret_cast<uint32_t *>(a.P.dist + r + 2 * m);
-            const uint32_t bits = 32u - (uint32_t)__clz((int)(kmax - kmin)), drop = bits > 2 * kRbDigit ? bits - 2 * kRbDigit : 0u;
+            const uint32_t drop = range > 2 * kRbDigit ? range - 2 * kRbDigit : 0u;
             for (uint32_t k = tid; k < m; k += kRB) {
                 kx[k] = ((uint32_t)(dbits(dist[k]) >> 32) - kmin) >> drop;
                 vx[k] = k;  // what a range of no bits keeps
             }
             __syncthreads();
-            const int where = rb_radix(kx, vx, ky, vy, m, bits - drop, reinterpret_cast<uint32_t *>(sh.buf), sh.warp_tot);
+            const int where = rb_radix(kx, vx, ky, vy, m, range - drop, reinterpret_cast<uint32_t *>(sh.buf), sh.warp_tot);
             const uint32_t *ks = where ? ky : kx, *vs = where ? vy : vx;
             uint32_t *didx = a.P.idx + r;
             double *ddist = a.P.dist + r;
@@ -930,25 +982,7 @@ __device__ bool rb_sort_particles(const RbArgs &a, uint32_t slot, RbShared &sh, 
                 ddist[k] = dist[src];
             }
             __syncthreads();
-            // runs of equal keys: insertion sort by the full squared distance (stable)
-            for (uint32_t k = tid; k < m; k += kRB) {
-                if ((k == 0 || ks[k] != ks[k - 1]) && k + 1 < m && ks[k + 1] == ks[k]) {
-                    uint32_t e = k + 1;
-                    while (e < m && ks[e] == ks[k]) ++e;
-                    for (uint32_t i = k + 1; i < e; ++i) {
-                        const double dv = ddist[i];
-                        const uint32_t iv = didx[i];
-                        uint32_t j = i;
-                        while (j > k && ddist[j - 1] > dv) {
-                            ddist[j] = ddist[j - 1];
-                            didx[j] = didx[j - 1];
-                            --j;
-                        }
-                        ddist[j] = dv;
-                        didx[j] = iv;
-                    }
-                }
-            }
+            rb_fix_runs(ks, ddist, didx, m);
             __syncthreads();
             int tie = 0;
             for (uint32_t k = tid + 1; k < m; k += kRB) tie |= rb_sqrt_tie(ddist[k - 1], ddist[k]);
