@@ -2525,8 +2525,13 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
         unsigned long long *d_rstats = trace.on ? A.get<unsigned long long>((size_t)kRbStats * nb) : nullptr;
         double4_32a *tm0 = use_rounds ? nullptr : A.get<double4_32a>(Tu), *tm1 = use_rounds ? nullptr : A.get<double4_32a>(Tu);
         if (A.failed) return kErrOutOfMemory;
+        RbSeg *d_seg = use_rounds ? nullptr : A.get<RbSeg>(nb);
+        uint2 *enode = use_rounds ? nullptr : A.get<uint2>(kt.nodes);
+        if (A.failed) return kErrOutOfMemory;
         int rb_grid = 1;
         if (!use_rounds) {
+            k_node_slices<<<grid_for(kt.nodes, 256), 256, 0, s>>>(kt.nodes, kt.nbeg, kt.nend, epos, enode);
+            c.launches++;
             k_member_terms<<<grid_for(Tu, 256), 256, 0, s>>>(Tu, tr.pos, tr.vel, tm0, tm1);
             c.launches++;
             PLAN_CUDA(cudaMemsetAsync(d_needsort, 0, nb, s));
@@ -2596,6 +2601,7 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
                 for (uint32_t sl : todo) fin[sl] = 0;
                 PLAN_CUDA(cudaMemcpyAsync(d_fin, fin.data(), nb, cudaMemcpyHostToDevice, s));
                 PLAN_CUDA(cudaMemsetAsync(d_head, 0, 4, s));
+                PLAN_CUDA(cudaMemsetAsync(d_seg, 0, nb * sizeof(RbSeg), s));
                 int r = st.up_list(todo, st.d_list);
                 if (r) return r;
                 Arena &S = c.scratch;
@@ -2633,7 +2639,8 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
                 ra.tm0 = tm0;
                 ra.tm1 = tm1;
                 ra.E = E;
-                ra.epos = epos;
+                ra.enode = enode;
+                ra.seg = d_seg;
                 ra.owner = owner;
                 ra.rank_of = rank_of;
                 ra.slot_of_rank = slot_of_rank;
@@ -2868,8 +2875,8 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
                                      (unsigned)pass, active_all.size(), calls, acc, w[0], w[13], w[1], w[2], w[12], w[10], w[3] / 1000, w[4] / 1000,
                                      w[14] / 1000, w[15], w[16] / 1000, w[5] / 1000, w[6] / 1000, w[8] / 1000, w[9] / 1000, w[7], w[11]);
                         for (int q = 0; q < 7; ++q) std::fprintf(stderr, " %llu/%llu", w[17 + q], w[24 + q] / 1000);
-                        std::fprintf(stderr, " | tiles %llu set-up kcycles %llu; predicted %llu held %llu taken %llu\n", w[32], w[31] / 1000, w[33],
-                                     w[34], w[35]);
+                        std::fprintf(stderr, " | tiles %llu set-up kcycles %llu; predicted %llu held %llu taken %llu; frontier kcycles %llu slices %llu entries %llu\n", w[32], w[31] / 1000, w[33],
+                                     w[34], w[35], w[36] / 1000, w[37] / 1000, w[38]);
                     }
                 }
             }

@@ -75,6 +75,15 @@ __host__ __device__ inline bool ck_after(uint32_t j) {
     return j % 3 == 0 && ((j / 3) & (j / 3 - 1)) == 0;
 }
 
+// A clump's room in the member pool besides its members: the capacity of its present segment
+// (0 where the host packed it), the segment it left last and the sort buffers. Calls go back and
+// forth between two segments that grow by half, so a launch needs a few times the members
+// instead of a segment per call, and the pool does not fill up: a launch that stops for a
+// compaction costs the blocks that wait for one another their order.
+struct RbSeg {
+    uint32_t cap, spare, spare_cap, buf, buf_cap;
+};
+
 struct RbArgs {
     const uint32_t *list;  // clumps of this launch, in key-rank order
     uint32_t n;
@@ -91,7 +100,8 @@ struct RbArgs {
     FTree ft;
     const double4_32a *vel;
     const double4_32a *tm0, *tm1;  // per point: (m, m x, m y, m z), (m vx, m vy, m vz, 0)
-    const uint32_t *E, *epos;
+    const uint32_t *E;
+    const uint2 *enode;    // per node: its slice of the eligible points E
     uint32_t *owner;
     const uint32_t *rank_of, *slot_of_rank, *tent;
     uint32_t *dmax, *dset;
@@ -104,6 +114,7 @@ struct RbArgs {
     uint32_t *ccall;       // per slot: calls of the clump's run done (persists across launches)
     uint32_t *dcall, *dfirst;  // per deferral record / per slot: the earliest call that made it
     Ckpt ck;               // ck.n null: no checkpoints
+    RbSeg *seg;            // per slot, zero at the start of a launch
 };
 
 // per-point products for the member sums (src/tree.hpp:4436-4440: mass, pos * mass,
@@ -166,6 +177,25 @@ __device__ uint32_t rb_scan_excl(uint32_t *a, uint32_t n, uint32_t *warp_tot) {
     return total;
 }
 
+// per node, its slice of the eligible points (epos: eligible points below a point)
+__global__ void k_node_slices(uint32_t nodes, const uint32_t *nbeg, const uint32_t *nend, const uint32_t *epos, uint2 *enode) {
+    const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n < nodes) enode[n] = make_uint2(epos[nbeg[n]], epos[nend[n]]);
+}
+
+// ball_class with the node's slice at hand
+__device__ __forceinline__ int rb_class(const KTree &t, const FTree &f, uint2 e, uint32_t node, const BallQ &b) {
+    const float4 nh = f.nhi[node], nl = f.nlo[node];
+    if (e.x == e.y) return 3;
+    int c = f_contained(nh, nl, b.qh, b.ql, b.rf);
+    if (c < 0) c = node_contained(t.ncf[node], b.cx, b.cy, b.cz, b.r) ? 1 : 0;
+    if (c) return 1;
+    c = f_intersects(nh, nl, b.qh, b.ql, b.rf);
+    if (c < 0) c = node_intersects(t.ncf[node], b.cx, b.cy, b.cz, b.r) ? 1 : 0;
+    if (c) return t.nnd[node] == 0 ? 2 : 4;
+    return 3;
+}
+
 struct RbShared {
     unsigned char *buf;  // kRbSmem bytes, reused by every phase
     uint32_t *warp_tot;
@@ -178,6 +208,37 @@ struct RbShared {
     double *sd;          // acceptance state in FP64: x y z vx vy vz M
 };
 
+// room for n entries, half as many on top where the pool has them (cap: what was taken)
+__device__ __forceinline__ uint32_t rb_alloc(const Pool &P, uint32_t n, uint32_t &cap) {
+    cap = n + n / 2;
+    uint32_t o = cap > n ? pool_try_alloc(P, cap) : kNone;
+    if (o == kNone) {
+        cap = n;
+        o = pool_try_alloc(P, n);
+    }
+    return o;
+}
+
+// the segment a clump left last, or a new one in its place, with room for n entries
+__device__ __forceinline__ uint32_t rb_spare(const Pool &P, RbSeg &g, uint32_t n) {
+    if (g.spare_cap >= n) return g.spare;
+    uint32_t cap;
+    const uint32_t o = rb_alloc(P, n, cap);
+    if (o != kNone) {
+        g.spare = o;
+        g.spare_cap = cap;
+    }
+    return o;
+}
+
+// the members moved from the present segment at o to the spare one
+__device__ __forceinline__ void rb_switch(RbSeg &g, uint32_t o) {
+    const uint32_t cap = g.cap;
+    g.cap = g.spare_cap;
+    g.spare = o;
+    g.spare_cap = cap;
+}
+
 // ------------------------------------------------------------------ one SearchBound call
 // Returns the number of accepted particles, or kNone when the member pool is full (nothing
 // changed).
@@ -185,7 +246,7 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     uint32_t *front = reinterpret_cast<uint32_t *>(sh.buf), *front2 = front + kRbFront, *fcnt = front2 + kRbFront;
     uint8_t *fcls = reinterpret_cast<uint8_t *>(fcnt + kRbFront), *fcls2 = fcls + kRbFront;
-    uint32_t &s_nf = sh.u[0], &s_expand = sh.u[1], &s_noff = sh.u[2], &s_nel = sh.u[3], &s_f = sh.u[4], &s_m0 = sh.u[5],
+    uint32_t &s_nf = sh.u[0], &s_noff = sh.u[2], &s_nel = sh.u[3], &s_f = sh.u[4], &s_m0 = sh.u[5],
              &s_o = sh.u[6], &s_S = sh.u[7];
     const long long t0 = clock64();
     if (tid == 0) {
@@ -196,9 +257,6 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
         sh.st[7] = a.ct.hill[slot];
         s_m0 = a.ct.mn[slot];
         s_o = a.ct.moff[slot];
-        front[0] = 0;
-        fcls[0] = 0;
-        s_nf = 1;
         s_nel = 0;
         const double4_32a c0 = a.com0[slot];  // how far this clump's balls reach from its centre before rebinding
         const double dx = c.x - c0.x, dy = c.y - c0.y, dz = c.z - c0.z;
@@ -209,8 +267,9 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
     const BallQ ball = make_ball(sh.st[1], sh.st[2], sh.st[3], sh.st[7]);
     const KTree &t = a.t;
     // 1) breadth-first frontier (classes 1..4; 0 = not yet classified): the levels of at most 32
-    // entries by warp 0 alone, without block barriers (a level costs it the latency of its node
-    // loads; a level of the whole block costs six barriers and a scan on top)
+    // entries by warp 0 alone, without block barriers; then 512 entries at a time, one per
+    // thread, from one half of the buffer to the other. A level costs the latency of its node
+    // loads, so a node's slice of eligible points is stored per node (enode).
     if (wid == 0) {
         uint32_t nf = 1, node = 0;
         int cls = 0;
@@ -220,8 +279,7 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
                     atomicOr(a.err, (unsigned)kDevErrBadNode);
                     cls = 3;
                 } else {
-                    uint32_t eb, ee;
-                    cls = ball_class(t, a.ft, a.epos, node, ball, eb, ee);
+                    cls = rb_class(t, a.ft, a.enode[node], node, ball);
                 }
             }
             const bool down = (uint32_t)lane < nf && cls == 4;
@@ -253,75 +311,72 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
         if (lane == 0) s_nf = nf;
     }
     __syncthreads();
+    uint32_t nf = s_nf;
     for (int level = 0; level < 40; ++level) {
-        const uint32_t nf = s_nf;
-        if (tid == 0) s_expand = 0;
-        __syncthreads();
-        for (uint32_t i = tid; i < nf; i += kRB) {
-            const uint32_t node = front[i];
-            int cls = fcls[i];
+        uint32_t base = 0;
+        bool expand = false, fits = true;
+        for (uint32_t i0 = 0; i0 < nf; i0 += kRB) {
+            const uint32_t i = i0 + tid, node = i < nf ? front[i] : 0u;
+            int cls = i < nf ? fcls[i] : 3;
             if (cls == 0) {
                 if (node >= t.nodes) {
                     atomicOr(a.err, (unsigned)kDevErrBadNode);
                     cls = 3;
                 } else {
-                    uint32_t eb, ee;
-                    cls = ball_class(t, a.ft, a.epos, node, ball, eb, ee);
+                    cls = rb_class(t, a.ft, a.enode[node], node, ball);
                 }
                 fcls[i] = (uint8_t)cls;
             }
-            fcnt[i] = cls == 4 ? t.nnd[node] : (cls == 3 ? 0u : 1u);
-            if (cls == 4) s_expand = 1;
-        }
-        __syncthreads();
-        if (!s_expand) break;
-        const uint32_t total = rb_scan_excl(fcnt, nf, sh.warp_tot);
-        if (total > kRbFront) break;
-        for (uint32_t i = tid; i < nf; i += kRB) {
-            const int cls = fcls[i];
-            const uint32_t o = fcnt[i];
-            if (cls == 1 || cls == 2) {
-                front2[o] = front[i];
-                fcls2[o] = (uint8_t)cls;
-            } else if (cls == 4) {
-                const uint32_t c0 = t.nfd[front[i]], nc = t.nnd[front[i]];
-                for (uint32_t c = 0; c < nc; ++c) {
-                    front2[o + c] = c0 + c;
-                    fcls2[o + c] = 0;
-                }
+            const uint32_t c0 = cls == 4 ? t.nfd[node] : 0u, n = cls == 4 ? t.nnd[node] : (cls == 3 ? 0u : 1u);
+            uint32_t incl = n;
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t o = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += o;
             }
+            if (lane == 31) sh.warp_tot[wid] = incl;
+            expand = __syncthreads_or(cls == 4) || expand;
+            uint32_t at = base + incl - n, total = 0;
+            for (int w = 0; w < kRbWarps; ++w) {
+                const uint32_t c = sh.warp_tot[w];
+                if (w < wid) at += c;
+                total += c;
+            }
+            base += total;
+            fits = fits && base <= kRbFront;
+            if (fits)
+                for (uint32_t c = 0; c < n; ++c) {
+                    front2[at + c] = cls == 4 ? c0 + c : node;
+                    fcls2[at + c] = cls == 4 ? 0 : (uint8_t)cls;
+                }
+            __syncthreads();  // the totals are read, the next step's follow
         }
-        __syncthreads();
-        for (uint32_t i = tid; i < total; i += kRB) {
-            front[i] = front2[i];
-            fcls[i] = fcls2[i];
-        }
-        if (tid == 0) s_nf = total;
-        __syncthreads();
+        if (!expand || !fits) break;  // the classes of this level are kept
+        uint32_t *f = front; front = front2; front2 = f;
+        uint8_t *g = fcls; fcls = fcls2; fcls2 = g;
+        nf = base;
     }
-    const uint32_t nf = s_nf;
+    const long long tq1 = clock64();
     // 2) each entry's slice of eligible points: its start (front2) and length (fcnt), scanned
     for (uint32_t i = tid; i < nf; i += kRB) {
-        uint32_t eb = 0, ee = 0;
+        uint2 e = make_uint2(0, 0);
         int cls = fcls[i];
         if (front[i] >= t.nodes) {
             cls = 3;
-        } else if (cls == 0) {
-            cls = ball_class(t, a.ft, a.epos, front[i], ball, eb, ee);
         } else {
-            eb = a.epos[t.nbeg[front[i]]];
-            ee = a.epos[t.nend[front[i]]];
+            e = a.enode[front[i]];
+            if (cls == 0) cls = rb_class(t, a.ft, e, front[i], ball);
         }
         fcls[i] = (uint8_t)cls;
-        front2[i] = eb;
-        fcnt[i] = cls == 3 ? 0u : ee - eb;
+        front2[i] = e.x;
+        fcnt[i] = cls == 3 ? 0u : e.y - e.x;
     }
     __syncthreads();
     const uint32_t S = rb_scan_excl(fcnt, nf, sh.warp_tot);
+    const long long tq2 = clock64();
     // 3) the new segment: the members, then room for every scanned point
     if (tid == 0) {
         s_S = S;
-        s_noff = pool_try_alloc(a.P, s_m0 + S);
+        s_noff = rb_spare(a.P, a.seg[slot], s_m0 + S);
     }
     __syncthreads();
     if (s_noff == kNone) return kNone;
@@ -652,6 +707,9 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
             stat[4] += (unsigned long long)(t2 - t1);
             stat[12] += rounds;
             stat[13] += S;
+            stat[36] += (unsigned long long)(tq1 - t0);
+            stat[37] += (unsigned long long)(tq2 - tq1);
+            stat[38] += nf;
             stat[10] += sh.u[12];
             stat[14] += sh.u[13];  // warp 0's windows: cycles, number, and cycles up to the last update
             stat[15] += sh.u[14];
@@ -663,10 +721,9 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
             stat[35] += sh.u[18];  // taken either way
         }
         if (nacc) {
+            rb_switch(a.seg[slot], o);
             a.ct.moff[slot] = no;
             a.ct.mn[slot] = m0 + nacc;
-        } else {
-            atomicCAS(a.P.top, no + m0 + S, no);  // give the segment back when nothing was taken after it
         }
     }
     __syncthreads();
@@ -795,7 +852,7 @@ __device__ __forceinline__ bool rb_sqrt_tie(double s0, double s1) {
 // false when the pool has no room for a large sort (the clump is then left with needsort).
 __device__ bool rb_sort_particles(const RbArgs &a, uint32_t slot, RbShared &sh, unsigned long long *stat) {
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    uint32_t &s_o = sh.u[8], &s_m = sh.u[9], &s_tie = sh.u[10], &s_r = sh.u[11];
+    uint32_t &s_o = sh.u[8], &s_m = sh.u[9], &s_tie = sh.u[10], &s_r = sh.u[11], &s_x = sh.u[12];
     uint32_t *s_kmin = sh.u + 20, *s_kmax = s_kmin + kRbWarps;
     const long long t0 = clock64();
     if (tid == 0) {
@@ -956,16 +1013,30 @@ __device__ bool rb_sort_particles(const RbArgs &a, uint32_t slot, RbShared &sh, 
         __syncthreads();
     } else {
         // 3b) large: radix sort by the leading 2 kRbDigit bits of the range (above the smallest),
-        // with the position as payload, into three fresh pool areas (D: the sorted segment; X,
-        // Y: sort buffers, given back after)
-        if (tid == 0) s_r = pool_try_alloc(a.P, 3 * m);
+        // with the position as payload, in the clump's sort buffers; the members then go in order
+        // to the spare segment
+        if (tid == 0) {
+            RbSeg &g = a.seg[slot];
+            s_r = rb_spare(a.P, g, m);
+            if (s_r != kNone && g.buf_cap < 2 * m) {
+                uint32_t cap;
+                const uint32_t x = rb_alloc(a.P, 2 * m, cap);
+                if (x == kNone) {
+                    s_r = kNone;
+                } else {
+                    g.buf = x;
+                    g.buf_cap = cap;
+                }
+            }
+            s_x = g.buf;
+        }
         __syncthreads();
         const uint32_t r = s_r;
         if (r == kNone) {
             ok = false;
         } else {
-            uint32_t *kx = a.P.idx + r + m, *ky = a.P.idx + r + 2 * m;
-            uint32_t *vx = reinterpret_cast<uint32_t *>(a.P.dist + r + m), *vy = reinterpret_cast<uint32_t *>(a.P.dist + r + 2 * m);
+            uint32_t *kx = a.P.idx + s_x, *ky = kx + m;
+            uint32_t *vx = reinterpret_cast<uint32_t *>(a.P.dist + s_x), *vy = vx + m;
             const uint32_t drop = range > 2 * kRbDigit ? range - 2 * kRbDigit : 0u;
             for (uint32_t k = tid; k < m; k += kRB) {
                 kx[k] = ((uint32_t)(dbits(dist[k]) >> 32) - kmin) >> drop;
@@ -989,9 +1060,9 @@ __device__ bool rb_sort_particles(const RbArgs &a, uint32_t slot, RbShared &sh, 
             if (__syncthreads_or(tie)) {
                 if (tid == 0) s_tie = 1;  // the unsorted segment at o is intact
             } else if (tid == 0) {
+                rb_switch(a.seg[slot], o);
                 a.ct.moff[slot] = r;
             }
-            if (tid == 0) atomicCAS(a.P.top, r + 3 * m, r + m);  // give X and Y back when they are on top
             __syncthreads();
         }
     }
