@@ -36,7 +36,7 @@
 constexpr int kRB = 512;                      // threads of a rebinding block
 constexpr int kRbWarps = kRB / 32;
 constexpr uint32_t kRbFront = 4096;           // frontier entries of the ball search
-constexpr uint32_t kRbSmall = 4096;           // members sorted in shared memory
+constexpr uint32_t kRbSmall = 2048;           // members sorted in shared memory
 constexpr uint32_t kRbOnePass = 512;          // members sorted by one digit
 constexpr uint32_t kWaitLimit = 1u << 25;     // bounded waits on blockers: sleeps of 1 us per 2^24 points
 constexpr uint32_t kCallLimit = 1u << 20;     // calls of one clump in one launch
@@ -48,12 +48,11 @@ constexpr uint32_t kRbDigit = 11;
 constexpr size_t kRbRadixBytes = ((size_t)kRbWarps << kRbDigit) * 4;  // a counter per digit and warp
 // dynamic shared memory, reused by every phase: the frontier, the acceptance tile (per
 // candidate: FP64 position and velocity, index, FP32 form), the stage of the sums, and the
-// largest, the sort's counters with the keys and positions of a small clump
+// largest, the sort's counters with the records and sorted pairs of a small clump
 constexpr size_t kRbTileBytes = (size_t)kRB * (64 + 4 + sizeof(CandF));
-constexpr size_t kRbSmem = kRbRadixBytes + (size_t)kRbSmall * 16;
+constexpr size_t kRbSmem = kRbRadixBytes + (size_t)kRbSmall * 28;
 static_assert(kRbFront * 14 <= kRbSmem, "frontier");
 static_assert(kRbTileBytes <= kRbSmem, "acceptance tile");
-static_assert(kRbSmall * 12 <= kRbRadixBytes, "the sorted members over the counters");
 
 // Checkpoints of the clumps' runs, by key rank: after the calls ck_after() selects, the
 // sorted member list (index, squared distance) and the state (M, centre, velocity, Hill
@@ -248,6 +247,7 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
     uint8_t *fcls = reinterpret_cast<uint8_t *>(fcnt + kRbFront), *fcls2 = fcls + kRbFront;
     uint32_t &s_nf = sh.u[0], &s_noff = sh.u[2], &s_nel = sh.u[3], &s_f = sh.u[4], &s_m0 = sh.u[5],
              &s_o = sh.u[6], &s_S = sh.u[7];
+    uint32_t *s_cnt = sh.u + 20;  // per warp, four counts
     const long long t0 = clock64();
     if (tid == 0) {
         const double4_32a c = a.ct.com[slot], v = a.ct.vcom[slot];
@@ -383,29 +383,62 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
     const uint32_t m0 = s_m0, o = s_o, no = s_noff;
     for (uint32_t k = tid; k < m0; k += kRB) a.P.idx[no + k] = a.P.idx[o + k];
     uint32_t *elig = a.P.idx + no + m0;
-    for (uint32_t base = 0; base < S; base += kRB) {
-        const uint32_t tt = base + tid;
-        bool keep = false;
-        uint32_t q = 0;
-        if (tt < S) {
-            uint32_t lo = 0, hi = nf;  // the last entry starting at or before tt
+    // 2048 points a step, four per thread with their loads on the way together: a step costs the
+    // latency of three dependent loads however many points it takes
+    constexpr int kIn = 4;
+    uint32_t found = 0;
+    for (uint32_t base = 0; base < S; base += kIn * kRB) {
+        uint32_t q[kIn], ow[kIn];
+        float v[kIn];
+        bool have[kIn], all[kIn], keep[kIn];
+#pragma unroll
+        for (int j = 0; j < kIn; ++j) {
+            const uint32_t tt = base + j * kRB + tid;
+            have[j] = tt < S;
+            uint32_t lo = 0, hi = have[j] ? nf : 0;  // the last entry starting at or before tt
             while (hi - lo > 1) {
                 const uint32_t mid = (lo + hi) >> 1;
                 if (fcnt[mid] <= tt) lo = mid;
                 else hi = mid;
             }
-            q = a.E[front2[lo] + (tt - fcnt[lo])];
-            keep = fcls[lo] == 1 || in_ball(t, a.ft, ball, q);
-            // this clump's own claims are its members: the acceptance would only skip them
-            if (keep && __ldcg(&a.owner[q]) == myrank) keep = false;
+            q[j] = have[j] ? a.E[front2[lo] + (tt - fcnt[lo])] : 0u;
+            all[j] = have[j] && fcls[lo] == 1;
         }
-        uint32_t r;
-        const uint32_t tot = rb_block_rank(keep, r, sh.warp_tot);
-        if (keep) elig[s_nel + r] = q;
+#pragma unroll
+        for (int j = 0; j < kIn; ++j) {
+            // this clump's own claims are its members: the acceptance would only skip them
+            ow[j] = have[j] ? __ldcg(&a.owner[q[j]]) : myrank;
+            v[j] = have[j] && !all[j] ? f_dr2(ball.qh, ball.ql, a.ft.phi[q[j]], a.ft.plo[q[j]]) : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < kIn; ++j) {
+            keep[j] = have[j] && ow[j] != myrank;
+            if (keep[j] && !all[j]) {
+                if (f_lo(v[j]) > ball.rr32 * (1.f + kRel)) keep[j] = false;
+                else if (!(f_hi(v[j]) < ball.rr32 * (1.f - kRel))) keep[j] = point_dr2(ball.cx, ball.cy, ball.cz, t.pos[q[j]]) <= ball.rr;
+            }
+        }
+        unsigned m[kIn];
+#pragma unroll
+        for (int j = 0; j < kIn; ++j) {
+            m[j] = __ballot_sync(0xffffffffu, keep[j]);
+            if (lane == 0) s_cnt[j * kRbWarps + wid] = __popc(m[j]);
+        }
         __syncthreads();
-        if (tid == 0) s_nel += tot;
+        uint32_t at[kIn], run = found;
+#pragma unroll
+        for (int j = 0; j < kIn; ++j) {
+            for (int w = 0; w < kRbWarps; ++w) {
+                if (w == wid) at[j] = run;
+                run += s_cnt[j * kRbWarps + w];
+            }
+            if (keep[j]) elig[at[j] + __popc(m[j] & ((1u << lane) - 1u))] = q[j];
+        }
+        found = run;
         __syncthreads();
     }
+    if (tid == 0) s_nel = found;
+    __syncthreads();
     const uint32_t nel = s_nel;
     const long long t1 = clock64();
     // 4) the reference's sequential acceptance (src/tree.hpp:4686-4706), 512 candidates at a
@@ -731,32 +764,42 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
 }
 
 // ------------------------------------------------------------------ SortParticles
-// Stable block sort of n keys of `bits` bits with their positions, by digits of kRbDigit bits:
-// (ki, position) to (ko, vo) and back, as many passes as the keys need (bits <= 2 kRbDigit).
-// Returns 1 when the result is in (ko, vo), 0 when in (ki, vi). Every warp counts and then
-// places a segment of its own with counters of its own, so a pass takes four block barriers
-// however long the segments are (with one 512-wide step at a time and three barriers in each,
-// four passes over 50,000 members took 1.27 M cycles; see kRbDigit for the digits).
-__device__ int rb_radix(uint32_t *ki, uint32_t *vi, uint32_t *ko, uint32_t *vo, uint32_t n, uint32_t bits, uint32_t *smem, uint32_t *warp_tot) {
+// Stable block sort of n (squared distance, member) pairs by `bits` bits of key (the top 32 bits
+// of the distance above kmin, without the lowest `drop`; bits <= 2 kRbDigit), by digits of
+// kRbDigit bits: one pass goes from (dist, idx) to (od, oi), two go through rec. Every warp
+// counts and then places a segment of its own with counters of its own, so a pass takes four
+// block barriers however long the segments are.
+//
+// What bounds a pass is the placing: 32 lanes write to 32 lines, a wavefront each. The pair
+// therefore travels as one 16-byte record in the first pass and goes straight to its place in
+// the second (96 wavefronts per 32 members, where a key, a position and a gather of both arrays
+// at the end took 192).
+struct __align__(16) RbRec {
+    double d;
+    uint32_t i, pad;
+};
+
+__device__ void rb_radix(const double *dist, const uint32_t *idx, RbRec *rec, double *od, uint32_t *oi, uint32_t n, uint32_t kmin, uint32_t drop,
+                         uint32_t bits, uint32_t *smem, uint32_t *warp_tot) {
     constexpr uint32_t kBins = 1u << kRbDigit, kPer = kBins / kRB;
     static_assert(kPer == 4, "a thread scans four digits");
     const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, full = 0xffffffffu;
     const uint32_t seg = ((n + kRbWarps * 32 - 1) / (kRbWarps * 32)) * 32, b = min(n, wid * seg), e = min(n, b + seg);
     uint32_t *cnt = smem + wid * kBins;
-    int where = 0;
-    for (uint32_t sh = 0; sh < bits; sh += kRbDigit) {
-        const uint32_t *kin = where ? ko : ki, *vin = where ? vo : vi;
-        uint32_t *kout = where ? ki : ko, *vout = where ? vi : vo;
+    const uint32_t passes = bits > kRbDigit ? 2 : 1;
+    for (uint32_t pass = 0; pass < passes; ++pass) {
+        const uint32_t sh = pass * kRbDigit;
+        auto digit = [&](double d) { return (((((uint32_t)(dbits(d) >> 32)) - kmin) >> drop) >> sh) & (kBins - 1); };
         uint4 *z = reinterpret_cast<uint4 *>(smem);
         for (uint32_t d = tid; d < kBins * kRbWarps / 4; d += kRB) z[d] = make_uint4(0, 0, 0, 0);
         __syncthreads();
         for (uint32_t i = b + lane; i < e; i += 128) {
-            uint32_t k[4];
+            double k[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) k[j] = i + 32 * j < e ? kin[i + 32 * j] : 0u;
+            for (int j = 0; j < 4; ++j) k[j] = i + 32 * j < e ? (pass ? rec[i + 32 * j].d : dist[i + 32 * j]) : 0.0;
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                if (i + 32 * j < e) atomicAdd(&cnt[(k[j] >> sh) & (kBins - 1)], 1u);
+                if (i + 32 * j < e) atomicAdd(&cnt[digit(k[j])], 1u);
         }
         __syncthreads();
         {  // exclusive prefix over (digit, warp): four digits per thread
@@ -790,52 +833,78 @@ __device__ int rb_radix(uint32_t *ki, uint32_t *vi, uint32_t *ko, uint32_t *vo, 
         }
         __syncthreads();
         for (uint32_t i0 = b; i0 < e; i0 += 128) {
-            uint32_t k[4], v[4];
+            double k[4];
+            uint32_t v[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const uint32_t i = i0 + 32 * j + lane;
-                k[j] = i < e ? kin[i] : 0u;
-                v[j] = i < e ? (sh ? vin[i] : i) : 0u;
+                if (pass) {
+                    const uint4 r = i < e ? *reinterpret_cast<const uint4 *>(&rec[i]) : make_uint4(0, 0, 0, 0);
+                    k[j] = dfrom(((uint64_t)r.y << 32) | r.x);
+                    v[j] = r.z;
+                } else {
+                    k[j] = i < e ? dist[i] : 0.0;
+                    v[j] = i < e ? idx[i] : 0u;
+                }
             }
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const bool some = i0 + 32 * j + lane < e;
-                const uint32_t d = some ? (k[j] >> sh) & (kBins - 1) : kBins;
+                const uint32_t d = some ? digit(k[j]) : kBins;
                 const uint32_t peers = __match_any_sync(full, d), rk = __popc(peers & ((1u << lane) - 1u));
                 const uint32_t off = some ? cnt[d] : 0u;
                 __syncwarp();
                 if (some && rk == 0) cnt[d] = off + __popc(peers);
                 __syncwarp();
                 if (some) {
-                    kout[off + rk] = k[j];
-                    vout[off + rk] = v[j];
+                    if (pass + 1 < passes) {
+                        const uint64_t kb = dbits(k[j]);
+                        *reinterpret_cast<uint4 *>(&rec[off + rk]) = make_uint4((uint32_t)kb, (uint32_t)(kb >> 32), v[j], 0);
+                    } else {
+                        od[off + rk] = k[j];
+                        oi[off + rk] = v[j];
+                    }
                 }
             }
         }
         __syncthreads();
-        where ^= 1;
     }
-    return where;
 }
 
-// runs of equal keys: insertion sort by the full squared distance (stable), a thread per run
-__device__ __forceinline__ void rb_fix_runs(const uint32_t *ks, double *dist, uint32_t *idx, uint32_t m) {
+// Runs of equal keys: insertion sort by the full squared distance (stable), a thread per run.
+// Most runs are pairs, so every thread reads its entry's and the next two distances at once
+// (coalesced), and a pair out of order changes places.
+__device__ __forceinline__ void rb_fix_runs(double *dist, uint32_t *idx, uint32_t m, uint32_t kmin, uint32_t drop) {
+    auto key = [&](double d) { return ((uint32_t)(dbits(d) >> 32) - kmin) >> drop; };
+    // a run changes only within itself, and its keys are equal: what a thread reads of another
+    // thread's run has the same key before and after
     for (uint32_t k = threadIdx.x; k + 1 < m; k += kRB) {
-        if ((k == 0 || ks[k] != ks[k - 1]) && ks[k + 1] == ks[k]) {
-            uint32_t e = k + 1;
-            while (e < m && ks[e] == ks[k]) ++e;
-            for (uint32_t i = k + 1; i < e; ++i) {
-                const double dv = dist[i];
-                const uint32_t iv = idx[i];
-                uint32_t j = i;
-                while (j > k && dist[j - 1] > dv) {
-                    dist[j] = dist[j - 1];
-                    idx[j] = idx[j - 1];
-                    --j;
-                }
-                dist[j] = dv;
-                idx[j] = iv;
+        const double d0 = dist[k], d1 = dist[k + 1];
+        const uint32_t k1 = key(d0), k2 = key(d1), k0 = k ? key(dist[k - 1]) : ~k1, k3 = k + 2 < m ? key(dist[k + 2]) : ~k2;
+        if (k0 == k1 || k1 != k2) continue;
+        if (k2 != k3) {
+            if (dbits(d0) > dbits(d1)) {
+                const uint32_t i0 = idx[k], i1 = idx[k + 1];
+                dist[k] = d1;
+                dist[k + 1] = d0;
+                idx[k] = i1;
+                idx[k + 1] = i0;
             }
+            continue;
+        }
+        uint32_t e = k + 3;
+        while (e < m && key(dist[e]) == k1) ++e;
+        for (uint32_t i = k + 1; i < e; ++i) {
+            const double dv = dist[i];
+            const uint32_t iv = idx[i];
+            uint32_t j = i;
+            while (j > k && dbits(dist[j - 1]) > dbits(dv)) {
+                dist[j] = dist[j - 1];
+                idx[j] = idx[j - 1];
+                --j;
+            }
+            dist[j] = dv;
+            idx[j] = iv;
         }
     }
 }
@@ -846,6 +915,23 @@ __device__ __forceinline__ bool rb_sqrt_tie(double s0, double s1) {
     const unsigned long long b0 = (unsigned long long)__double_as_longlong(s0), b1 = (unsigned long long)__double_as_longlong(s1);
     if (b1 - b0 > 64ull) return false;  // more than a few ulps apart: the roots differ
     return sqrt(s0) == sqrt(s1);
+}
+
+// whether this thread's neighbours among m sorted squared distances tie
+__device__ __forceinline__ int rb_ties(const double *dist, uint32_t m) {
+    int tie = 0;
+    for (uint32_t k0 = threadIdx.x + 1; k0 < m; k0 += 4 * kRB) {
+        double x[4], y[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t k = k0 + j * kRB;
+            x[j] = k < m ? dist[k - 1] : 0.0;
+            y[j] = k < m ? dist[k] : 1.0;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) tie |= rb_sqrt_tie(x[j], y[j]);
+    }
+    return tie;
 }
 
 // SortParticles with the Hill radius after it (src/tree.hpp:4446-4512, 4715-4717). Returns
@@ -976,32 +1062,19 @@ __device__ bool rb_sort_particles(const RbArgs &a, uint32_t slot, RbShared &sh, 
     // the keys of the sort: the leading bits of the range above the smallest
     const uint32_t range = 32u - (uint32_t)__clz((int)(kmax - kmin));
     if (m <= kRbSmall) {
-        // 3a) in shared memory, behind the counters: the keys and positions, then (over the
-        // counters) the members in order. Up to kRbOnePass members one digit is enough: over some
-        // 64 octaves it leaves runs of a few equal keys to the insertion sort.
+        // 3a) in shared memory, behind the counters: the records and the sorted pairs. Up to
+        // kRbOnePass members one digit is enough: over some 64 octaves it leaves runs of a few
+        // equal keys to the insertion sort.
         const uint32_t most = m <= kRbOnePass && range <= 26 ? kRbDigit : 2 * kRbDigit, drop = range > most ? range - most : 0u;
-        uint32_t *kx = reinterpret_cast<uint32_t *>(sh.buf + kRbRadixBytes), *ky = kx + kRbSmall, *vx = ky + kRbSmall, *vy = vx + kRbSmall;
-        for (uint32_t k = tid; k < m; k += kRB) {
-            kx[k] = ((uint32_t)(dbits(dist[k]) >> 32) - kmin) >> drop;
-            vx[k] = k;  // what a range of no bits keeps
-        }
-        __syncthreads();
-        const int where = rb_radix(kx, vx, ky, vy, m, range - drop, reinterpret_cast<uint32_t *>(sh.buf), sh.warp_tot);
-        const uint32_t *ks = where ? ky : kx, *vs = where ? vy : vx;
-        double *sd = reinterpret_cast<double *>(sh.buf);
+        RbRec *rec = reinterpret_cast<RbRec *>(sh.buf + kRbRadixBytes);
+        double *sd = reinterpret_cast<double *>(rec + kRbSmall);
         uint32_t *si = reinterpret_cast<uint32_t *>(sd + kRbSmall);
-        for (uint32_t k = tid; k < m; k += kRB) {
-            const uint32_t src = vs[k];
-            si[k] = idx[src];
-            sd[k] = dist[src];
-        }
-        __syncthreads();
-        rb_fix_runs(ks, sd, si, m);
+        rb_radix(dist, idx, rec, sd, si, m, kmin, drop, range - drop, reinterpret_cast<uint32_t *>(sh.buf), sh.warp_tot);
+        rb_fix_runs(sd, si, m, kmin, drop);
         __syncthreads();
         // (every size: below 17 members the library's insertion sort is stable by distance,
         // which an order by squared distance only equals when no two roots tie)
-        int tie = 0;
-        for (uint32_t k = tid + 1; k < m; k += kRB) tie |= rb_sqrt_tie(sd[k - 1], sd[k]);
+        const int tie = rb_ties(sd, m);
         if (__syncthreads_or(tie)) {
             if (tid == 0) s_tie = 1;
         } else {
@@ -1012,15 +1085,14 @@ __device__ bool rb_sort_particles(const RbArgs &a, uint32_t slot, RbShared &sh, 
         }
         __syncthreads();
     } else {
-        // 3b) large: radix sort by the leading 2 kRbDigit bits of the range (above the smallest),
-        // with the position as payload, in the clump's sort buffers; the members then go in order
-        // to the spare segment
+        // 3b) large: the records in the clump's sort buffer (16-byte aligned in the distances'
+        // half of the pool), the sorted pairs in its spare segment
         if (tid == 0) {
             RbSeg &g = a.seg[slot];
             s_r = rb_spare(a.P, g, m);
-            if (s_r != kNone && g.buf_cap < 2 * m) {
+            if (s_r != kNone && g.buf_cap < 2 * m + 1) {
                 uint32_t cap;
-                const uint32_t x = rb_alloc(a.P, 2 * m, cap);
+                const uint32_t x = rb_alloc(a.P, 2 * m + 1, cap);
                 if (x == kNone) {
                     s_r = kNone;
                 } else {
@@ -1035,28 +1107,14 @@ __device__ bool rb_sort_particles(const RbArgs &a, uint32_t slot, RbShared &sh, 
         if (r == kNone) {
             ok = false;
         } else {
-            uint32_t *kx = a.P.idx + s_x, *ky = kx + m;
-            uint32_t *vx = reinterpret_cast<uint32_t *>(a.P.dist + s_x), *vy = vx + m;
             const uint32_t drop = range > 2 * kRbDigit ? range - 2 * kRbDigit : 0u;
-            for (uint32_t k = tid; k < m; k += kRB) {
-                kx[k] = ((uint32_t)(dbits(dist[k]) >> 32) - kmin) >> drop;
-                vx[k] = k;  // what a range of no bits keeps
-            }
-            __syncthreads();
-            const int where = rb_radix(kx, vx, ky, vy, m, range - drop, reinterpret_cast<uint32_t *>(sh.buf), sh.warp_tot);
-            const uint32_t *ks = where ? ky : kx, *vs = where ? vy : vx;
+            RbRec *rec = reinterpret_cast<RbRec *>(a.P.dist + ((s_x + 1) & ~1u));
             uint32_t *didx = a.P.idx + r;
             double *ddist = a.P.dist + r;
-            for (uint32_t k = tid; k < m; k += kRB) {
-                const uint32_t src = vs[k];
-                didx[k] = idx[src];
-                ddist[k] = dist[src];
-            }
+            rb_radix(dist, idx, rec, ddist, didx, m, kmin, drop, range - drop, reinterpret_cast<uint32_t *>(sh.buf), sh.warp_tot);
+            rb_fix_runs(ddist, didx, m, kmin, drop);
             __syncthreads();
-            rb_fix_runs(ks, ddist, didx, m);
-            __syncthreads();
-            int tie = 0;
-            for (uint32_t k = tid + 1; k < m; k += kRB) tie |= rb_sqrt_tie(ddist[k - 1], ddist[k]);
+            const int tie = rb_ties(ddist, m);
             if (__syncthreads_or(tie)) {
                 if (tid == 0) s_tie = 1;  // the unsorted segment at o is intact
             } else if (tid == 0) {
@@ -1145,7 +1203,7 @@ __device__ void rb_checkpoint(const RbArgs &a, uint32_t slot, uint32_t rank, uin
 __global__ void __launch_bounds__(kRB, 1) k_rebind_loop(RbArgs a) {
     extern __shared__ __align__(16) unsigned char rb_dyn[];
     __shared__ uint32_t warp_tot[kRbWarps];
-    __shared__ uint32_t u[20 + 2 * kRbWarps];
+    __shared__ uint32_t u[20 + 4 * kRbWarps];
     __shared__ double st[8], sums[8], sd[8], tk[32 * 8], hist[33 * 8];
     __shared__ float sf[16];
     __shared__ uint32_t s_item;
