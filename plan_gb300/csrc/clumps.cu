@@ -728,83 +728,6 @@ __device__ __forceinline__ double div_by_rcp(double num, double den, double y) {
     return fma(fma(-q0, den, num), y, q0);
 }
 
-// RemoveUnboundParticles (src/tree.hpp:4615-4674) for a list of clumps, one block each. The
-// six quotients by the remaining mass share one correctly rounded reciprocal (div_by_rcp).
-__global__ void __launch_bounds__(256) k_unbind(const uint32_t *list, CT ct, Pool P, const double4_32a *pos, const double4_32a *vel, CP cp) {
-    __shared__ double sM, scx, scy, scz, svx, svy, svz;
-    __shared__ int s_best;
-    __shared__ uint32_t s_back;
-    uint32_t s = list[blockIdx.x];
-    const uint32_t o = ct.moff[s];
-    if (threadIdx.x == 0) {
-        sM = ct.M[s];
-        double4_32a c = ct.com[s], v = ct.vcom[s];
-        scx = c.x; scy = c.y; scz = c.z;
-        svx = v.x; svy = v.y; svz = v.z;
-        s_back = ct.mn[s] - 1;
-    }
-    __syncthreads();
-    int i = (int)ct.mn[s] - 1;
-    while (i >= 1) {
-        int lo = max(1, i - (int)blockDim.x + 1);
-        if (threadIdx.x == 0) s_best = -1;
-        __syncthreads();
-        int j = i - (int)threadIdx.x;
-        bool unbound = false;
-        double Mr = 0;
-        if (j >= lo) {
-            uint32_t pi = P.idx[o + j];
-            double4_32a p = pos[pi], v = vel[pi];
-            double M = sM;
-            Mr = M - p.w;  // > 0: at least two members remain
-            const double y = __drcp_rn(Mr);
-            double cx = div_by_rcp(scx * M - p.x * p.w, Mr, y), cy = div_by_rcp(scy * M - p.y * p.w, Mr, y),
-                   cz = div_by_rcp(scz * M - p.z * p.w, Mr, y);
-            double vx = div_by_rcp(svx * M - v.x * p.w, Mr, y), vy = div_by_rcp(svy * M - v.y * p.w, Mr, y),
-                   vz = div_by_rcp(svz * M - v.z * p.w, Mr, y);
-            double dx = cx - p.x;
-            double ex = (vx - 0.0 * dx) - v.x, ey = (vy - cp.shear * dx) - v.y, ez = (vz - 0.0 * dx) - v.z;
-            double e = +0.5 / M * norm2_3(ex, ey, ez) - cp.G / norm3(cx - p.x, cy - p.y, cz - p.z);
-            unbound = e > 0;
-        }
-        if (unbound) atomicMax(&s_best, j);
-        __syncthreads();
-        int b = s_best;
-        if (b < 0) {
-            i = lo - 1;
-            __syncthreads();
-            continue;
-        }
-        if ((int)threadIdx.x == i - b) {  // the thread that evaluated b updates the state
-            uint32_t pi = P.idx[o + b];
-            double4_32a p = pos[pi], v = vel[pi];
-            double M = sM;
-            double Mr2 = M - p.w;
-            const double y2 = __drcp_rn(Mr2);
-            scx = div_by_rcp(scx * M - p.x * p.w, Mr2, y2); scy = div_by_rcp(scy * M - p.y * p.w, Mr2, y2);
-            scz = div_by_rcp(scz * M - p.z * p.w, Mr2, y2);
-            svx = div_by_rcp(svx * M - v.x * p.w, Mr2, y2); svy = div_by_rcp(svy * M - v.y * p.w, Mr2, y2);
-            svz = div_by_rcp(svz * M - v.z * p.w, Mr2, y2);
-            sM = Mr2;
-            // swap with the back and pop (src/tree.hpp:4660-4663)
-            uint32_t bk = s_back;
-            uint32_t tmp = P.idx[o + b];
-            P.idx[o + b] = P.idx[o + bk];
-            P.idx[o + bk] = tmp;
-            s_back = bk - 1;
-        }
-        __syncthreads();
-        i = b - 1;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        ct.mn[s] = s_back + 1;
-        ct.M[s] = sM;
-        ct.com[s] = make_double4_32a(scx, scy, scz, 0);
-        ct.vcom[s] = make_double4_32a(svx, svy, svz, 0);
-    }
-}
-
 // Hill-sphere rebinding (src/tree.hpp:4678-4711).
 //
 // RecursiveBallSearch visits the children of a node in order and every node covers a
@@ -1041,6 +964,7 @@ __device__ void defer_add(uint32_t *dset, uint8_t *dover, uint32_t *dmax, uint32
 }
 
 #include "rebind_loop.cuh"
+#include "unbind.cuh"
 
 // One SearchBoundParticlesWithinHillRadius call for every listed clump (one block each).
 // seq_mode = 1: the reference's shared in-clump flags, one clump at a time.
@@ -1994,7 +1918,10 @@ struct Stage {
         if (list.empty()) return kOk;
         int rc = up_list(list, d_list);
         if (rc) return rc;
-        k_unbind<<<(unsigned)list.size(), 256, 0, s>>>(d_list, ct, P, tr.pos, tr.vel, cp);
+        if (!tr.phi) return kErrDevice;  // the FP32 copies are made by the density stage
+        const FTree ft{tr.phi, tr.plo, tr.nhi, tr.nlo};
+        PLAN_CUDA(cudaFuncSetAttribute(k_unbind, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(UbShared)));
+        k_unbind<<<(unsigned)list.size(), kUb, sizeof(UbShared), s>>>(d_list, ct, P, tr.pos, tr.vel, ft, cp);
         c.launches++;
         PLAN_CUDA(cudaGetLastError());
         // RemoveUnboundParticles ends with SortParticles; every caller computes the Hill
