@@ -1834,10 +1834,10 @@ struct Stage {
             PLAN_CUDA(cudaMemcpyAsync(dl, large.data(), large.size() * 4, cudaMemcpyHostToDevice, s));
             PLAN_CUDA(cudaMemcpyAsync(db, base.data(), base.size() * 4, cudaMemcpyHostToDevice, s));
             k_large_gather<<<(unsigned)large.size(), 256, 0, s>>>(dl, (uint32_t)large.size(), db, ct, P, w0, w1, w2, pay);
-            rc = radix_sort96(w0, w1, w2, pay, tot, scr, sb, s);
+            rc = radix_sort96(w0, w1, w2, pay, tot, scr, sb, s, 0xfffu, true, &c.launches);
             if (rc) { S.used = mark; return rc; }
             k_large_scatter<<<(unsigned)large.size(), 256, 0, s>>>(dl, (uint32_t)large.size(), db, ct, P, w0, w1, pay, d_tie);
-            c.launches += 2 + 36;
+            c.launches += 2;
             PLAN_CUDA(cudaGetLastError());
             rc = sync();
             S.used = mark;
@@ -1918,7 +1918,6 @@ struct Stage {
         if (list.empty()) return kOk;
         int rc = up_list(list, d_list);
         if (rc) return rc;
-        if (!tr.phi) return kErrDevice;  // the FP32 copies are made by the density stage
         const FTree ft{tr.phi, tr.plo, tr.nhi, tr.nlo};
         PLAN_CUDA(cudaFuncSetAttribute(k_unbind, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(UbShared)));
         k_unbind<<<(unsigned)list.size(), kUb, sizeof(UbShared), s>>>(d_list, ct, P, tr.pos, tr.vel, ft, cp);
@@ -2433,7 +2432,6 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
         PLAN_CUDA(cudaMemsetAsync(tent, 0xff, (size_t)Tu * 4, s));
         KTree kt = ktree_of(tr);
         const FTree ftr{tr.phi, tr.plo, tr.nhi, tr.nlo};
-        if (!tr.phi) return kErrDevice;  // the FP32 copies are made by the density stage
         // speculative acceptance windows (exact by verification; PLAN_ACCEPT_SPECULATE=1)
         const char *spec_env = std::getenv("PLAN_ACCEPT_SPECULATE");
         const bool speculate = spec_env && *spec_env == '1';

@@ -253,8 +253,6 @@ int density_vs_scale(Context &c, const plan_params &p, double time, std::vector<
         for (const std::vector<double> *v : {&xs, &ys, &zs})
             if (!v->empty()) coord = std::fmax(coord, std::fmax(std::fabs(v->front()), std::fabs(v->back())) + g.sub1[0] + g.sub1[1] + g.sub1[2]);
         const DvsGeomF gf = dvs_geom_f(g, coord);
-        int rc = ensure_split(c, s);
-        if (rc) return rc;
         const FTree ft{tr.phi, tr.plo, tr.nhi, tr.nlo};
         const DevTreeView tv{ktree_of(tr)};
         const uint64_t ncentre = (uint64_t)g.nx * g.ny * g.nz * g.nlev;

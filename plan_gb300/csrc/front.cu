@@ -25,24 +25,35 @@ struct MassTable {
 };
 
 // ---------------------------------------------------------------- ingest
-__global__ void k_unpack(const unsigned char *rec, size_t n, double4_32a *pos, double4_32a *vel, uint32_t *type, uint32_t *kw0,
-                         uint32_t *kw1, uint32_t *kw2, uint32_t *kidx) {
-    size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const unsigned char *r = rec + 44 * i;
-    float f[7];
-    for (int k = 0; k < 7; ++k) {
-        uint32_t u = (uint32_t)r[4 * k] | ((uint32_t)r[4 * k + 1] << 8) | ((uint32_t)r[4 * k + 2] << 16) | ((uint32_t)r[4 * k + 3] << 24);
-        f[k] = __uint_as_float(u);
+// The 44-byte records of a block of 256 particles come in as one run of 16-byte loads through
+// shared memory (kWide: the records start on a 16-byte boundary; byte loads otherwise), so records
+// in page-locked host memory are read in place, once: the copy to the device before took longer
+// than the reading does (8 M records with the unpacking: 2.65 -> 2.27 ms; 206 GB/s over the link).
+template <bool kWide>
+__global__ void __launch_bounds__(256) k_unpack(const unsigned char *rec, uint32_t n, uint32_t first, double4_32a *pos, double4_32a *vel,
+                                                uint32_t *type, uint32_t *kw0, uint32_t *kw1, uint32_t *kw2, uint32_t *kidx) {
+    __shared__ __align__(16) uint32_t s_w[256 * 11];
+    const size_t r0 = (size_t)blockIdx.x * 256;
+    const uint32_t m = (uint32_t)min((size_t)256, n - r0);
+    if (kWide && m == 256) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(rec + 44 * r0);
+        uint4 *dst = reinterpret_cast<uint4 *>(s_w);
+        for (uint32_t k = threadIdx.x; k < 704; k += 256) dst[k] = src[k];
+    } else {
+        const unsigned char *src = rec + 44 * r0;
+        unsigned char *dst = reinterpret_cast<unsigned char *>(s_w);
+        for (uint32_t k = threadIdx.x; k < 44 * m; k += 256) dst[k] = src[k];
     }
-    auto u32at = [&](int off) {
-        return (uint32_t)r[off] | ((uint32_t)r[off + 1] << 8) | ((uint32_t)r[off + 2] << 16) | ((uint32_t)r[off + 3] << 24);
-    };
-    pos[i] = make_double4_32a((double)f[0], (double)f[1], (double)f[2], 0.0);
-    vel[i] = make_double4_32a((double)f[3], (double)f[4], (double)f[5], (double)f[6]);
-    type[i] = u32at(28);
-    kw0[i] = u32at(32);               // id_in_run: low 32 bits of the i64 (src/tree.hpp:1507)
-    kw1[i] = u32at(40) & 0xffffu;     // cpu_id as uint16 (src/tree.hpp:1510)
+    __syncthreads();
+    if (threadIdx.x >= m) return;
+    const uint32_t *u = s_w + 11 * threadIdx.x;
+    const size_t i = first + r0 + threadIdx.x;
+    auto f = [&](int k) { return (double)__uint_as_float(u[k]); };
+    pos[i] = make_double4_32a(f(0), f(1), f(2), 0.0);
+    vel[i] = make_double4_32a(f(3), f(4), f(5), f(6));
+    type[i] = u[7];
+    kw0[i] = u[8];             // id_in_run: low 32 bits of the i64 (src/tree.hpp:1507)
+    kw1[i] = u[10] & 0xffffu;  // cpu_id as uint16 (src/tree.hpp:1510)
     kw2[i] = 0;
     kidx[i] = (uint32_t)i;
 }
@@ -104,6 +115,16 @@ struct GhostGeom {
     double box_min1, box_max1, len0, len1, shear_dt;  // shear_dt = shear_speed * time
 };
 
+// (double)(int)(d / len): without the division where the quotient's integer is known. A d below
+// len in magnitude gives a quotient that rounds below 1, one below 2 len a quotient below 2. (The
+// divisions took most of the ghost kernels' time: 0.47 + 0.42 -> 0.25 + 0.20 ms at 8 M particles.)
+__device__ __forceinline__ double whole_boxes(double d, double len) {
+    const double a = fabs(d);
+    if (a < len) return 0.0;
+    if (a < 2.0 * len) return d < 0.0 ? -1.0 : 1.0;
+    return (double)(int)(d / len);
+}
+
 __global__ void k_ghost_count_x(const double4_32a *pos, uint32_t n, GhostGeom g, uint32_t *cnt) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -121,7 +142,7 @@ __global__ void k_ghost_write_x(double4_32a *pos, double4_32a *vel, uint32_t *ty
         double4_32a q = p;
         q.x = q.x - g.len0;
         double ny = q.y + g.shear_dt;
-        q.y = ny - (double)(int)((ny - g.box_min1) / g.len1) * g.len1;
+        q.y = ny - whole_boxes(ny - g.box_min1, g.len1) * g.len1;
         pos[o] = q; vel[o] = vel[i]; type[o] = type[i];
         ++o;
     }
@@ -129,7 +150,7 @@ __global__ void k_ghost_write_x(double4_32a *pos, double4_32a *vel, uint32_t *ty
         double4_32a q = p;
         q.x = q.x + g.len0;
         double ny = q.y - g.shear_dt;
-        q.y = ny + (double)(int)((g.box_max1 - ny) / g.len1) * g.len1;
+        q.y = ny + whole_boxes(g.box_max1 - ny, g.len1) * g.len1;
         pos[o] = q; vel[o] = vel[i]; type[o] = type[i];
     }
 }
@@ -163,25 +184,31 @@ __global__ void k_ghost_write_y(double4_32a *pos, double4_32a *vel, uint32_t *ty
 }
 
 // exact number of ghosts of all kinds (order independent), to size buffers before writing
-__global__ void k_ghost_total(const double4_32a *pos, uint32_t n, GhostGeom g, unsigned long long *tot) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) k_ghost_total(const double4_32a *pos, uint32_t n, GhostGeom g, unsigned long long *tot) {
+    __shared__ unsigned s_c[8];
     unsigned c = 0;
-    if (i < n) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double4_32a p = pos[i];
         if (p.x > g.hi[0]) {
             double ny = p.y + g.shear_dt;
-            double y = ny - (double)(int)((ny - g.box_min1) / g.len1) * g.len1;
+            double y = ny - whole_boxes(ny - g.box_min1, g.len1) * g.len1;
             c += 1 + (y < g.lo[1] ? 1 : 0) + (y > g.hi[1] ? 1 : 0);
         }
         if (p.x < g.lo[0]) {
             double ny = p.y - g.shear_dt;
-            double y = ny + (double)(int)((g.box_max1 - ny) / g.len1) * g.len1;
+            double y = ny + whole_boxes(g.box_max1 - ny, g.len1) * g.len1;
             c += 1 + (y < g.lo[1] ? 1 : 0) + (y > g.hi[1] ? 1 : 0);
         }
         c += (p.y < g.lo[1] ? 1 : 0) + (p.y > g.hi[1] ? 1 : 0);
     }
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(tot, (unsigned long long)c);
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((threadIdx.x & 31) == 0) s_c[threadIdx.x >> 5] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {  // one atomic per block (one per warp queued 440,000 on one address at 14 M points)
+        unsigned long long sum = 0;
+        for (int w = 0; w < 8; ++w) sum += s_c[w];
+        if (sum) atomicAdd(tot, sum);
+    }
 }
 
 // ---------------------------------------------------------------- box and keys
@@ -262,7 +289,7 @@ __global__ void k_run_starts(const uint32_t *flag, const uint32_t *rank, uint32_
 __global__ void k_sortpoints(const uint32_t *starts, uint32_t Tu, uint32_t T, const uint32_t *kidx, const uint32_t *kw0,
                              const uint32_t *kw1, const uint32_t *kw2, const double4_32a *in_pos, const double4_32a *in_vel, double4_32a *pos,
                              double4_32a *vel, uint32_t *orig, uint32_t *tk0, uint32_t *tk1, uint32_t *tk2, uint32_t *sink_n,
-                             uint32_t *sink_first) {
+                             uint32_t *sink_first, float4 *phi, float4 *plo) {
     uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= Tu) return;
     uint32_t j = starts[t], e = (t + 1 < Tu) ? starts[t + 1] : T;
@@ -282,6 +309,10 @@ __global__ void k_sortpoints(const uint32_t *starts, uint32_t Tu, uint32_t T, co
     }
     pos[t] = p;
     vel[t] = v;
+    // the FP32 hi/lo copy of the position, while it is in registers
+    const float hx = (float)p.x, hy = (float)p.y, hz = (float)p.z;
+    phi[t] = make_float4(hx, hy, hz, 0.f);
+    plo[t] = make_float4((float)(p.x - (double)hx), (float)(p.y - (double)hy), (float)(p.z - (double)hz), 0.f);
     orig[t] = src;  // particle ids equal the input-order index (src/tree.hpp:1558-1560, 1660)
     tk0[t] = kw0[j]; tk1[t] = kw1[j]; tk2[t] = kw2[j];
     sink_n[t] = e - j;
@@ -362,9 +393,20 @@ struct LevelBase {
     uint32_t base[33];
 };
 
+__device__ __forceinline__ void node_floats(const double4_32a c, float4 &hi, float4 &lo) {
+    const float hx = (float)c.x, hy = (float)c.y, hz = (float)c.z, hw = (float)c.w;
+    hi = make_float4(hx, hy, hz, hw);
+    lo = make_float4((float)(c.x - (double)hx), (float)(c.y - (double)hy), (float)(c.z - (double)hz), (float)(c.w - (double)hw));
+}
+
+// Every node's first point, parent, first daughter, orthant and level, and every point's leaf.
+// Centres and ends follow level by level (k_node_level): the centre of a node is its parent's
+// plus or minus its half width, three FP64 additions per node, where every point's own chain of
+// them down to its leaf held the FP64 pipe (2.1 ms of this kernel at 14 M points).
 __global__ void k_nodes(const uint8_t *lcp_prev, const uint8_t *leaf_lvl, const uint32_t *k0, const uint32_t *k1, const uint32_t *k2,
-                        uint32_t n, const uint32_t *bc, LevelBase lb, TreeBox box, double4_32a *ncf, uint32_t *nbeg, uint32_t *npar,
-                        uint32_t *nfd, uint32_t *nnd, uint8_t *north, uint8_t *nlev, uint32_t *leaf_of, uint32_t nn, unsigned *err) {
+                        uint32_t n, const uint32_t *bc, LevelBase lb, TreeBox box, double4_32a *ncf, float4 *nhi, float4 *nlo, uint32_t *nbeg,
+                        uint32_t *npar, uint32_t *nfd, uint32_t *nnd, uint8_t *north, uint8_t *nlev, uint32_t *leaf_of, uint32_t nn,
+                        unsigned *err) {
     __shared__ uint32_t s_cnt[32][8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -385,26 +427,22 @@ __global__ void k_nodes(const uint8_t *lcp_prev, const uint8_t *leaf_lvl, const 
     }
     __syncthreads();
     if (i == 0) {  // root (src/tree.hpp:2872-2881)
-        ncf[0] = make_double4_32a(box.root_center[0], box.root_center[1], box.root_center[2], box.half_width);
+        const double4_32a r = make_double4_32a(box.root_center[0], box.root_center[1], box.root_center[2], box.half_width);
+        ncf[0] = r;
+        node_floats(r, nhi[0], nlo[0]);
         nbeg[0] = 0;
         npar[0] = 0xffffffffu;
         nfd[0] = lb.base[1];
         north[0] = 0;
         nlev[0] = 1;
     }
-    double c[3] = {box.root_center[0], box.root_center[1], box.root_center[2]};
-    double hw = box.half_width;
     uint32_t prev_idx = 0;
     const unsigned lt = (1u << lane) - 1u;
     for (int L = 1; L < 32; ++L) {
         bool st = starts_level(L, a, l);
         unsigned b = __ballot_sync(0xffffffffu, st);
-        if (i >= n) continue;
+        if (i >= n || L > l || (L < a && L < l)) continue;  // a point may share its leaf with the one before (a >= l)
         uint32_t excl = bc[(size_t)blockIdx.x * 32 + L] + s_cnt[L][warp] + __popc(b & lt);
-        if (L > l) continue;
-        int dg = key_digit(k0[i], k1[i], k2[i], L);
-        hw = 0.5 * hw;
-        for (int d = 0; d < 3; ++d) c[d] = c[d] + hw * (double)(((dg >> d) & 1) ? 1 : -1);
         if (L == l) {
             uint32_t lf = lb.base[L] + excl - (st ? 0u : 1u);
             if (lf < nn) leaf_of[i] = lf;
@@ -418,10 +456,9 @@ __global__ void k_nodes(const uint8_t *lcp_prev, const uint8_t *leaf_lvl, const 
             atomicOr(err, (unsigned)kDevErrBadNode);
             continue;
         }
-        ncf[idx] = make_double4_32a(c[0], c[1], c[2], hw);
         nbeg[idx] = i;
         npar[idx] = parent;
-        north[idx] = (uint8_t)dg;
+        north[idx] = (uint8_t)key_digit(k0[i], k1[i], k2[i], L);
         nlev[idx] = (uint8_t)(L + 1);
         nfd[idx] = 0;
         if (L > a + 1) nfd[prev_idx] = idx;  // this node is the first daughter of its parent
@@ -430,19 +467,50 @@ __global__ void k_nodes(const uint8_t *lcp_prev, const uint8_t *leaf_lvl, const 
     }
 }
 
-// node ends, one tree level at a time from the top: the next sibling's begin, or the
-// parent's end for the last daughter
-__global__ void k_node_end_level(uint32_t first, uint32_t count, const uint32_t *nbeg, const uint32_t *npar, const uint32_t *nfd,
-                                 const uint32_t *nnd, uint32_t *nend, uint32_t nn, unsigned *err) {
-    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= count) return;
-    uint32_t idx = first + k;
-    uint32_t p = npar[idx];
-    if (p >= nn || idx + 1 > nn) {
+struct NodeArrays {
+    double4_32a *ncf;
+    float4 *nhi, *nlo;
+    const uint32_t *nbeg, *npar, *nfd, *nnd;
+    uint32_t *nend;
+    const uint8_t *north;
+    uint32_t nn;
+};
+
+// A node's centre from its parent's, and its end: the next sibling's begin, or the parent's end
+// for the last daughter.
+__device__ __forceinline__ void node_from_parent(const NodeArrays &t, uint32_t idx, unsigned *err) {
+    const uint32_t p = t.npar[idx];
+    if (p >= t.nn || idx + 1 > t.nn) {
         atomicOr(err, (unsigned)kDevErrBadNode);
         return;
     }
-    nend[idx] = (idx + 1 < nfd[p] + nnd[p] && idx + 1 < nn) ? nbeg[idx + 1] : nend[p];
+    t.nend[idx] = (idx + 1 < t.nfd[p] + t.nnd[p] && idx + 1 < t.nn) ? t.nbeg[idx + 1] : t.nend[p];
+    double4_32a c = t.ncf[p];
+    const double hw = 0.5 * c.w;
+    const int dg = t.north[idx];
+    c.x = c.x + ((dg & 1) ? hw : -hw);
+    c.y = c.y + ((dg & 2) ? hw : -hw);
+    c.z = c.z + ((dg & 4) ? hw : -hw);
+    c.w = hw;
+    t.ncf[idx] = c;
+    node_floats(c, t.nhi[idx], t.nlo[idx]);
+}
+
+// one tree level, from the top
+__global__ void k_node_level(uint32_t first, uint32_t count, NodeArrays t, unsigned *err) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < count) node_from_parent(t, first + k, err);
+}
+
+// Levels [from, to), short ones (at most kNarrow nodes each), in one block: a launch per level
+// costs more than two rounds of the block.
+constexpr uint32_t kNarrow = 2048;
+
+__global__ void __launch_bounds__(1024) k_node_levels(LevelBase lb, int from, int to, NodeArrays t, unsigned *err) {
+    for (int L = from; L < to; ++L) {
+        for (uint32_t idx = lb.base[L] + threadIdx.x; idx < lb.base[L + 1]; idx += blockDim.x) node_from_parent(t, idx, err);
+        __syncthreads();
+    }
 }
 
 }  // namespace
@@ -475,9 +543,8 @@ int build_octree(Context &c, double4_32a *in_pos, double4_32a *in_vel, const uin
         k_keys_keep_mass<<<grid_for(T, 256), 256, 0, s>>>(in_pos, T, box, kw0, kw1, kw2, kidx);
     }
     c.launches++;
-    int rc = radix_sort96(kw0, kw1, kw2, kidx, T, scr, sort_bytes, s);
+    int rc = radix_sort96(kw0, kw1, kw2, kidx, T, scr, sort_bytes, s, 0xfffu, true, &c.launches);
     if (rc) return rc;
-    c.launches += 36;
     if (after_sort) cudaEventRecord(after_sort, s);
 
     // sink folding (src/tree.hpp:2608-2651)
@@ -526,10 +593,11 @@ int build_octree(Context &c, double4_32a *in_pos, double4_32a *in_vel, const uin
     tr.tk2 = A.get<uint32_t>(Tu);
     tr.sink_n = A.get<uint32_t>(Tu);
     tr.sink_first = A.get<uint32_t>(Tu);
-    tr.leaf_of = A.get<uint32_t>(Tu);
+    tr.phi = A.get<float4>(Tu);
+    tr.plo = A.get<float4>(Tu);
     if (A.failed) return kErrOutOfMemory;
     k_sortpoints<<<grid_for(Tu, 256), 256, 0, s>>>(starts, Tu, T, kidx, kw0, kw1, kw2, in_pos, in_vel, tr.pos, tr.vel, tr.orig, tr.tk0,
-                                                   tr.tk1, tr.tk2, tr.sink_n, tr.sink_first);
+                                                   tr.tk1, tr.tk2, tr.sink_n, tr.sink_first, tr.phi, tr.plo);
     c.launches++;
     tr.nsinks = T - Tu;
     tr.leaf_size = leaf;
@@ -562,28 +630,41 @@ int build_octree(Context &c, double4_32a *in_pos, double4_32a *in_vel, const uin
     const uint32_t nn = run;
     tr.nodes = nn;
     tr.ncf = A.get<double4_32a>(nn);
+    tr.nhi = A.get<float4>(nn);
+    tr.nlo = A.get<float4>(nn);
+    // zeroed together
+    char *zero = A.get<char>(0);
+    tr.leaf_of = A.get<uint32_t>(Tu);
     tr.nbeg = A.get<uint32_t>(nn);
     tr.nend = A.get<uint32_t>(nn);
     tr.npar = A.get<uint32_t>(nn);
     tr.nfd = A.get<uint32_t>(nn);
     uint32_t *nnd32 = A.get<uint32_t>(nn);
+    const size_t zero_bytes = (size_t)(reinterpret_cast<char *>(nnd32 + nn) - zero);
     tr.north = A.get<uint8_t>(nn);
     tr.nlev = A.get<uint8_t>(nn);
     if (A.failed) return kErrOutOfMemory;
-    PLAN_CUDA(cudaMemsetAsync(nnd32, 0, (size_t)nn * 4, s));
-    PLAN_CUDA(cudaMemsetAsync(tr.nfd, 0, (size_t)nn * 4, s));
-    PLAN_CUDA(cudaMemsetAsync(tr.npar, 0, (size_t)nn * 4, s));
-    PLAN_CUDA(cudaMemsetAsync(tr.nbeg, 0, (size_t)nn * 4, s));
-    PLAN_CUDA(cudaMemsetAsync(tr.nend, 0, (size_t)nn * 4, s));
-    PLAN_CUDA(cudaMemsetAsync(tr.leaf_of, 0, (size_t)Tu * 4, s));
-    k_nodes<<<nb, 256, 0, s>>>(lcp_prev, leaf_lvl, tr.tk0, tr.tk1, tr.tk2, Tu, bc, lb, box, tr.ncf, tr.nbeg, tr.npar, tr.nfd, nnd32,
-                               tr.north, tr.nlev, tr.leaf_of, nn, c.d_err);
+    PLAN_CUDA(cudaMemsetAsync(zero, 0, zero_bytes, s));
+    k_nodes<<<nb, 256, 0, s>>>(lcp_prev, leaf_lvl, tr.tk0, tr.tk1, tr.tk2, Tu, bc, lb, box, tr.ncf, tr.nhi, tr.nlo, tr.nbeg, tr.npar, tr.nfd,
+                               nnd32, tr.north, tr.nlev, tr.leaf_of, nn, c.d_err);
     PLAN_CUDA(cudaMemcpyAsync(tr.nend, &Tu, 4, cudaMemcpyHostToDevice, s));
     c.launches++;
-    for (int L = 1; L < 32; ++L) {
-        if (!lc[L]) continue;
-        k_node_end_level<<<grid_for(lc[L], 256), 256, 0, s>>>(lb.base[L], lc[L], tr.nbeg, tr.npar, tr.nfd, nnd32, tr.nend, nn, c.d_err);
-        c.launches++;
+    {
+        const NodeArrays t{tr.ncf, tr.nhi, tr.nlo, tr.nbeg, tr.npar, tr.nfd, nnd32, tr.nend, tr.north, nn};
+        int last = 31;
+        while (last > 0 && !lc[last]) --last;
+        for (int L = 1; L <= last;) {
+            int e = L;
+            while (e <= last && lc[e] <= kNarrow) ++e;
+            if (e > L) {
+                k_node_levels<<<1, 1024, 0, s>>>(lb, L, e, t, c.d_err);
+                L = e;
+            } else {
+                k_node_level<<<grid_for(lc[L], 256), 256, 0, s>>>(lb.base[L], lc[L], t, c.d_err);
+                ++L;
+            }
+            c.launches++;
+        }
     }
     PLAN_CUDA(cudaGetLastError());
     tr.nnd = reinterpret_cast<uint8_t *>(nnd32);  // num_daughters kept as u32
@@ -631,13 +712,14 @@ int build_tree(Context &c, const plan_lis_view &v, plan_params &p, int first_fil
     c.scratch.used = 0;
     c.scratch.failed = false;
     Arena &S = c.scratch;
-    unsigned char *d_rec = S.get<unsigned char>((size_t)N * 44);
+    // the records, and the sort of the ids in their place once they are unpacked
+    const size_t sortA = std::max(radix_sort96_scratch_bytes(N), scan_u32_scratch_bytes(N));
+    unsigned char *d_rec = S.get<unsigned char>(std::max((size_t)N * 44, sortA));
+    void *scrA = d_rec;
     double4_32a *tmp_pos = S.get<double4_32a>(N), *tmp_vel = S.get<double4_32a>(N);
     uint32_t *tmp_type = S.get<uint32_t>(N);
     uint32_t *aw0 = S.get<uint32_t>(N), *aw1 = S.get<uint32_t>(N), *aw2 = S.get<uint32_t>(N), *aidx = S.get<uint32_t>(N);
     unsigned long long *d_desc = S.get<unsigned long long>(4);
-    size_t sortA = radix_sort96_scratch_bytes(N);
-    void *scrA = S.take(sortA);
     uint32_t *sel_src = nullptr, *sel_rank = nullptr, *sel_tot = nullptr;
     if (p.user_box) {
         sel_src = S.get<uint32_t>(N);
@@ -646,33 +728,42 @@ int build_tree(Context &c, const plan_lis_view &v, plan_params &p, int first_fil
     }
     if (S.failed) return kErrOutOfMemory;
 
-    // 1. upload and unpack; a single block already in device memory is read in place
-    const unsigned char *src = d_rec;
-    cudaPointerAttributes pa{};
-    if (v.nblocks == 1 && cudaPointerGetAttributes(&pa, v.records[0]) == cudaSuccess && pa.type == cudaMemoryTypeDevice &&
-        pa.device == c.device) {
-        src = static_cast<const unsigned char *>(v.records[0]);
-        c.counters[20] = 0;
-    } else {
-        cudaGetLastError();
+    // 1. unpack: blocks in this device's memory or in page-locked host memory are read in place,
+    // others are copied first
+    {
         size_t at = 0;
+        uint64_t uploaded = 0;
         for (uint32_t b = 0; b < v.nblocks; ++b) {
-            PLAN_CUDA(cudaMemcpyAsync(d_rec + at * 44, v.records[b], v.counts[b] * 44, cudaMemcpyDefault, s));
-            at += v.counts[b];
+            const size_t m = v.counts[b];
+            if (!m) continue;
+            const unsigned char *src = d_rec + at * 44;
+            cudaPointerAttributes pa{};
+            const bool known = cudaPointerGetAttributes(&pa, v.records[b]) == cudaSuccess;
+            if (!known) cudaGetLastError();
+            if (known && pa.type == cudaMemoryTypeDevice && pa.device == c.device) {
+                src = static_cast<const unsigned char *>(v.records[b]);
+            } else {
+                if (known && pa.type == cudaMemoryTypeHost && pa.devicePointer) src = static_cast<const unsigned char *>(pa.devicePointer);
+                else PLAN_CUDA(cudaMemcpyAsync(d_rec + at * 44, v.records[b], m * 44, cudaMemcpyDefault, s));
+                uploaded += m * 44;
+            }
+            auto unpack = (reinterpret_cast<uintptr_t>(src) & 15) == 0 ? k_unpack<true> : k_unpack<false>;
+            unpack<<<grid_for(m, 256), 256, 0, s>>>(src, (uint32_t)m, (uint32_t)at, tmp_pos, tmp_vel, tmp_type, aw0, aw1, aw2, aidx);
+            c.launches++;
+            at += m;
         }
-        c.counters[20] = (uint64_t)N * 44;  // bytes uploaded
+        PLAN_CUDA(cudaGetLastError());
+        c.counters[20] = uploaded;
     }
-    k_unpack<<<grid_for(N, 256), 256, 0, s>>>(src, N, tmp_pos, tmp_vel, tmp_type, aw0, aw1, aw2, aidx);
     PLAN_CUDA(cudaMemsetAsync(d_desc, 0, 32, s));
     k_count_descents<<<grid_for(N, 256), 256, 0, s>>>(aw0, aw1, N, d_desc);
-    c.launches += 2;
+    c.launches++;
     unsigned long long h_desc[2];
     PLAN_CUDA(cudaMemcpyAsync(h_desc, d_desc, 16, cudaMemcpyDeviceToHost, s));
     PLAN_CUDA(cudaStreamSynchronize(s));
     if (h_desc[0]) {  // not yet in (cpu_id, id_in_run) order (src/tree.hpp:1552-1557)
-        int rc = radix_sort96(aw0, aw1, aw2, aidx, N, scrA, sortA, s, 0x0ffu);
+        int rc = radix_sort96(aw0, aw1, aw2, aidx, N, scrA, sortA, s, 0x0ffu, false, &c.launches);
         if (rc) return rc;
-        c.launches += 24;
     }
     c.counters[10] = h_desc[1];  // duplicate (cpu_id, id_in_run) pairs: order left stable
 
@@ -754,7 +845,7 @@ int build_tree(Context &c, const plan_lis_view &v, plan_params &p, int first_fil
     uint64_t G = 0;
     if (!p.no_ghost) {
         // over every particle of the file: an upper bound when a user box keeps fewer
-        k_ghost_total<<<grid_for((uint32_t)N64, 256), 256, 0, s>>>(tmp_pos, (uint32_t)N64, g, d_desc + 2);
+        k_ghost_total<<<std::min(grid_for((uint32_t)N64, 256), 152u * 8u), 256, 0, s>>>(tmp_pos, (uint32_t)N64, g, d_desc + 2);
         PLAN_CUDA(cudaMemcpyAsync(&G, d_desc + 2, 8, cudaMemcpyDeviceToHost, s));
         PLAN_CUDA(cudaStreamSynchronize(s));
         c.launches++;
@@ -829,6 +920,7 @@ int build_tree(Context &c, const plan_lis_view &v, plan_params &p, int first_fil
     PLAN_CUDA(cudaStreamSynchronize(s));
     c.launches++;
     double mn[3], mx[3];
+    c.scratch.used = 0;  // the octree takes its own
     for (int d = 0; d < 3; ++d) { mn[d] = h_mm[d]; mx[d] = h_mm[3 + d]; }
     for (int b = 1; b < mmb; ++b)
         for (int d = 0; d < 3; ++d) { mn[d] = std::min(h_mm[6 * b + d], mn[d]); mx[d] = std::max(h_mm[6 * b + 3 + d], mx[d]); }

@@ -124,9 +124,8 @@ int hop_groups(Context &c, const uint32_t *densest, double thr, HopGroups &out, 
     size_t sb = radix_sort96_scratch_bytes(m);
     void *scr2 = c.scratch.take(sb);
     if (!scr2) return kErrOutOfMemory;
-    rc = radix_sort96(w0, w1, w2, out.members, m, scr2, sb, s);
+    rc = radix_sort96(w0, w1, w2, out.members, m, scr2, sb, s, 0xfffu, false, &c.launches);
     if (rc) return rc;
-    c.launches += 36;
     // group table: one entry per root, ascending (the std::map order of src/tree.hpp:4855)
     uint32_t *flag = c.scratch.get<uint32_t>(m + 1), *rank = c.scratch.get<uint32_t>(m + 1);
     void *scr3 = c.scratch.take(scan_u32_scratch_bytes(m + 1));
@@ -146,6 +145,7 @@ int hop_groups(Context &c, const uint32_t *densest, double thr, HopGroups &out, 
     c.launches += 2;
     out.peak = nxt;  // root per tree point (valid for above-threshold points)
     out.above = above;
+    c.scratch.used = 0;  // later work on the stream may reuse it
     PLAN_CUDA(cudaGetLastError());
     return kOk;
 }

@@ -359,9 +359,8 @@ int morton_sort_std(Context &c, uint32_t *w0, uint32_t *w1, uint32_t *w2, uint32
         c.launches++;
     }
     // the final insertion sort keeps equal keys in place: a stable sort finishes
-    int rc = radix_sort96(w0, w1, w2, ix, n, scr, sb, s);
+    int rc = radix_sort96(w0, w1, w2, ix, n, scr, sb, s, 0xfffu, false, &c.launches);
     if (rc) return rc;
-    c.launches += 36;
     PLAN_CUDA(cudaGetLastError());
     return kOk;
 }

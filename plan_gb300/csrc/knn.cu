@@ -69,25 +69,6 @@ __global__ void __launch_bounds__(128) k_density_at(KTree t, const double *q3, c
     }
 }
 
-// ---------------------------------------------------------------- FP32-filtered kernels
-__global__ void k_split_points(const double4_32a *pos, uint32_t n, float4 *hi, float4 *lo) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double4_32a p = pos[i];
-    float hx = (float)p.x, hy = (float)p.y, hz = (float)p.z;
-    hi[i] = make_float4(hx, hy, hz, 0.f);
-    lo[i] = make_float4((float)(p.x - (double)hx), (float)(p.y - (double)hy), (float)(p.z - (double)hz), 0.f);
-}
-
-__global__ void k_split_nodes(const double4_32a *ncf, uint32_t n, float4 *hi, float4 *lo) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double4_32a c = ncf[i];
-    float hx = (float)c.x, hy = (float)c.y, hz = (float)c.z, hw = (float)c.w;
-    hi[i] = make_float4(hx, hy, hz, hw);
-    lo[i] = make_float4((float)(c.x - (double)hx), (float)(c.y - (double)hy), (float)(c.z - (double)hz), (float)(c.w - (double)hw));
-}
-
 template <int KMAX, int SPL>
 __global__ void __launch_bounds__(128) k_density_list(KTree t, const uint32_t *list, const uint32_t *nlist, uint32_t k, double fpo3,
                                                       SplineCells sc, double *dens, unsigned *err) {
@@ -378,22 +359,6 @@ int launch_by_k(uint32_t k, F f) {
 
 }  // namespace
 
-// FP32 hi/lo copies of points and node centres for the filtered kernels
-int ensure_split(Context &c, cudaStream_t s) {
-    DevTree &tr = c.tree;
-    if (tr.phi) return kOk;
-    tr.phi = c.arena.get<float4>(tr.Tu);
-    tr.plo = c.arena.get<float4>(tr.Tu);
-    tr.nhi = c.arena.get<float4>(tr.nodes);
-    tr.nlo = c.arena.get<float4>(tr.nodes);
-    if (c.arena.failed) return kErrOutOfMemory;
-    k_split_points<<<grid_for(tr.Tu, 256), 256, 0, s>>>(tr.pos, tr.Tu, tr.phi, tr.plo);
-    k_split_nodes<<<grid_for(tr.nodes, 256), 256, 0, s>>>(tr.ncf, tr.nodes, tr.nhi, tr.nlo);
-    c.launches += 2;
-    PLAN_CUDA(cudaGetLastError());
-    return kOk;
-}
-
 // Blocks for a list whose length only the device knows: enough to fill the GPU.
 static unsigned list_blocks(Context &c) {
     int sms = 152;
@@ -418,13 +383,11 @@ int launch_density(Context &c, const plan_params &p, uint32_t k, cudaStream_t s)
     if (k > 64) return kErrUnsupported;
     KTree t = ktree_of(c.tree);
     const double fpo3 = 3.14159265358979323846 * 4. / 3.;
-    int rc = ensure_split(c, s);
-    if (rc) return rc;
     FTree f{c.tree.phi, c.tree.plo, c.tree.nhi, c.tree.nlo};
     const uint32_t n = c.tree.Tu;
     const size_t mark = c.scratch.used;
     RedoLists redo;
-    rc = redo.take(c, n, s);
+    int rc = redo.take(c, n, s);
     if (rc) return rc;
     const SplineCells sc = c.fs.spline;
     const unsigned lb = list_blocks(c);
@@ -468,13 +431,11 @@ int launch_density(Context &c, const plan_params &p, uint32_t k, cudaStream_t s)
 int launch_densest(Context &c, const plan_params &p, uint32_t k, double threshold, uint32_t *densest, cudaStream_t s) {
     if (k > 64) return kErrUnsupported;
     KTree t = ktree_of(c.tree);
-    int rc = ensure_split(c, s);
-    if (rc) return rc;
     FTree f{c.tree.phi, c.tree.plo, c.tree.nhi, c.tree.nlo};
     const uint32_t n = c.tree.Tu;
     const size_t mark = c.scratch.used;
     RedoLists redo;
-    rc = redo.take(c, n, s);
+    int rc = redo.take(c, n, s);
     if (rc) return rc;
     const unsigned lb = list_blocks(c);
     PLAN_CUDA(cudaEventRecord(c.kev[0], s));
@@ -508,8 +469,6 @@ int launch_density_at(Context &c, const double *d_q3, const double *d_est, uint3
     KTree t = ktree_of(c.tree);
     const double fpo3 = 3.14159265358979323846 * 4. / 3.;
     const bool spl = !c.fs.median_kernel;
-    int rc = ensure_split(c, s);
-    if (rc) return rc;
     FTree f{c.tree.phi, c.tree.plo, c.tree.nhi, c.tree.nlo};
     const size_t mark = c.scratch.used;
     uint32_t *heap = c.scratch.get<uint32_t>(nq + 1), *nheap = c.scratch.get<uint32_t>(4);
@@ -519,7 +478,7 @@ int launch_density_at(Context &c, const double *d_q3, const double *d_est, uint3
     }
     PLAN_CUDA(cudaMemsetAsync(nheap, 0, 4, s));
     // a warp per query; the queries with distance ties go to the exact heap path
-    rc = launch_by_k(k, [&](auto km, int threads) {
+    int rc = launch_by_k(k, [&](auto km, int threads) {
         constexpr int KM = decltype(km)::value;
         auto kern = spl ? k_exact_w<kOpSpline> : k_exact_w<kOpMedian>;
         kern<<<(nq + kWkWarps - 1) / kWkWarps, 32 * kWkWarps, 0, s>>>(t, f, d_q3, d_est, 0.0, nullptr, nullptr, nq, k, fpo3, c.fs.spline,
@@ -546,8 +505,6 @@ int knn_positions(Context &c, const double *pos3, uint32_t nq, uint32_t k, doubl
     if (k > 128) return kErrUnsupported;
     if (nq == 0) return kOk;
     cudaStream_t s = c.stream;
-    int rc = ensure_split(c, s);
-    if (rc) return rc;
     StreamBuf<double> d_q(s), d_d(s);
     StreamBuf<uint32_t> d_i(s), d_redo(s);
     PLAN_CUDA(d_q.alloc((size_t)nq * 3));
@@ -558,7 +515,7 @@ int knn_positions(Context &c, const double *pos3, uint32_t nq, uint32_t k, doubl
     PLAN_CUDA(cudaMemcpyAsync(d_q.p, pos3, (size_t)nq * 3 * 8, cudaMemcpyHostToDevice, s));
     KTree t = ktree_of(c.tree);
     FTree f{c.tree.phi, c.tree.plo, c.tree.nhi, c.tree.nlo};
-    rc = launch_by_k(k, [&](auto km, int threads) {
+    int rc = launch_by_k(k, [&](auto km, int threads) {
         constexpr int KM = decltype(km)::value;
         k_exact_w<kOpKnn><<<(nq + kWkWarps - 1) / kWkWarps, 32 * kWkWarps, 0, s>>>(t, f, d_q.p, nullptr, est, nullptr, nullptr, nq, k, 0.0,
                                                                                 c.fs.spline, WkOut{nullptr, d_i.p, d_d.p, d_redo.p + 1, d_redo.p},

@@ -117,7 +117,6 @@ int write_parlists_device(Context &c, const plan_catalogue &cat, int file_number
 int knn_positions(Context &c, const double *pos3, uint32_t nq, uint32_t k, double est, uint32_t *idx, double *dr2);
 
 // Kernel launch helpers shared across translation units
-int ensure_split(Context &c, cudaStream_t s);  // the tree's FP32 hi/lo copies
 int launch_density(Context &c, const plan_params &p, uint32_t k, cudaStream_t s);
 int launch_densest(Context &c, const plan_params &p, uint32_t k, double threshold, uint32_t *densest, cudaStream_t s);
 

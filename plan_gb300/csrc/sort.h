@@ -11,10 +11,11 @@ namespace plan {
 
 // Stable LSD radix sort of (w2:w1:w0) 96-bit keys carrying `payload`, in place.
 // pass_mask selects which of the 12 byte-digits may be sorted (bit p = byte p, byte 0 is
-// the least significant byte of w0); constant digits are skipped automatically.
+// the least significant byte of w0); constant digits are skipped automatically. few_low: keys
+// with equal w2 and w1 are expected to be few. *launched grows by the kernels launched.
 size_t radix_sort96_scratch_bytes(size_t n);
 int radix_sort96(uint32_t *w0, uint32_t *w1, uint32_t *w2, uint32_t *payload, size_t n, void *scratch, size_t scratch_bytes,
-                 cudaStream_t stream, unsigned pass_mask = 0xfffu);
+                 cudaStream_t stream, unsigned pass_mask = 0xfffu, bool few_low = false, uint64_t *launched = nullptr);
 
 // Exclusive scan of n u32 values (out may alias in); *total receives the sum when non-null
 // (device pointer).
