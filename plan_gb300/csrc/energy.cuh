@@ -61,8 +61,36 @@ struct PairParticle {
     float x, y, z, m;
 };
 
-// One row particle p against the columns col[0, cn) of its tile: sum of m_q / r in FP32 with
-// Neumaier's compensation (the returned pair is sum, compensation); the caller multiplies by
+// A queue item of the GPU pass: row tile ti and up to Q column tiles from tj on (one slot of the
+// result each). Wide items share the FP64 sum of their rows over more pairs; Q grows with the
+// group alone, so that a group's sums do not depend on the batch, and only where the group by
+// itself still makes more items than the GPU has SMs (272 at 32 row tiles, 544 at 64).
+PLAN_EN_HD inline uint32_t strip_of(uint64_t T) { return T >= 64 ? 4u : T >= 32 ? 2u : 1u; }
+
+// Items of the last U row tiles: the u-th of them from the end has u column tiles.
+PLAN_EN_HD inline uint64_t strip_items_below(uint64_t U, uint64_t Q) {
+    const uint64_t a = U / Q, b = U % Q;
+    return Q * (a * (a + 1) / 2) + b * (a + 1);
+}
+
+PLAN_EN_HD inline uint64_t strip_items(uint64_t T) { return strip_items_below(T, strip_of(T)); }
+
+// Item `local` of a group of T row tiles: rows from the first, strips from the diagonal on.
+PLAN_EN_HD inline void strip_of_item(uint64_t local, uint64_t T, uint64_t &ti, uint64_t &tj, uint64_t &te) {
+    const uint64_t Q = strip_of(T), all = strip_items_below(T, Q);
+    uint64_t lo = 0, hi = T - 1;  // the last row tile whose first item is not after local
+    while (lo < hi) {
+        const uint64_t mid = (lo + hi + 1) / 2;
+        if (all - strip_items_below(T - mid, Q) <= local) lo = mid;
+        else hi = mid - 1;
+    }
+    ti = lo;
+    tj = ti + Q * (local - (all - strip_items_below(T - ti, Q)));
+    te = tj + Q < T ? tj + Q : T;
+}
+
+// One row particle p against the columns col[0, cn) of its tile: m_q / r in FP32 added to sum with
+// Neumaier's compensation (in comp); the caller multiplies by
 // m_p in FP64, so no pair's mass product is rounded in FP32 (equal masses would otherwise
 // round every term the same way). Columns k <= skip_to are left out (a diagonal tile: each
 // pair once); coincident pairs are left out and counted. On the GPU 1/r is the hardware
@@ -70,7 +98,7 @@ struct PairParticle {
 // at most, against the stated 10^-6 on the sums); the CPU replay divides by the square root.
 PLAN_EN_HD inline void pair_row_sum(const PairParticle &p, const PairParticle *col, uint32_t cn, int skip_to, float &sum, float &comp,
                                     uint32_t &zeros) {
-    float s = 0.f, c = 0.f;
+    float s = sum, c = comp;
     for (uint32_t k = 0; k < cn; ++k) {
         if ((int)k <= skip_to) continue;
         const PairParticle q = col[k];
