@@ -26,6 +26,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <numeric>
+#include <unordered_map>
 #include <vector>
 
 #include "catalogue.h"
@@ -43,7 +44,9 @@ namespace {
 
 constexpr uint32_t kNone = 0xffffffffu;
 constexpr int kSmallSort = 2048;
-constexpr uint32_t kBigKinematics = 4096;  // larger clumps sum with ordered_sum_chunk
+// Clumps with more members sum with ordered_sum_chunk, a block each: a chunk of 256 takes 5,000
+// cycles there and 16,400 in a lane's chain of FP64 adds.
+constexpr uint32_t kBigKinematics = 512;
 
 struct CP {
     double G, shear, Omega;
@@ -339,6 +342,7 @@ __global__ void __launch_bounds__(128) k_dispersion(const uint32_t *list, uint32
     if (t >= n) return;
     const uint32_t s = list[t];
     const uint32_t o = ct.moff[s], m = ct.mn[s];
+    if (m > kBigKinematics) return;  // k_dispersion_big
     if (m == 0) {
         if (lane == 0) too_large[t] = 0;
         return;
@@ -359,6 +363,30 @@ __global__ void __launch_bounds__(128) k_dispersion(const uint32_t *list, uint32
     if (lane == 0) {
         double x = tol * P.dist[o + m - 1];
         too_large[t] = (acc / (double)m > x * x) ? 1 : 0;
+    }
+}
+
+// The same for larger clumps: the block stages 256 squares at a time (the next ones on their way
+// meanwhile), warp 0 adds them in order.
+__global__ void __launch_bounds__(256) k_dispersion_big(const uint32_t *list, CT ct, Pool P, double tol, uint8_t *too_large) {
+    __shared__ __align__(16) double term[kSumStage];
+    __shared__ uint2 steps[kSumChunk];
+    const uint32_t s = list[blockIdx.x];
+    const uint32_t o = ct.moff[s], m = ct.mn[s];
+    if (m <= kBigKinematics) return;
+    const uint32_t at = sum_slot(threadIdx.x);
+    double acc = 0.0, d = P.dist[o + threadIdx.x];
+    for (uint32_t base = 0; base < m; base += kSumChunk) {
+        term[at] = d * d;
+        __syncthreads();
+        const uint32_t k = base + kSumChunk + threadIdx.x;
+        d = k < m ? P.dist[o + k] : 0.0;
+        if (threadIdx.x < 32) ordered_sum_chunk(term, acc, steps);
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        const double x = tol * P.dist[o + m - 1];
+        too_large[blockIdx.x] = (acc / (double)m > x * x) ? 1 : 0;
     }
 }
 
@@ -406,6 +434,15 @@ __global__ void k_large_scatter(const uint32_t *list, uint32_t nl, const uint32_
 }
 
 // ---------------------------------------------------------------- merge sweeps
+// the slot of every live key, the last one of equal keys (slot_of_key starts at kNone)
+__global__ void k_slot_of_key(uint32_t C, CT ct, uint32_t *slot_of_key) {
+    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= C || !ct.alive[s]) return;
+    uint32_t *at = &slot_of_key[ct.key[s]];
+    uint32_t was = atomicCAS(at, kNone, s);
+    if (was != kNone) atomicMax(at, s);
+}
+
 __global__ void k_mark_live(uint32_t C, CT ct, uint32_t *flag) {
     uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= C) return;
@@ -466,6 +503,58 @@ __global__ void k_ball_clumps(int pass, uint32_t C, CT ct, KTree t, bool hill_mo
              },
              err);
     if (pass == 0) cnt[s] = n;
+}
+
+// The same search with a warp per clump over all nct clump points (in tree order, which is the
+// traversal's), for clump sets where that is the smaller work: a thread's FP64 walk of the clump
+// tree took 0.1 ms for 100 clumps, this 6 us (0.1 ms for 1,600, growing with the square of the
+// number from there on; the walk's time grows with its logarithm). The ball holds the points within it, decided in FP32 unless too
+// close to its surface; there the point takes the walk's own way, the FP64 tests of the nodes
+// above it. (A point inside the ball by more than the rounding of its key lies in nodes that all
+// meet the ball, one outside by as much in none that it contains.)
+constexpr uint32_t kBruteClumps = 8192;
+
+__device__ inline bool ball_takes(const KTree &t, uint32_t q, double x, double y, double z, double r) {
+    uint32_t n = t.leaf_of[q];
+    bool in = point_dr2(x, y, z, t.pos[q]) <= r * r;
+    for (int guard = 0; guard < 40; ++guard) {
+        const double4_32a nc = t.ncf[n];
+        if (node_contained(nc, x, y, z, r)) in = true;
+        else if (!node_intersects(nc, x, y, z, r)) in = false;
+        if (n == 0) break;
+        n = t.npar[n];
+    }
+    return in;
+}
+
+__global__ void __launch_bounds__(128) k_ball_brute(int pass, uint32_t C, CT ct, KTree t, FTree ft, uint32_t nct, bool hill_mode, double hillf,
+                                                    double max_radius, uint32_t *cnt, const uint32_t *off, uint32_t *cand) {
+    const uint32_t lane = threadIdx.x & 31, s = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (s >= C) return;
+    if (!(ct.alive[s] && ct.mask[s])) {
+        if (pass == 0 && lane == 0) cnt[s] = 0;
+        return;
+    }
+    const double4_32a c = ct.com[s];
+    const double r = merge_radius(ct, s, hill_mode, hillf) + max_radius;
+    const float4 qh = make_float4((float)c.x, (float)c.y, (float)c.z, 0.f);
+    const float4 ql = make_float4((float)(c.x - (double)qh.x), (float)(c.y - (double)qh.y), (float)(c.z - (double)qh.z), 0.f);
+    const float rr = (float)(r * r), skin = 4.f * (float)r * (float)t.box.half_width * 1.862645149230957e-09f;  // 2^-29 of the box
+    const float inner = rr * (1.f - 2.f * kRel) - skin, outer = rr * (1.f + 2.f * kRel) + skin;
+    uint32_t n = 0, o = pass ? off[s] : 0;
+    for (uint32_t q0 = 0; q0 < nct; q0 += 32) {
+        const uint32_t q = q0 + lane;
+        bool in = false;
+        if (q < nct) {
+            const float v = f_dr2(qh, ql, ft.phi[q], ft.plo[q]);
+            if (f_hi(v) < inner) in = true;
+            else if (!(f_lo(v) > outer)) in = ball_takes(t, q, c.x, c.y, c.z, r);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (pass && in) cand[o + n + __popc(m & ((1u << lane) - 1u))] = q;
+        n += __popc(m);
+    }
+    if (pass == 0 && lane == 0) cnt[s] = n;
 }
 
 // Per candidate pair: contained, or intersecting and bound (then the saddle decides).
@@ -1641,6 +1730,22 @@ __global__ void k_rip(uint32_t C, CT ct, Pool P, uint8_t *pending, uint32_t *cha
 
 // CalculateAngularMomentum sums (src/tree.hpp:4721-4747), unnormalised: per-member terms by
 // the warp, the three running sums in member order by lanes 0..2
+__device__ __forceinline__ void angmom_terms(const double4_32a &p, const double4_32a &v, const double4_32a &c, const double4_32a &vc, const CP &cp,
+                                             double &jx, double &jy, double &jz) {
+    double drx = p.x - c.x, dry = p.y - c.y, drz = p.z - c.z;
+    double sx = 0. * p.x, sy = cp.shear * p.x, sz = 0. * p.x;
+    double cx0 = 0. * c.x, cy0 = cp.shear * c.x, cz0 = 0. * c.x;
+    double dvx = (v.x - sx) - (vc.x - cx0), dvy = (v.y - sy) - (vc.y - cy0), dvz = (v.z - sz) - (vc.z - cz0);
+    double tx = dry * dvz - drz * dvy, ty = drz * dvx - drx * dvz, tz = drx * dvy - dry * dvx;
+    double ax = -drx * drz, ay = -dry * drz, az = (drx * drx + dry * dry);
+    tx = tx + cp.Omega * ax;
+    ty = ty + cp.Omega * ay;
+    tz = tz + cp.Omega * az;
+    jx = p.w * tx;
+    jy = p.w * ty;
+    jz = p.w * tz;
+}
+
 __global__ void __launch_bounds__(128) k_angmom(const uint32_t *list, uint32_t n, CT ct, Pool P, const double4_32a *pos,
                                                 const double4_32a *vel, CP cp) {
     __shared__ double tile[4][3][32];
@@ -1649,6 +1754,7 @@ __global__ void __launch_bounds__(128) k_angmom(const uint32_t *list, uint32_t n
     if (t >= n) return;
     const uint32_t s = list[t];
     const uint32_t o = ct.moff[s], m = ct.mn[s];
+    if (m > kBigKinematics) return;  // k_angmom_big
     const double4_32a c = ct.com[s], vc = ct.vcom[s];
     double acc = 0;
     for (uint32_t base = 0; base < m; base += 32) {
@@ -1656,18 +1762,7 @@ __global__ void __launch_bounds__(128) k_angmom(const uint32_t *list, uint32_t n
         if (k < m) {
             uint32_t i = P.idx[o + k];
             double4_32a p = pos[i], v = vel[i];
-            double drx = p.x - c.x, dry = p.y - c.y, drz = p.z - c.z;
-            double sx = 0. * p.x, sy = cp.shear * p.x, sz = 0. * p.x;
-            double cx0 = 0. * c.x, cy0 = cp.shear * c.x, cz0 = 0. * c.x;
-            double dvx = (v.x - sx) - (vc.x - cx0), dvy = (v.y - sy) - (vc.y - cy0), dvz = (v.z - sz) - (vc.z - cz0);
-            double tx = dry * dvz - drz * dvy, ty = drz * dvx - drx * dvz, tz = drx * dvy - dry * dvx;
-            double ax = -drx * drz, ay = -dry * drz, az = (drx * drx + dry * dry);
-            tx = tx + cp.Omega * ax;
-            ty = ty + cp.Omega * ay;
-            tz = tz + cp.Omega * az;
-            tile[wid][0][lane] = p.w * tx;
-            tile[wid][1][lane] = p.w * ty;
-            tile[wid][2][lane] = p.w * tz;
+            angmom_terms(p, v, c, vc, cp, tile[wid][0][lane], tile[wid][1][lane], tile[wid][2][lane]);
         }
         __syncwarp();
         const uint32_t cnt = min(32u, m - base);
@@ -1677,6 +1772,45 @@ __global__ void __launch_bounds__(128) k_angmom(const uint32_t *list, uint32_t n
     }
     double jx = __shfl_sync(0xffffffffu, acc, 0), jy = __shfl_sync(0xffffffffu, acc, 1), jz = __shfl_sync(0xffffffffu, acc, 2);
     if (lane == 0) ct.J[s] = make_double4_32a(jx, jy, jz, 0);
+}
+
+// The same for larger clumps, as k_dispersion_big: three sums in three warps.
+__global__ void __launch_bounds__(256) k_angmom_big(const uint32_t *list, CT ct, Pool P, const double4_32a *pos, const double4_32a *vel, CP cp) {
+    __shared__ __align__(16) double term[3 * kSumStage];
+    __shared__ uint2 steps[3 * kSumChunk];
+    __shared__ double res[3];
+    const uint32_t s = list[blockIdx.x];
+    const uint32_t o = ct.moff[s], m = ct.mn[s];
+    if (m <= kBigKinematics) return;
+    const double4_32a c = ct.com[s], vc = ct.vcom[s];
+    const int w = threadIdx.x >> 5;
+    const uint32_t at = sum_slot(threadIdx.x);
+    double acc = 0.0;
+    double4_32a p, v;
+    bool have;
+    auto fetch = [&](uint32_t k) {
+        have = k < m;
+        if (have) {
+            const uint32_t i = P.idx[o + k];
+            p = pos[i];
+            v = vel[i];
+        }
+    };
+    fetch(threadIdx.x);
+    for (uint32_t base = 0; base < m; base += kSumChunk) {
+        double jx = 0.0, jy = 0.0, jz = 0.0;
+        if (have) angmom_terms(p, v, c, vc, cp, jx, jy, jz);
+        term[at] = jx;
+        term[kSumStage + at] = jy;
+        term[2 * kSumStage + at] = jz;
+        __syncthreads();
+        fetch(base + kSumChunk + threadIdx.x);
+        if (w < 3) ordered_sum_chunk(term + w * kSumStage, acc, steps + w * kSumChunk);
+        __syncthreads();
+    }
+    if (w < 3 && (threadIdx.x & 31) == 0) res[w] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) ct.J[s] = make_double4_32a(res[0], res[1], res[2], 0);
 }
 
 // copy every live segment into the other pool buffer at packed offsets
@@ -1870,7 +2004,8 @@ struct Stage {
         int rc = up_list(list, d_list);
         if (rc) return rc;
         k_dispersion<<<(unsigned)((list.size() + 3) / 4), 128, 0, s>>>(d_list, (uint32_t)list.size(), ct, P, tol, d_flag8);
-        c.launches++;
+        k_dispersion_big<<<(unsigned)list.size(), 256, 0, s>>>(d_list, ct, P, tol, d_flag8);
+        c.launches += 2;
         return down(res, d_flag8, list.size());
     }
 
@@ -2167,7 +2302,11 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
             // candidates
             uint32_t ncand = 0;
             if (nct) {
-                k_ball_clumps<<<grid_for(C, 128), 128, 0, s>>>(0, C, ct, kct, hill_mode, hillf, max_radius, d_cnt, nullptr, nullptr, c.d_err);
+                if (nct <= kBruteClumps)
+                    k_ball_brute<<<(C + 3) / 4, 128, 0, s>>>(0, C, ct, kct, FTree{ctree.phi, ctree.plo, ctree.nhi, ctree.nlo}, ctree.Tu, hill_mode, hillf,
+                                                             max_radius, d_cnt, nullptr, nullptr);
+                else
+                    k_ball_clumps<<<grid_for(C, 128), 128, 0, s>>>(0, C, ct, kct, hill_mode, hillf, max_radius, d_cnt, nullptr, nullptr, c.d_err);
                 const size_t sm2 = c.scratch.used;
                 void *scr2 = c.scratch.take(sb);
                 rc = scan_u32(d_cnt, d_off, C, d_tot, scr2, sb, s);
@@ -2188,7 +2327,11 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
             PLAN_CUDA(cudaMemsetAsync(d_nrl, 0, 4, s));
             uint32_t nsaddle = 0;
             if (ncand) {
-                k_ball_clumps<<<grid_for(C, 128), 128, 0, s>>>(1, C, ct, kct, hill_mode, hillf, max_radius, d_cnt, d_off, d_cand, c.d_err);
+                if (nct <= kBruteClumps)
+                    k_ball_brute<<<(C + 3) / 4, 128, 0, s>>>(1, C, ct, kct, FTree{ctree.phi, ctree.plo, ctree.nhi, ctree.nlo}, ctree.Tu, hill_mode, hillf,
+                                                             max_radius, d_cnt, d_off, d_cand);
+                else
+                    k_ball_clumps<<<grid_for(C, 128), 128, 0, s>>>(1, C, ct, kct, hill_mode, hillf, max_radius, d_cnt, d_off, d_cand, c.d_err);
                 k_cand_owner<<<grid_for(C, 256), 256, 0, s>>>(C, d_cnt, d_off, d_cp1);
                 PLAN_CUDA(cudaMemsetAsync(st.d_u + 16, 0, 4, s));
                 k_pair_eval<<<grid_for(ncand, 128), 128, 0, s>>>(ncand, d_cp1, d_cand, ctree.vel, ct, st.slot_of_key, st.cp, hill_mode,
@@ -2303,14 +2446,21 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
         std::vector<uint32_t> keys_now;
         rc = st.down(keys_now, ct.key, C);
         if (rc) return rc;
-        std::vector<uint32_t> sok(Tu, kNone);
+        std::unordered_map<uint32_t, uint32_t> sok;  // the last slot of each key among the live ones
         for (uint32_t i = 0; i < C; ++i) if (alive[i]) sok[keys_now[i]] = i;
-        for (uint32_t k : dk) if (sok[k] != kNone) { alive[sok[k]] = 0; }
-        if (delete_count < start_num && sok[0] != kNone && alive[sok[0]]) { alive[sok[0]] = 0; ++quirk; }
-        std::vector<uint32_t> sok_dev(Tu, kNone);
-        for (uint32_t i = 0; i < C; ++i) if (alive[i]) sok_dev[keys_now[i]] = i;
+        auto drop = [&](uint32_t k) {
+            auto it = sok.find(k);
+            if (it == sok.end()) return false;
+            const bool was = alive[it->second] != 0;
+            alive[it->second] = 0;
+            return was;
+        };
+        for (uint32_t k : dk) drop(k);
+        if (delete_count < start_num && drop(0)) ++quirk;
         PLAN_CUDA(cudaMemcpyAsync(ct.alive, alive.data(), C, cudaMemcpyHostToDevice, s));
-        PLAN_CUDA(cudaMemcpyAsync(st.slot_of_key, sok_dev.data(), (size_t)Tu * 4, cudaMemcpyHostToDevice, s));
+        PLAN_CUDA(cudaMemsetAsync(st.slot_of_key, 0xff, (size_t)Tu * 4, s));
+        k_slot_of_key<<<grid_for(C, 256), 256, 0, s>>>(C, ct, st.slot_of_key);
+        c.launches++;
         rc = st.live_order(live);
         if (rc) return rc;
         num_planetesimals = (uint32_t)live.size() + ((delete_count < start_num && quirk) ? 0 : 0);
@@ -3085,7 +3235,8 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
         rc = st.up_list(live, st.d_list);
         if (rc) return rc;
         k_angmom<<<(unsigned)((live.size() + 3) / 4), 128, 0, s>>>(st.d_list, (uint32_t)live.size(), ct, P, tr.pos, tr.vel, st.cp);
-        c.launches++;
+        k_angmom_big<<<(unsigned)live.size(), 256, 0, s>>>(st.d_list, ct, P, tr.pos, tr.vel, st.cp);
+        c.launches += 2;
     }
     cudaEventRecord(ev[5], s);
     PLAN_CUDA(cudaStreamSynchronize(s));

@@ -80,6 +80,30 @@ __global__ void k_chunk_scan(const uint32_t *in, uint32_t *out, size_t n, const 
     }
 }
 
+// Up to kOneBlock values: one block, kOneBlock / kT consecutive values per thread (three launches
+// for a few thousand values cost three times as much).
+constexpr int kOneBlock = 16 * kT;
+
+__global__ void __launch_bounds__(kT) k_scan_one(const uint32_t *in, uint32_t *out, int n, uint32_t *d_total) {
+    __shared__ uint32_t s_warp[32];
+    constexpr int kMine = kOneBlock / kT;
+    const int per = (n + kT - 1) / kT, base = threadIdx.x * per;
+    uint32_t v[kMine], s = 0;
+#pragma unroll
+    for (int k = 0; k < kMine; ++k) {
+        v[k] = k < per && base + k < n ? in[base + k] : 0;
+        s += v[k];
+    }
+    uint32_t tot;
+    uint32_t e = block_exclusive(s, s_warp, tot);
+#pragma unroll
+    for (int k = 0; k < kMine; ++k) {
+        if (k < per && base + k < n) out[base + k] = e;
+        e += v[k];
+    }
+    if (threadIdx.x == 0 && d_total) *d_total = tot;
+}
+
 }  // namespace
 
 size_t scan_u32_scratch_bytes(size_t n) { return ((n + kChunk - 1) / kChunk + 1) * sizeof(uint32_t) + 256; }
@@ -88,6 +112,11 @@ int scan_u32(const uint32_t *in, uint32_t *out, size_t n, uint32_t *d_total, voi
     if (scratch_bytes < scan_u32_scratch_bytes(n)) return kErrArgument;
     if (n == 0) {
         if (d_total) PLAN_CUDA(cudaMemsetAsync(d_total, 0, 4, stream));
+        return kOk;
+    }
+    if (n <= (size_t)kOneBlock) {
+        k_scan_one<<<1, kT, 0, stream>>>(in, out, (int)n, d_total);
+        PLAN_CUDA(cudaGetLastError());
         return kOk;
     }
     size_t m = (n + kChunk - 1) / kChunk;
