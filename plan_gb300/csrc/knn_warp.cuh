@@ -112,16 +112,16 @@ __device__ __forceinline__ uint32_t wk_select(const uint32_t *key, uint32_t n, u
 }
 
 // Keeps the buffered candidates with keys at or below limit, in place; returns their number.
-__device__ __forceinline__ uint32_t wk_filter(WkBuf &s, uint32_t n, uint32_t limit) {
+__device__ __forceinline__ uint32_t wk_filter(uint32_t *key, uint32_t *ix, uint32_t n, uint32_t limit) {
     const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1u;
     uint32_t m = 0;
     for (uint32_t j = 0; j < n; j += 32) {
-        const uint32_t v = j + lane < n ? s.key[j + lane] : 0xffffffffu, p = j + lane < n ? s.ix[j + lane] : 0u;
+        const uint32_t v = j + lane < n ? key[j + lane] : 0xffffffffu, p = j + lane < n ? ix[j + lane] : 0u;
         const bool keep = j + lane < n && v <= limit;
         const unsigned b = __ballot_sync(0xffffffffu, keep);
         if (keep) {
-            s.key[m + __popc(b & below)] = v;
-            s.ix[m + __popc(b & below)] = p;
+            key[m + __popc(b & below)] = v;
+            ix[m + __popc(b & below)] = p;
         }
         m += __popc(b);
         __syncwarp();
@@ -131,13 +131,13 @@ __device__ __forceinline__ uint32_t wk_filter(WkBuf &s, uint32_t n, uint32_t lim
 
 // Drops the candidates that cannot be among the k nearest: tau becomes a key that no member of
 // the exact k-set exceeds.
-__device__ __forceinline__ void wk_compact(WkBuf &s, uint32_t k, uint32_t &n, uint32_t &tau) {
+__device__ __forceinline__ void wk_compact(uint32_t *key, uint32_t *ix, uint32_t k, uint32_t &n, uint32_t &tau) {
     __syncwarp();
     if (n < k) return;
     uint32_t count;
-    const float thr = f_hi(__uint_as_float(wk_select(s.key, n, k, count)));
+    const float thr = f_hi(__uint_as_float(wk_select(key, n, k, count)));
     tau = min(tau, __float_as_uint((thr + 2e-24f) * (1.f + 4.f * kRel)));
-    n = wk_filter(s, n, tau);
+    n = wk_filter(key, ix, n, tau);
 }
 
 // The walk. False when candidates at equal distances overflow the buffer. visited < k only
@@ -158,7 +158,7 @@ __device__ inline bool wk_collect(const KTree &t, const FTree &f, const WkQuery 
             unsigned m = __ballot_sync(full, v <= tau);
             if (!m) return;
             if (n + __popc(m) > kWkPoints) {
-                wk_compact(s, k, n, tau);
+                wk_compact(s.key, s.ix, k, n, tau);
                 m = __ballot_sync(full, v <= tau);
                 if (n + __popc(m) > kWkPoints) {
                     over = true;
@@ -253,7 +253,7 @@ __device__ __forceinline__ bool wk_kset(WkBuf &s, uint32_t k, uint32_t n, uint32
     in = __reduce_max_sync(0xffffffffu, in);
     out = __reduce_min_sync(0xffffffffu, out);
     if (!(f_hi(__uint_as_float(in)) < f_lo(__uint_as_float(out)))) return false;
-    wk_filter(s, n, T);
+    wk_filter(s.key, s.ix, n, T);
     return true;
 }
 
@@ -291,7 +291,7 @@ __device__ inline void warp_sort_pairs(unsigned long long *key, uint32_t *ix, ui
 // members, or the k-th and the next, are equally far: their order is the library heap's.
 __device__ __forceinline__ bool wk_sorted(const KTree &t, const WkQuery &q, WkBuf &s, uint32_t k, uint32_t n, uint32_t tau) {
     const uint32_t lane = threadIdx.x & 31;
-    wk_compact(s, k, n, tau);
+    wk_compact(s.key, s.ix, k, n, tau);
     if (n < k || n > kWkExact) return false;
     __syncwarp();
     for (uint32_t j = lane; j < n; j += 32) {
