@@ -300,30 +300,83 @@ __global__ void k_lib_order(const uint32_t *list, uint32_t n, CT ct, Pool P, con
 }
 
 // radii after a sort (src/tree.hpp:4461-4511)
-__global__ void k_one10th(const uint32_t *list, CT ct, Pool P, const double4_32a *pos, const double *dens) {
-    __shared__ uint32_t s_in, s_out;
+//
+// A block per clump: four gathers of densities on their way per thread; the outer mass in chunks
+// of the integer sum, where masses are not negative (the running sum then never falls, and the
+// chunk that passes the limit is the only one added member by member). The largest clump of
+// 262,144 particles (45,800 members) took 0.21 ms with one gather at a time and a thread's adds,
+// now 0.06.
+__global__ void __launch_bounds__(256) k_one10th(const uint32_t *list, CT ct, Pool P, const double4_32a *pos, const double *dens) {
+    __shared__ __align__(16) double term[kSumStage];
+    __shared__ uint2 steps[kSumChunk];
+    __shared__ uint32_t s_in, s_out, s_bad, s_at;
     uint32_t s = list[blockIdx.x];
-    const uint32_t o = ct.moff[s], m = ct.mn[s];
+    const uint32_t o = ct.moff[s], m = ct.mn[s], tid = threadIdx.x, lane = tid & 31;
     if (m == 0) return;
-    if (threadIdx.x == 0) { s_in = kNone; s_out = 0; }
-    __syncthreads();
-    const double tenth = dens[P.idx[o + m / 2]] / 10.;
-    for (uint32_t k = threadIdx.x; k < m; k += blockDim.x) {
-        double d = dens[P.idx[o + k]];
-        if (d < tenth) atomicMin(&s_in, k);       // first member below a tenth of the median's density
-        if (d > tenth) atomicMax(&s_out, k + 1);  // last member above it (stored +1)
+    if (tid == 0) {
+        s_in = kNone;
+        s_out = 0;
+        s_bad = 0;
+        s_at = kNone;
     }
     __syncthreads();
-    if (threadIdx.x != 0) return;
+    const double tenth = dens[P.idx[o + m / 2]] / 10.;
+    uint32_t in = kNone, out = 0;  // first member below a tenth of the median's density, last one above it (+1)
+    constexpr int kIn = 4;
+    for (uint32_t k0 = tid; k0 < m; k0 += kIn * 256) {
+        double d[kIn];
+#pragma unroll
+        for (int j = 0; j < kIn; ++j) d[j] = k0 + j * 256 < m ? dens[P.idx[o + k0 + j * 256]] : tenth;
+#pragma unroll
+        for (int j = 0; j < kIn; ++j) {
+            if (d[j] < tenth) in = min(in, k0 + j * 256);
+            if (d[j] > tenth) out = max(out, k0 + j * 256 + 1);
+        }
+    }
+    in = __reduce_min_sync(0xffffffffu, in);
+    out = __reduce_max_sync(0xffffffffu, out);
+    if (lane == 0) {
+        atomicMin(&s_in, in);
+        atomicMax(&s_out, out);
+    }
+    // r: the member, counted from the outside, at which the mass passes a twentieth
+    const double tenth_mass = ct.M[s] * (1.0 - 0.95);
+    const uint32_t at = sum_slot(tid);
+    double tm = 0.;
+    double w = tid < m ? pos[P.idx[o + m - 1 - tid]].w : 0.;
+    for (uint32_t base = 0; base < m; base += kSumChunk) {
+        const uint32_t cnt = min((uint32_t)kSumChunk, m - base), k = base + kSumChunk + tid;
+        term[at] = w;
+        if (!(w >= 0.)) s_bad = 1;
+        __syncthreads();
+        w = k < m ? pos[P.idx[o + m - 1 - k]].w : 0.;
+        if (tid < 32) {
+            bool serial = s_bad != 0 || m <= kBigKinematics;
+            double end = tm;
+            if (!serial) {
+                ordered_sum_chunk(term, end, steps);
+                serial = end > tenth_mass;
+            }
+            if (serial) {
+                for (uint32_t j = 0; j < cnt; ++j) {
+                    tm = tm + term[sum_slot(j)];
+                    if (tm > tenth_mass) {
+                        if (lane == 0) s_at = base + j;
+                        break;
+                    }
+                }
+            } else {
+                tm = end;
+            }
+        }
+        __syncthreads();
+        if (s_at != kNone) break;
+    }
+    if (tid != 0) return;
+    const uint32_t r = s_at != kNone ? m - s_at : 0;
     double rin = (s_in != kNone) ? P.dist[o + s_in] : P.dist[o + m - 1];
     double rout = P.dist[o + (s_out ? s_out - 1 : 0)];
     double r10 = (rin + rout) / 2.;
-    double tm = 0., tenth_mass = ct.M[s] * (1.0 - 0.95);
-    uint32_t r = m;
-    for (; r > 0; --r) {
-        tm = tm + pos[P.idx[o + r - 1]].w;
-        if (tm > tenth_mass) break;
-    }
     double r2s = P.dist[o + (r ? r - 1 : 0)];
     if (rin > 0 && rout / rin > 2.5) r10 = (r2s < rout) ? r2s : rout;
     else r10 = (r2s < r10) ? r2s : r10;
@@ -507,8 +560,8 @@ __global__ void k_ball_clumps(int pass, uint32_t C, CT ct, KTree t, bool hill_mo
 
 // The same search with a warp per clump over all nct clump points (in tree order, which is the
 // traversal's), for clump sets where that is the smaller work: a thread's FP64 walk of the clump
-// tree took 0.1 ms for 100 clumps, this 6 us (0.1 ms for 1,600, growing with the square of the
-// number from there on; the walk's time grows with its logarithm). The ball holds the points within it, decided in FP32 unless too
+// tree took 0.1 ms for 100 clumps, this 6 us (0.03 ms for 1,600, growing with the square of the
+// number; the walk's time grows with its logarithm). The ball holds the points within it, decided in FP32 unless too
 // close to its surface; there the point takes the walk's own way, the FP64 tests of the nodes
 // above it. (A point inside the ball by more than the rounding of its key lies in nodes that all
 // meet the ball, one outside by as much in none that it contains.)
@@ -542,17 +595,26 @@ __global__ void __launch_bounds__(128) k_ball_brute(int pass, uint32_t C, CT ct,
     const float rr = (float)(r * r), skin = 4.f * (float)r * (float)t.box.half_width * 1.862645149230957e-09f;  // 2^-29 of the box
     const float inner = rr * (1.f - 2.f * kRel) - skin, outer = rr * (1.f + 2.f * kRel) + skin;
     uint32_t n = 0, o = pass ? off[s] : 0;
-    for (uint32_t q0 = 0; q0 < nct; q0 += 32) {
-        const uint32_t q = q0 + lane;
-        bool in = false;
-        if (q < nct) {
-            const float v = f_dr2(qh, ql, ft.phi[q], ft.plo[q]);
-            if (f_hi(v) < inner) in = true;
-            else if (!(f_lo(v) > outer)) in = ball_takes(t, q, c.x, c.y, c.z, r);
+    constexpr int kIn = 4;  // points a lane has on their way
+    for (uint32_t q0 = 0; q0 < nct; q0 += 32 * kIn) {
+        float v[kIn];
+#pragma unroll
+        for (int j = 0; j < kIn; ++j) {
+            const uint32_t q = q0 + 32 * j + lane;
+            v[j] = q < nct ? f_dr2(qh, ql, ft.phi[q], ft.plo[q]) : 0.f;
         }
-        const unsigned m = __ballot_sync(0xffffffffu, in);
-        if (pass && in) cand[o + n + __popc(m & ((1u << lane) - 1u))] = q;
-        n += __popc(m);
+#pragma unroll
+        for (int j = 0; j < kIn; ++j) {
+            const uint32_t q = q0 + 32 * j + lane;
+            bool in = false;
+            if (q < nct) {
+                if (f_hi(v[j]) < inner) in = true;
+                else if (!(f_lo(v[j]) > outer)) in = ball_takes(t, q, c.x, c.y, c.z, r);
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            if (pass && in) cand[o + n + __popc(m & ((1u << lane) - 1u))] = q;
+            n += __popc(m);
+        }
     }
     if (pass == 0 && lane == 0) cnt[s] = n;
 }
@@ -782,28 +844,49 @@ __global__ void k_merge(uint32_t npred, const uint32_t *pred_list, const uint32_
 }
 
 // Re-key every clump to its densest sub-peak in key order (src/tree.hpp:4156-4182).
-__global__ void k_rekey(uint32_t C, CT ct, const uint32_t *order, uint32_t n, Pool P, const double *dens, uint32_t *slot_of_key,
-                        uint32_t *nfail) {
-    if (threadIdx.x || blockIdx.x) return;
+//
+// One block: the decisions a thread per clump, then the few clumps that change, gathered in order,
+// by one thread (1,564 clumps of 262,144 particles: 0.43 ms with one thread for all, now less than 0.05).
+constexpr int kRekeyThreads = 512;
+
+__global__ void __launch_bounds__(kRekeyThreads) k_rekey(uint32_t C, CT ct, const uint32_t *order, uint32_t n, Pool P, const double *dens,
+                                                         uint32_t *slot_of_key, uint32_t *nfail) {
+    __shared__ uint32_t s_slot[kRekeyThreads], s_warp[kRekeyThreads / 32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
     // decisions first (all against the keys before re-keying), then the re-insertions
-    uint32_t fails = 0;
-    for (uint32_t r = 0; r < n; ++r) {
+    for (uint32_t r = tid; r < n; r += kRekeyThreads) {
         uint32_t s = order[r];
         uint32_t best = ct.key[s];
         for (uint32_t e = ct.sub_head[s]; e != kNone; e = P.sub_next[e])
             if (dens[best] < dens[P.sub_peak[e]]) best = P.sub_peak[e];
         ct.peak[s] = best;  // staged in peak; applied below
     }
-    for (uint32_t r = 0; r < n; ++r) {
-        uint32_t s = order[r];
-        uint32_t nk = ct.peak[s], ok = ct.key[s];
-        if (nk == ok) continue;
-        if (slot_of_key[nk] != kNone) { ++fails; ct.peak[s] = ok; continue; }  // emplace fails: keep the old key
-        slot_of_key[ok] = kNone;
-        slot_of_key[nk] = s;
-        ct.key[s] = nk;
+    __syncthreads();
+    uint32_t fails = 0;
+    for (uint32_t r0 = 0; r0 < n; r0 += kRekeyThreads) {
+        const uint32_t r = r0 + tid, s = r < n ? order[r] : 0;
+        const bool moves = r < n && ct.peak[s] != ct.key[s];
+        const unsigned b = __ballot_sync(0xffffffffu, moves);
+        if (lane == 0) s_warp[tid >> 5] = __popc(b);
+        __syncthreads();
+        uint32_t before = 0, all = 0;
+        for (uint32_t u = 0; u < kRekeyThreads / 32; ++u) {
+            if (u < tid >> 5) before += s_warp[u];
+            all += s_warp[u];
+        }
+        if (moves) s_slot[before + __popc(b & ((1u << lane) - 1u))] = s;
+        __syncthreads();
+        if (tid == 0)
+            for (uint32_t u = 0; u < all; ++u) {
+                const uint32_t x = s_slot[u], nk = ct.peak[x], ok = ct.key[x];
+                if (slot_of_key[nk] != kNone) { ++fails; ct.peak[x] = ok; continue; }  // emplace fails: keep the old key
+                slot_of_key[ok] = kNone;
+                slot_of_key[nk] = x;
+                ct.key[x] = nk;
+            }
+        __syncthreads();
     }
-    *nfail += fails;
+    if (tid == 0) *nfail += fails;
 }
 
 // RN(num / den) given y = RN(1 / den): q0 = RN(num y), then Markstein's correction
@@ -2490,7 +2573,7 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
     if (!live.empty()) {
         int rc2 = st.up_list(live, st.d_list2);
         if (rc2) return rc2;
-        k_rekey<<<1, 1, 0, s>>>(C, ct, st.d_list2, (uint32_t)live.size(), P, tr.dens, st.slot_of_key, st.d_u + 30);
+        k_rekey<<<1, kRekeyThreads, 0, s>>>(C, ct, st.d_list2, (uint32_t)live.size(), P, tr.dens, st.slot_of_key, st.d_u + 30);
         c.launches++;
         rc = st.live_order(live);
         if (rc) return rc;
