@@ -984,7 +984,7 @@ __device__ __forceinline__ bool in_ball(const KTree &t, const FTree &f, const Ba
     const float v = f_dr2(b.qh, b.ql, f.phi[p], f.plo[p]);
     if (f_hi(v) < b.rr32 * (1.f - kRel)) return true;
     if (f_lo(v) > b.rr32 * (1.f + kRel)) return false;
-    return point_dr2(b.cx, b.cy, b.cz, t.pos[p]) <= b.rr;
+    return point_within(t.pos + p, b.cx, b.cy, b.cz, b.rr);
 }
 
 __device__ __forceinline__ int ball_class(const KTree &t, const FTree &f, const uint32_t *epos, uint32_t node, const BallQ &b, uint32_t &eb,
@@ -993,11 +993,14 @@ __device__ __forceinline__ int ball_class(const KTree &t, const FTree &f, const 
     ee = epos[t.nend[node]];
     if (eb == ee) return 3;
     const float4 nh = f.nhi[node], nl = f.nlo[node];
-    int cont = f_contained(nh, nl, b.qh, b.ql, b.rf);
-    if (cont < 0) cont = node_contained(t.ncf[node], b.cx, b.cy, b.cz, b.r) ? 1 : 0;
-    if (cont) return 1;
+    const int cont = f_contained(nh, nl, b.qh, b.ql, b.rf);
+    if (cont > 0) return 1;
     int inter = f_intersects(nh, nl, b.qh, b.ql, b.rf);
-    if (inter < 0) inter = node_intersects(t.ncf[node], b.cx, b.cy, b.cz, b.r) ? 1 : 0;
+    if (cont < 0 || inter < 0) {
+        const int c = node_class(t.ncf + node, b.cx, b.cy, b.cz, b.r);
+        if (c == 1) return 1;
+        inter = c;
+    }
     if (inter) return t.nnd[node] == 0 ? 2 : 4;
     return 3;
 }

@@ -22,7 +22,7 @@
 namespace plan {
 
 constexpr int kWkWarps = 4;           // warps (queries) per block
-constexpr uint32_t kWkNodes = 768;    // nodes to classify: 32 at a time up to kWkWide, then one at a time,
+constexpr uint32_t kWkNodes = 704;    // nodes to classify: 32 at a time up to kWkWide, then one at a time,
 constexpr uint32_t kWkWide = 256;     // when each of the tree's 32 levels adds at most seven (256 + 224 + 224)
 constexpr uint32_t kWkPoints = 512;   // buffered candidates (at least four times the largest k, 128)
 constexpr uint32_t kWkSmall = 8;      // ranges up to this length share the lanes (the default leaf size)
@@ -72,20 +72,13 @@ __device__ __forceinline__ double wk_first_radius(const KTree &t, const WkQuery 
     return knn_first_radius(t, q.x, q.y, q.z, leaf, k, err);
 }
 
-// 1 contained, 2 met, 0 neither, in FP64. A call, not inlined: an inlined body is short enough for
-// the compiler to run it under a predicate instead of a branch, and an FP64 instruction holds the
-// SM's pipe for 16 cycles also where no lane takes part (it was 77% busy that way).
-static __device__ __noinline__ int wk_class_exact(const double4_32a *nc, double x, double y, double z, double r) {
-    if (node_contained(*nc, x, y, z, r)) return 1;
-    return node_intersects(*nc, x, y, z, r) ? 2 : 0;
-}
-
+// 1 contained, 2 met, 0 neither
 __device__ __forceinline__ int wk_class(const KTree &t, const FTree &f, uint32_t node, const WkQuery &q, double r, float rf) {
     const float4 nh = f.nhi[node], nl = f.nlo[node];
     const int c = f_contained(nh, nl, q.h, q.l, rf);
     if (c > 0) return 1;
     const int m = f_intersects(nh, nl, q.h, q.l, rf);
-    if (c < 0 || m < 0) return wk_class_exact(t.ncf + node, q.x, q.y, q.z, r);
+    if (c < 0 || m < 0) return node_class(t.ncf + node, q.x, q.y, q.z, r);
     return m ? 2 : 0;
 }
 

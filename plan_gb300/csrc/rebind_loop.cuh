@@ -126,8 +126,21 @@ __global__ void k_member_terms(uint32_t Tu, const double4_32a *pos, const double
     tm1[q] = make_double4_32a(v.x * p.w, v.y * p.w, v.z * p.w, 0.0);
 }
 
+// (calls, so that no FP64 instruction is run under a predicate where it is not needed)
+static __device__ __noinline__ float2 split_call(double x) {
+    float2 s;
+    split_f(x, s.x, s.y);
+    return s;
+}
+
+static __device__ __noinline__ bool equal_roots(double a, double b) { return sqrt(a) == sqrt(b); }
+
 __device__ __forceinline__ void split_any(double x, float &h, float &l) {
-    if (!split_hilo_bits(x, h, l)) split_f(x, h, l);
+    if (!split_hilo_bits(x, h, l)) {
+        const float2 s = split_call(x);
+        h = s.x;
+        l = s.y;
+    }
 }
 
 // block-wide compaction offset of this thread's flag; returns the block total
@@ -186,12 +199,15 @@ __global__ void k_node_slices(uint32_t nodes, const uint32_t *nbeg, const uint32
 __device__ __forceinline__ int rb_class(const KTree &t, const FTree &f, uint2 e, uint32_t node, const BallQ &b) {
     const float4 nh = f.nhi[node], nl = f.nlo[node];
     if (e.x == e.y) return 3;
-    int c = f_contained(nh, nl, b.qh, b.ql, b.rf);
-    if (c < 0) c = node_contained(t.ncf[node], b.cx, b.cy, b.cz, b.r) ? 1 : 0;
-    if (c) return 1;
-    c = f_intersects(nh, nl, b.qh, b.ql, b.rf);
-    if (c < 0) c = node_intersects(t.ncf[node], b.cx, b.cy, b.cz, b.r) ? 1 : 0;
-    if (c) return t.nnd[node] == 0 ? 2 : 4;
+    const int cont = f_contained(nh, nl, b.qh, b.ql, b.rf);
+    if (cont > 0) return 1;
+    int inter = f_intersects(nh, nl, b.qh, b.ql, b.rf);
+    if (cont < 0 || inter < 0) {
+        const int c = node_class(t.ncf + node, b.cx, b.cy, b.cz, b.r);
+        if (c == 1) return 1;
+        inter = c;
+    }
+    if (inter) return t.nnd[node] == 0 ? 2 : 4;
     return 3;
 }
 
@@ -415,7 +431,7 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
             keep[j] = have[j] && ow[j] != myrank;
             if (keep[j] && !all[j]) {
                 if (f_lo(v[j]) > ball.rr32 * (1.f + kRel)) keep[j] = false;
-                else if (!(f_hi(v[j]) < ball.rr32 * (1.f - kRel))) keep[j] = point_dr2(ball.cx, ball.cy, ball.cz, t.pos[q[j]]) <= ball.rr;
+                else if (!(f_hi(v[j]) < ball.rr32 * (1.f - kRel))) keep[j] = point_within(t.pos + q[j], ball.cx, ball.cy, ball.cz, ball.rr);
             }
         }
         unsigned m[kIn];
@@ -911,10 +927,9 @@ __device__ __forceinline__ void rb_fix_runs(double *dist, uint32_t *idx, uint32_
 
 // any two neighbours of a sorted run of squared distances whose square roots are equal
 __device__ __forceinline__ bool rb_sqrt_tie(double s0, double s1) {
-    if (s0 == s1) return true;
     const unsigned long long b0 = (unsigned long long)__double_as_longlong(s0), b1 = (unsigned long long)__double_as_longlong(s1);
     if (b1 - b0 > 64ull) return false;  // more than a few ulps apart: the roots differ
-    return sqrt(s0) == sqrt(s1);
+    return equal_roots(s0, s1);
 }
 
 // whether this thread's neighbours among m sorted squared distances tie

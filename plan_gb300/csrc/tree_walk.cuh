@@ -61,12 +61,25 @@ __device__ __forceinline__ bool node_intersects(const double4_32a nc, double qx,
     return m2 <= r * r;
 }
 
+// 1 contained, 2 met, 0 neither, in FP64. A call, not inlined: an inlined body is short enough for
+// the compiler to run it under a predicate instead of a branch, and an FP64 instruction holds the
+// SM's pipe for 16 cycles also where no lane takes part (it was 77% busy that way).
+static __device__ __noinline__ int node_class(const double4_32a *nc, double x, double y, double z, double r) {
+    if (node_contained(*nc, x, y, z, r)) return 1;
+    return node_intersects(*nc, x, y, z, r) ? 2 : 0;
+}
+
 __device__ __forceinline__ double point_dr2(double qx, double qy, double qz, const double4_32a p) {
     double dx = qx - p.x, dy = qy - p.y, dz = qz - p.z;
     double s = dx * dx;
     s = s + dy * dy;
     s = s + dz * dz;
     return s;
+}
+
+// whether a point lies within r2 of the query: a call for the same reason
+static __device__ __noinline__ bool point_within(const double4_32a *p, double qx, double qy, double qz, double r2) {
+    return point_dr2(qx, qy, qz, *p) <= r2;
 }
 
 // visit(begin, end, leaf_partial) for each contained node (leaf_partial = false) or each
