@@ -567,7 +567,7 @@ __global__ void k_ball_clumps(int pass, uint32_t C, CT ct, KTree t, bool hill_mo
 // meet the ball, one outside by as much in none that it contains.)
 constexpr uint32_t kBruteClumps = 8192;
 
-__device__ inline bool ball_takes(const KTree &t, uint32_t q, double x, double y, double z, double r) {
+static __device__ __noinline__ bool ball_takes(const KTree &t, uint32_t q, double x, double y, double z, double r) {
     uint32_t n = t.leaf_of[q];
     bool in = point_dr2(x, y, z, t.pos[q]) <= r * r;
     for (int guard = 0; guard < 40; ++guard) {

@@ -20,23 +20,10 @@ namespace {
 
 struct DevTreeView {
     KTree t;
-    __device__ void node(uint32_t n, double &x, double &y, double &z, double &hw) const {
-        const double4_32a f = t.ncf[n];
-        x = f.x;
-        y = f.y;
-        z = f.z;
-        hw = f.w;
-    }
     __device__ uint32_t begin(uint32_t n) const { return t.nbeg[n]; }
     __device__ uint32_t end(uint32_t n) const { return t.nend[n]; }
     __device__ uint32_t first(uint32_t n) const { return t.nfd[n]; }
     __device__ uint32_t daughters(uint32_t n) const { return t.nnd[n]; }
-    __device__ void point(uint32_t q, double &x, double &y, double &z) const {
-        const double4_32a p = t.pos[q];
-        x = p.x;
-        y = p.y;
-        z = p.z;
-    }
 };
 
 // Query tid in the order they are taken: variant by variant, the largest radius first (the
@@ -45,6 +32,13 @@ __device__ __forceinline__ uint64_t dvs_order(const DvsGeom &g, uint64_t tid) {
     const uint64_t cells = (uint64_t)g.nx * g.ny * g.nz;
     const uint32_t v = (uint32_t)(tid / cells);
     return (tid % cells) * g.nvar + (v < (uint32_t)g.nlev ? g.nlev - 1 - v : v);
+}
+
+// A node's class in FP64: a call, so that no FP64 instruction is run under a predicate for nodes
+// that FP32 decides.
+static __device__ __noinline__ int dvs_class_call(const double4_32a *node, double x, double y, double z, int lev, const DvsGeom &g) {
+    const double c[3] = {x, y, z}, nc[3] = {node->x, node->y, node->z};
+    return dvs_class(c, nc, node->w, g.radius[lev], g.maxd[lev], g);
 }
 
 // A node's class in FP32, in FP64 where that cannot tell.
@@ -61,9 +55,7 @@ struct NodeClass {
         const float nf[3] = {h.x, h.y, h.z};
         const int cls = dvs_class_f(cf, nf, h.w, lev, gf);
         if (cls >= 0) return cls;
-        double nc[3], hw;
-        tv.node(n, nc[0], nc[1], nc[2], hw);
-        return dvs_class(c, nc, hw, g.radius[lev], g.maxd[lev], g);
+        return dvs_class_call(tv.t.ncf + n, c[0], c[1], c[2], lev, g);
     }
 };
 
@@ -120,10 +112,7 @@ __global__ void __launch_bounds__(32 * kDvsWarps) k_dvs(DevTreeView tv, FTree ft
                     if (f_hi(v) < rr32 * (1.f - kRel)) {
                         ++in;
                     } else if (!(f_lo(v) > rr32 * (1.f + kRel))) {
-                        double px, py, pz;
-                        tv.point(p, px, py, pz);
-                        const double dx = x - px, dy = y - py, dz = z - pz;
-                        if (dx * dx + dy * dy + dz * dz <= rr) ++in;
+                        if (point_within(tv.t.pos + p, x, y, z, rr)) ++in;
                     }
                 }
                 inside += __reduce_add_sync(full, in);
