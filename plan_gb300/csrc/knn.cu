@@ -5,10 +5,12 @@
 // ancestor of the query's leaf holding >= k/4 points), collects every point of every node
 // the sphere contains or intersects (the intersect test keeps the reference's comparison of
 // a squared distance against r at src/tree.hpp:3030), doubles the radius until >= k points
-// were visited and keeps the k closest visited points in a heap. This kernel reproduces it
-// point for point: a count-only traversal per radius (node tests, no per-point work), then
-// one collecting traversal at the final radius that feeds a heap with the library's
-// sifting order, so ties resolve as in the reference. FP64 throughout, no contraction.
+// were visited and keeps the k closest visited points in a heap. The visited set and, without
+// distance ties, the k kept do not depend on the order of the walk: a warp per query finds them
+// in FP32 with error bounds (knn_warp.cuh). Queries with ties go to a thread per query that
+// reproduces the reference point for point in FP64: a count-only traversal per radius (node
+// tests, no per-point work), then one collecting traversal at the final radius that feeds a heap
+// with the library's sifting order. No contraction.
 #include <cmath>
 #include <cstdlib>
 #include <type_traits>
