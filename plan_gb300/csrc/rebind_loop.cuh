@@ -38,6 +38,10 @@ constexpr int kRbWarps = kRB / 32;
 constexpr uint32_t kRbFront = 4096;           // frontier entries of the ball search
 constexpr uint32_t kRbSmall = 2048;           // members sorted in shared memory
 constexpr uint32_t kRbOnePass = 512;          // members sorted by one digit
+// Updates of a window up to which the lanes share the splitting of its states: with 6 to a window
+// (1,048,576 particles of the benchmark's mixture) a window takes 5,700 cycles instead of 7,200,
+// with 27 (524,288) 1% more than with a lane splitting the seven values it needs.
+constexpr uint32_t kRbFewStates = 12;
 constexpr uint32_t kWaitLimit = 1u << 25;     // bounded waits on blockers: sleeps of 1 us per 2^24 points
 constexpr uint32_t kCallLimit = 1u << 20;     // calls of one clump in one launch
 constexpr int kRbStats = 40;                  // counters per slot
@@ -219,6 +223,7 @@ struct RbShared {
     double *sums;        // the member sums
     double *tk;          // a window's updates: per acceptance m x .. m vz, M', 1 / M'
     double *hist;        // the states of a window: x y z vx vy vz M, before it and after each update
+    float *histf;        // the states of a window as float pairs: hi of the seven, lo of the seven
     float *sf;           // acceptance state for every thread: hi[6], lo[6], Mf
     double *sd;          // acceptance state in FP64: x y z vx vy vz M
 };
@@ -505,21 +510,6 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
             sh.sd[6] = M;
         }
     }
-    // the clump's state as the FP32 tests read it
-    auto publish = [&](double c, double mass) {
-        if (lane < 6) {
-            float h, l;
-            split_f(c, h, l);
-            sh.sf[lane] = h;
-            sh.sf[6 + lane] = l;
-            sh.sd[lane] = c;
-        }
-        if (lane == 0) {
-            sh.sf[12] = (float)mass;
-            sh.sd[6] = mass;
-        }
-        __syncwarp();
-    };
     // warp 0: candidate k against the state in FP32
     auto test = [&](const CandF &cf) { return bound_hilo_fast(cf, sh.sf[12], sh.sf, sh.sf + 6, G32, shear32); };
     // warp 0 takes the window of the tile's candidates from at on; returns where the next one
@@ -601,14 +591,32 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
         else updates(std::false_type());
         __syncwarp();
         const long long tw1 = clock64();
-        // every candidate against the state before it
+        // every candidate against the state before it, in float pairs: those of a few states are
+        // shared out over the lanes, of many each lane splits its own state's
+        const bool few = cnt <= kRbFewStates;
+        if (few) {
+            for (uint32_t i = (uint32_t)lane; i < 7 * (cnt + 1); i += 32) {
+                const uint32_t j = (i * 9363u) >> 16, c = i - 7 * j;  // i / 7
+                float h, l;
+                split_any(sh.hist[8 * j + c], h, l);
+                sh.histf[14 * j + c] = h;
+                sh.histf[14 * j + 7 + c] = l;
+            }
+            __syncwarp();
+        }
         bool bound = false, unsure = false;
         const double *S = sh.hist + 8 * rank;
         if (has && (uint32_t)lane < lim) {
-            float h[6], l[6], mh, ml;
-            for (int c = 0; c < 6; ++c) split_any(S[c], h[c], l[c]);
-            split_any(S[6], mh, ml);
-            const int r = bound_hilo_fast(cf, mh, h, l, G32, shear32);
+            int r;
+            if (few) {
+                const float *f = sh.histf + 14 * rank;
+                r = bound_hilo_fast(cf, f[6], f, f + 7, G32, shear32);
+            } else {
+                float h[6], l[6], mh, ml;
+                for (int c = 0; c < 6; ++c) split_any(S[c], h[c], l[c]);
+                split_any(S[6], mh, ml);
+                r = bound_hilo_fast(cf, mh, h, l, G32, shear32);
+            }
             bound = r == 1;
             unsure = r < 0;
         }
@@ -632,7 +640,19 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
         nacc += n;
         comp = lane < 6 ? sh.hist[8 * n + lane] : 0.0;
         M = sh.hist[8 * n + 6];
-        publish(comp, M);
+        if (lane < 7) {  // the state for the next tests
+            float h, l;
+            if (few) {
+                h = sh.histf[14 * n + lane];
+                l = sh.histf[14 * n + 7 + lane];
+            } else {
+                split_any(sh.hist[8 * n + lane], h, l);
+            }
+            sh.sf[lane < 6 ? lane : 12] = h;
+            if (lane < 6) sh.sf[6 + lane] = l;
+            sh.sd[lane] = sh.hist[8 * n + lane];
+        }
+        __syncwarp();
         if (stat && lane == 0) {
             sh.u[13] += (uint32_t)(clock64() - tw0);
             sh.u[14] += 1;
@@ -1220,9 +1240,9 @@ __global__ void __launch_bounds__(kRB, 1) k_rebind_loop(RbArgs a) {
     __shared__ uint32_t warp_tot[kRbWarps];
     __shared__ uint32_t u[20 + 4 * kRbWarps];
     __shared__ double st[8], sums[8], sd[8], tk[32 * 8], hist[33 * 8];
-    __shared__ float sf[16];
+    __shared__ float sf[16], histf[(kRbFewStates + 1) * 14];
     __shared__ uint32_t s_item;
-    RbShared sh{rb_dyn, warp_tot, u, st, sums, tk, hist, sf, sd};
+    RbShared sh{rb_dyn, warp_tot, u, st, sums, tk, hist, histf, sf, sd};
     const int tid = threadIdx.x;
     for (uint32_t guard = 0; guard <= a.n; ++guard) {
         if (tid == 0) s_item = atomicAdd(a.head, 1u);
