@@ -58,8 +58,8 @@ REBIND_BYTES_PER_MEMBER = 28
 # mixture (the first rebinding launch of a 1M snapshot; the density launch of a 4M one);
 # traffic grows with the units processed, so a full-size launch's traffic is taken as units
 # times these figures
-REBIND_TRAFFIC_PER_MEMBER = (642_154_240 + 417_524_992) / 662_193    # first launch, 1M snapshot: 1,600 B
-DENSITY_TRAFFIC_PER_POINT = (928_974_848 + 483_069_184) / 6_736_104  # 4M snapshot: 209.6 B
+REBIND_TRAFFIC_PER_MEMBER = (403_026_688 + 81_891_840) / 663_881      # first launch, 1M snapshot: 730 B
+DENSITY_TRAFFIC_PER_POINT = (686_419_456 + 52_584_448) / 6_736_104    # 4M snapshot: 109.7 B
 # the catalogue of the benchmarked snapshot as the unmodified reference writes it
 # (tests/golden/w2_16m, made by tests/golden/make_golden.py)
 GOLDEN_FULL = ROOT / "tests" / "golden" / "w2_16m" / "meta.json"
@@ -410,7 +410,7 @@ def run_gpu(args) -> None:
             "limited_by": "dependent FP64 update chains and exact ordered member sums, not bandwidth"}
     dens_avg = float(np.mean(dens_ms))
     achieved = DENSITY_BYTES_PER_POINT * tree_points / (dens_avg / 1e3) / 1e9 if dens_avg > 0 else None
-    roof_dens = {"kernel": "k_density_f (KNN + median density, FP32-filtered exact traversal)", "bound": "hbm", "achieved": achieved,
+    roof_dens = {"kernel": "k_density_w (KNN + median density, FP32-filtered exact traversal, a warp per query)", "bound": "hbm", "achieved": achieved,
                  "peak": peak, "unit": "GB/s", "frac": achieved / peak if achieved else None, "peak_kind": f"{peak_kind} HBM copy bandwidth",
                  "traffic": DENSITY_TRAFFIC_PER_POINT * tree_points, "bytes_per_unit": DENSITY_BYTES_PER_POINT,
                  "units_per_launch": tree_points, "launch_ms": dens_avg}
