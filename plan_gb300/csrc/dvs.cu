@@ -59,6 +59,14 @@ struct NodeClass {
     }
 };
 
+struct DvsWarp {
+    uint32_t at;
+    __device__ uint32_t lane() const { return at; }
+    __device__ uint32_t load(const uint32_t *word) const { return *(volatile const uint32_t *)word; }
+    __device__ uint32_t first(uint32_t v) const { return __shfl_sync(0xffffffffu, v, 0); }
+    __device__ uint32_t sum(uint32_t v) const { return __reduce_add_sync(0xffffffffu, v); }
+};
+
 // Only the largest count of each radius is wanted, so most queries end without a look at a
 // point: the points of contained nodes bound a query's count from below, those of the met
 // leaves on top bound it from above, and a query whose upper bound does not exceed the largest
@@ -97,27 +105,17 @@ __global__ void __launch_bounds__(32 * kDvsWarps) k_dvs(DevTreeView tv, FTree ft
         const NodeClass classify{tv, ft, g, gf, {x, y, z}, {(float)x, (float)y, (float)z}, lev};
         uint32_t inside = 0, partial = 0;  // of the whole warp, the same in every lane
         uint32_t top = 1, nleaf = 0;
-        // the listed leaves' points: true when the count cannot exceed the largest known
-        auto count_leaves = [&](bool stop) {
+        auto count_leaves = [&](const uint32_t *largest) {
             const double r = g.radius[lev], rr = r * r;
             const float rr32 = (float)rr;
             const float4 qh = make_float4(classify.cf[0], classify.cf[1], classify.cf[2], 0.f);
             const float4 ql = make_float4((float)(x - (double)qh.x), (float)(y - (double)qh.y), (float)(z - (double)qh.z), 0.f);
-            for (uint32_t k = 0; k < nleaf; ++k) {
-                if (stop && inside + partial <= *(volatile uint32_t *)&maxc[lev]) return;
-                const uint32_t b = tv.begin(leaves[k]), e = tv.end(leaves[k]);
-                uint32_t in = 0;
-                for (uint32_t p = b + lane; p < e; p += 32) {
-                    const float v = f_dr2(qh, ql, ft.phi[p], ft.plo[p]);
-                    if (f_hi(v) < rr32 * (1.f - kRel)) {
-                        ++in;
-                    } else if (!(f_lo(v) > rr32 * (1.f + kRel))) {
-                        if (point_within(tv.t.pos + p, x, y, z, rr)) ++in;
-                    }
-                }
-                inside += __reduce_add_sync(full, in);
-                partial -= e - b;
-            }
+            dvs_count_leaves(DvsWarp{lane}, tv, leaves, nleaf, largest, inside, partial, [&](uint32_t p) {
+                const float v = f_dr2(qh, ql, ft.phi[p], ft.plo[p]);
+                if (f_hi(v) < rr32 * (1.f - kRel)) return true;
+                if (f_lo(v) > rr32 * (1.f + kRel)) return false;
+                return point_within(tv.t.pos + p, x, y, z, rr);
+            });
         };
         if (lane == 0) list[0] = 0;
         __syncwarp();
@@ -151,7 +149,7 @@ __global__ void __launch_bounds__(32 * kDvsWarps) k_dvs(DevTreeView tv, FTree ft
                 partial += __reduce_add_sync(full, leaf ? size : 0u);
                 if (kCount) {
                     if (nleaf + __popc(lm) > kDvsLeaves) {
-                        count_leaves(false);
+                        count_leaves(nullptr);
                         nleaf = 0;
                         __syncwarp();
                         // the leaves of this step stay in partial: they are listed now
@@ -162,7 +160,7 @@ __global__ void __launch_bounds__(32 * kDvsWarps) k_dvs(DevTreeView tv, FTree ft
             }
             __syncwarp();
         }
-        if (kCount) count_leaves(true);
+        if (kCount) count_leaves(&maxc[lev]);
         // a query that stopped early is not above the largest count: what it counted is a lower bound
         if (lane == 0 && inside > *(volatile uint32_t *)&maxc[lev]) atomicMax(&maxc[lev], inside);
         __syncwarp();

@@ -289,6 +289,24 @@ PLAN_DVS_HD inline void dvs_walk(const Tree &t, Class classify, Contained contai
     }
 }
 
+// The points of the listed leaves, counted by a warp: inside grows by those within the ball, partial
+// falls by all of a leaf's. Where largest is given, the warp stops once the count cannot exceed it.
+// Other warps raise that word meanwhile, so the lanes must not each decide on a value of their
+// own: one that leaves would be missing in the next sum. Warp: lane(), and first(v) and sum(v)
+// over all lanes; load(word) reads what others write. near(p): whether point p lies within the ball.
+template <class Warp, class Tree, class Near>
+PLAN_DVS_HD inline void dvs_count_leaves(const Warp &w, const Tree &t, const uint32_t *leaves, uint32_t nleaf, const uint32_t *largest,
+                                         uint32_t &inside, uint32_t &partial, Near near) {
+    for (uint32_t k = 0; k < nleaf; ++k) {
+        if (largest && inside + partial <= w.first(w.lane() == 0 ? w.load(largest) : 0u)) return;
+        const uint32_t b = t.begin(leaves[k]), e = t.end(leaves[k]);
+        uint32_t in = 0;
+        for (uint32_t p = b + w.lane(); p < e; p += 32) in += near(p) ? 1u : 0u;
+        inside += w.sum(in);
+        partial -= e - b;
+    }
+}
+
 // RecursiveBallSearchCountWithShear (src/tree.hpp:3382-3402): the points of the contained nodes
 // and those of the met leaves within r, compared without the image. Tree provides node(n, cx,
 // cy, cz, hw), begin(n), end(n), first(n), daughters(n) and point(q, x, y, z).
