@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(256) k_kinematics_big(const uint32_t *list, CT
                                                         int with_hill, double G, double Omega) {
     static_assert(kSumChunk == 256, "one member per thread");
     __shared__ __align__(16) double term[7 * kSumStage];
-    __shared__ uint2 steps[7 * kSumChunk];
+    __shared__ __align__(16) uint2 steps[7 * kSumChunk];
     __shared__ double res[7];
     const uint32_t s = list[blockIdx.x];
     const uint32_t o = ct.moff[s], m = ct.mn[s];
@@ -308,7 +308,7 @@ __global__ void k_lib_order(const uint32_t *list, uint32_t n, CT ct, Pool P, con
 // now 0.06.
 __global__ void __launch_bounds__(256) k_one10th(const uint32_t *list, CT ct, Pool P, const double4_32a *pos, const double *dens) {
     __shared__ __align__(16) double term[kSumStage];
-    __shared__ uint2 steps[kSumChunk];
+    __shared__ __align__(16) uint2 steps[kSumChunk];
     __shared__ uint32_t s_in, s_out, s_bad, s_at;
     uint32_t s = list[blockIdx.x];
     const uint32_t o = ct.moff[s], m = ct.mn[s], tid = threadIdx.x, lane = tid & 31;
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(128) k_dispersion(const uint32_t *list, uint32
 // meanwhile), warp 0 adds them in order.
 __global__ void __launch_bounds__(256) k_dispersion_big(const uint32_t *list, CT ct, Pool P, double tol, uint8_t *too_large) {
     __shared__ __align__(16) double term[kSumStage];
-    __shared__ uint2 steps[kSumChunk];
+    __shared__ __align__(16) uint2 steps[kSumChunk];
     const uint32_t s = list[blockIdx.x];
     const uint32_t o = ct.moff[s], m = ct.mn[s];
     if (m <= kBigKinematics) return;
@@ -1863,7 +1863,7 @@ __global__ void __launch_bounds__(128) k_angmom(const uint32_t *list, uint32_t n
 // The same for larger clumps, as k_dispersion_big: three sums in three warps.
 __global__ void __launch_bounds__(256) k_angmom_big(const uint32_t *list, CT ct, Pool P, const double4_32a *pos, const double4_32a *vel, CP cp) {
     __shared__ __align__(16) double term[3 * kSumStage];
-    __shared__ uint2 steps[3 * kSumChunk];
+    __shared__ __align__(16) uint2 steps[3 * kSumChunk];
     __shared__ double res[3];
     const uint32_t s = list[blockIdx.x];
     const uint32_t o = ct.moff[s], m = ct.mn[s];

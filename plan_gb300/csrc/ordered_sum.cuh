@@ -65,7 +65,8 @@ __device__ __forceinline__ long long sum_scan(long long v, uint32_t lane) {  // 
 }
 
 // The sum after the chunk at src (terms at sum_slot(k)) is added to s, or false where that
-// takes the term-by-term loop. list: kSumChunk entries of this warp.
+// takes the term-by-term loop. src: on a 16-byte boundary. list: kSumChunk entries of this warp;
+// their two-entry loads start on a 16-byte boundary wherever the list itself does.
 __device__ __forceinline__ bool sum_chunk_int(const double *src, double &s, uint2 *list) {
     const uint32_t lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu;
@@ -213,6 +214,10 @@ __device__ __forceinline__ bool sum_chunk_int(const double *src, double &s, uint
             c = w - (x - ((m >> 1) + 1));
         };
         uint32_t i = 0;
+        if (reinterpret_cast<uintptr_t>(list) & 8) {
+            step(list[0].x, list[0].y);
+            i = 1;
+        }
         for (; i + 4 <= count; i += 4) {
             const uint4 e0 = *reinterpret_cast<const uint4 *>(list + i), e1 = *reinterpret_cast<const uint4 *>(list + i + 2);
             step(e0.x, e0.y);
