@@ -6,6 +6,8 @@
 // from the sorted keys but reproduces the reference's node numbering exactly: a node at
 // tree level L+1 gets index level_offset[L] + (rank of its key prefix among level-(L+1)
 // nodes), which is the depth-first creation order of FillTree within a level.
+#include <cuda.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -693,6 +695,28 @@ TreeBox make_box(const double center[3], double half_width) {
     return box;
 }
 
+// Whether all of [p, p + bytes) belongs to the allocation or registration that p lies in. The
+// type of a pointer's memory says nothing about its neighbours: a program may have page-locked
+// a part of a block, and a kernel that reads on beyond it faults where a copy would not.
+static bool within_allocation(const void *p, size_t bytes) {
+    static const auto get = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q{};
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<CUresult (*)(void *, CUpointer_attribute, CUdeviceptr)>(f);
+    }();
+    CUdeviceptr at = reinterpret_cast<uintptr_t>(p), start = 0;
+    size_t size = 0;
+    if (!get || get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) != CUDA_SUCCESS ||
+        get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) != CUDA_SUCCESS)
+        return false;
+    return at >= start && bytes <= size && at - start <= size - bytes;
+}
+
 // ------------------------------------------------------------------ host side of stage 1
 int build_tree(Context &c, const plan_lis_view &v, plan_params &p, int first_file, cudaStream_t s) {
     cudaEvent_t ev[6];
@@ -728,9 +752,10 @@ int build_tree(Context &c, const plan_lis_view &v, plan_params &p, int first_fil
     }
     if (S.failed) return kErrOutOfMemory;
 
-    // 1. unpack: blocks in this device's memory or in page-locked host memory are read in place,
-    // others are copied first
+    // 1. unpack: blocks that lie wholly in this device's memory or in page-locked host memory are
+    // read in place, others are copied first
     {
+        cudaGetLastError();  // what an earlier call left behind is not this one's
         size_t at = 0;
         uint64_t uploaded = 0;
         for (uint32_t b = 0; b < v.nblocks; ++b) {
@@ -738,8 +763,9 @@ int build_tree(Context &c, const plan_lis_view &v, plan_params &p, int first_fil
             if (!m) continue;
             const unsigned char *src = d_rec + at * 44;
             cudaPointerAttributes pa{};
-            const bool known = cudaPointerGetAttributes(&pa, v.records[b]) == cudaSuccess;
+            bool known = cudaPointerGetAttributes(&pa, v.records[b]) == cudaSuccess;
             if (!known) cudaGetLastError();
+            known = known && pa.type != cudaMemoryTypeUnregistered && within_allocation(v.records[b], m * 44);
             if (known && pa.type == cudaMemoryTypeDevice && pa.device == c.device) {
                 src = static_cast<const unsigned char *>(v.records[b]);
             } else {
