@@ -37,6 +37,7 @@
 #include "ordered_sum.cuh"
 #include "tree_walk.cuh"
 #include "knn_f32.cuh"
+#include "unbind_f32.cuh"
 
 namespace plan {
 
@@ -1046,11 +1047,6 @@ __device__ __forceinline__ bool bound_fp64(const double4_32a p, const double4_32
     const double e = +0.5 / M * norm2_3(ex, ey, ez) - cp.G / norm3(dx, y - p.y, z - p.z);
     return e < 0;
 }
-
-// A candidate as float hi/lo pairs (x = hi + lo to 2^-48): position, velocity, and its mass.
-struct CandF {
-    float ph[3], pl[3], vh[3], vl[3], w;
-};
 
 // The boundness test entirely in FP32 from hi/lo pairs of the state (sh, sl: x, y, z, vx,
 // vy, vz) and of the candidate: 1 bound, 0 not, -1 too close to call (then bound_fp64).

@@ -28,33 +28,6 @@ struct UbShared {
     uint32_t at;
 };
 
-// Whether the others bind the member: 1 unbound, 0 bound, -1 too close to call. With
-// Mr = M - m, the centre of the others differs from the member's position by (com - p) M / Mr.
-// The differences of float pairs carry a relative error below 2^-22 unless they cancel to less
-// than 2^-25 of the coordinates (refused); M / Mr and its products stay below 2^-20 while
-// Mr > M / 64; the rest as bound_hilo_fast. The FP64 form of the reference errs by 2^-50 of the
-// coordinates, far less than the margin on the same terms.
-__device__ __forceinline__ int ub_test(const CandF &c, const float *sf, float G, float shear) {
-    const float M = sf[12], Mr = M - c.w;
-    if (!(Mr > M * 0.015625f && M > 1e-30f && M < 1e30f)) return -1;
-    const float rho = __fdividef(M, Mr);
-    const float dx = ((sf[0] - c.ph[0]) + (sf[6] - c.pl[0])) * rho, dy = ((sf[1] - c.ph[1]) + (sf[7] - c.pl[1])) * rho;
-    const float dz = ((sf[2] - c.ph[2]) + (sf[8] - c.pl[2])) * rho;
-    const float ex = ((sf[3] - c.vh[0]) + (sf[9] - c.vl[0])) * rho, t1 = ((sf[4] - c.vh[1]) + (sf[10] - c.vl[1])) * rho, t2 = shear * dx;
-    const float ey = t1 - t2, ez = ((sf[5] - c.vh[2]) + (sf[11] - c.vl[2])) * rho;
-    const float K = ex * ex + ey * ey + ez * ez, D2 = dx * dx + dy * dy + dz * dz;
-    const float tiny = rho * rho * 8.8817842e-16f;  // 2^-50
-    if (!(K > 1e-30f && D2 > 1e-30f && K < 1e30f && D2 < 1e30f && D2 > sf[13] * tiny && K > sf[14] * tiny)) return -1;
-    const float rM = __fdividef(1.0f, M);
-    const float A = 0.5f * rM * K, B = G * rsqrtf(D2);
-    const float e = A - B;
-    const float margin = (fabsf(A) + fabsf(B)) * 7.62939453125e-06f                           // 2^-17
-                         + fabsf(ey) * (fabsf(t1) + fabsf(t2)) * 1.9073486328125e-06f * rM;   // 2^-19 / M
-    if (e > margin) return 1;
-    if (e < -margin) return 0;
-    return -1;
-}
-
 // The same as the reference writes it; S: x y z vx vy vz M.
 __device__ __forceinline__ bool ub_exact(const double4_32a p, const double4_32a v, const double *S, const CP &cp) {
     const double M = S[6], Mr = M - p.w;  // > 0: at least two members remain
