@@ -16,8 +16,6 @@
 // nearest; a tie at the k-boundary also sends the query to the exact heap path.
 #pragma once
 
-#include "tree_walk.cuh"
-
 namespace plan {
 
 struct FTree {
@@ -61,17 +59,19 @@ __device__ __forceinline__ int f_intersects(const float4 nh, const float4 nl, co
     int a = f_less(c2c, r, 1e-24f), b = f_less(c2c, nh.w, 1e-24f);
     if (a == 1 || b == 1) return 1;
     if (a == -1 || b == -1) return -1;
-    // exact box distance: q below, inside or above each face (differences q - c vs +-hw)
-    float m2 = 0.f;
+    // exact box distance: q below, inside or above each face (differences q - c vs +-hw). What is
+    // left beyond a face carries the roundings of the difference and of hw, 2^-22 (e + hw) at most,
+    // whatever the sphere's size: in its square 2^-21 hw e on top of the relative bound.
+    float m2 = 0.f, beyond = 0.f;
     float d3[3] = {-dx, -dy, -dz};  // q - c
     for (int k = 0; k < 3; ++k) {
         float u = d3[k];
         int below = f_less(u, -nh.w, 1e-14f), above = f_less(nh.w, u, 1e-14f);
         if (below == -1 || above == -1) return -1;
-        if (below == 1) { float e = u + nh.w; m2 += e * e; }
-        else if (above == 1) { float e = u - nh.w; m2 += e * e; }
+        if (below == 1) { float e = u + nh.w; m2 += e * e; beyond -= e; }
+        else if (above == 1) { float e = u - nh.w; m2 += e * e; beyond += e; }
     }
-    int in = f_less(r * r, m2, 1e-24f);  // m2 > r^2 means no intersection
+    int in = f_less(r * r, m2, 1e-24f + nh.w * beyond * 9.5367431640625e-07f);  // m2 > r^2 means no intersection
     if (in == -1) return -1;
     return in == 1 ? 0 : 1;
 }

@@ -18,6 +18,7 @@
 
 #include "exact64.cuh"
 #include "knn_f32.cuh"
+#include "tree_walk.cuh"
 
 namespace plan {
 
