@@ -36,7 +36,6 @@
 #include "sort.h"
 #include "ordered_sum.cuh"
 #include "tree_walk.cuh"
-#include "knn_f32.cuh"
 #include "unbind_f32.cuh"
 
 namespace plan {
@@ -609,8 +608,8 @@ __global__ void __launch_bounds__(128) k_ball_brute(int pass, uint32_t C, CT ct,
             const uint32_t q = q0 + 32 * j + lane;
             bool in = false;
             if (q < nct) {
-                if (f_hi(v[j]) < inner) in = true;
-                else if (!(f_lo(v[j]) > outer)) in = ball_takes(t, q, c.x, c.y, c.z, r);
+                if (f_hi(v[j], ft.tol) < inner) in = true;
+                else if (!(f_lo(v[j], ft.tol) > outer)) in = ball_takes(t, q, c.x, c.y, c.z, r);
             }
             const unsigned m = __ballot_sync(0xffffffffu, in);
             if (pass && in) cand[o + n + __popc(m & ((1u << lane) - 1u))] = q;
@@ -983,8 +982,8 @@ __device__ __forceinline__ BallQ make_ball(double cx, double cy, double cz, doub
 // RecursiveBallSearch keeps a leaf point when its squared distance is <= r^2
 __device__ __forceinline__ bool in_ball(const KTree &t, const FTree &f, const BallQ &b, uint32_t p) {
     const float v = f_dr2(b.qh, b.ql, f.phi[p], f.plo[p]);
-    if (f_hi(v) < b.rr32 * (1.f - kRel)) return true;
-    if (f_lo(v) > b.rr32 * (1.f + kRel)) return false;
+    if (f_hi(v, f.tol) < b.rr32 * (1.f - kRel)) return true;
+    if (f_lo(v, f.tol) > b.rr32 * (1.f + kRel)) return false;
     return point_within(t.pos + p, b.cx, b.cy, b.cz, b.rr);
 }
 
@@ -994,9 +993,9 @@ __device__ __forceinline__ int ball_class(const KTree &t, const FTree &f, const 
     ee = epos[t.nend[node]];
     if (eb == ee) return 3;
     const float4 nh = f.nhi[node], nl = f.nlo[node];
-    const int cont = f_contained(nh, nl, b.qh, b.ql, b.rf);
+    const int cont = f_contained(nh, nl, b.qh, b.ql, b.rf, f.tol);
     if (cont > 0) return 1;
-    int inter = f_intersects(nh, nl, b.qh, b.ql, b.rf);
+    int inter = f_intersects(nh, nl, b.qh, b.ql, b.rf, f.tol);
     if (cont < 0 || inter < 0) {
         const int c = node_class(t.ncf + node, b.cx, b.cy, b.cz, b.r);
         if (c == 1) return 1;
@@ -2135,7 +2134,7 @@ struct Stage {
         if (list.empty()) return kOk;
         int rc = up_list(list, d_list);
         if (rc) return rc;
-        const FTree ft{tr.phi, tr.plo, tr.nhi, tr.nlo};
+        const FTree ft = ftree_of(tr);
         PLAN_CUDA(cudaFuncSetAttribute(k_unbind, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(UbShared)));
         k_unbind<<<(unsigned)list.size(), kUb, sizeof(UbShared), s>>>(d_list, ct, P, tr.pos, tr.vel, ft, cp);
         c.launches++;
@@ -2385,7 +2384,7 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
             uint32_t ncand = 0;
             if (nct) {
                 if (nct <= kBruteClumps)
-                    k_ball_brute<<<(C + 3) / 4, 128, 0, s>>>(0, C, ct, kct, FTree{ctree.phi, ctree.plo, ctree.nhi, ctree.nlo}, ctree.Tu, hill_mode, hillf,
+                    k_ball_brute<<<(C + 3) / 4, 128, 0, s>>>(0, C, ct, kct, ftree_of(ctree), ctree.Tu, hill_mode, hillf,
                                                              max_radius, d_cnt, nullptr, nullptr);
                 else
                     k_ball_clumps<<<grid_for(C, 128), 128, 0, s>>>(0, C, ct, kct, hill_mode, hillf, max_radius, d_cnt, nullptr, nullptr, c.d_err);
@@ -2410,7 +2409,7 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
             uint32_t nsaddle = 0;
             if (ncand) {
                 if (nct <= kBruteClumps)
-                    k_ball_brute<<<(C + 3) / 4, 128, 0, s>>>(1, C, ct, kct, FTree{ctree.phi, ctree.plo, ctree.nhi, ctree.nlo}, ctree.Tu, hill_mode, hillf,
+                    k_ball_brute<<<(C + 3) / 4, 128, 0, s>>>(1, C, ct, kct, ftree_of(ctree), ctree.Tu, hill_mode, hillf,
                                                              max_radius, d_cnt, d_off, d_cand);
                 else
                     k_ball_clumps<<<grid_for(C, 128), 128, 0, s>>>(1, C, ct, kct, hill_mode, hillf, max_radius, d_cnt, d_off, d_cand, c.d_err);
@@ -2663,7 +2662,7 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
         PLAN_CUDA(cudaMemsetAsync(reach, 0, nb * 8, s));
         PLAN_CUDA(cudaMemsetAsync(tent, 0xff, (size_t)Tu * 4, s));
         KTree kt = ktree_of(tr);
-        const FTree ftr{tr.phi, tr.plo, tr.nhi, tr.nlo};
+        const FTree ftr = ftree_of(tr);
         // speculative acceptance windows (exact by verification; PLAN_ACCEPT_SPECULATE=1)
         const char *spec_env = std::getenv("PLAN_ACCEPT_SPECULATE");
         const bool speculate = spec_env && *spec_env == '1';

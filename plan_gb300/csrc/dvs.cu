@@ -12,7 +12,6 @@
 #include "dvs.cuh"
 #include "pipeline.h"
 #include "tree_walk.cuh"
-#include "knn_f32.cuh"
 
 namespace plan {
 
@@ -112,8 +111,8 @@ __global__ void __launch_bounds__(32 * kDvsWarps) k_dvs(DevTreeView tv, FTree ft
             const float4 ql = make_float4((float)(x - (double)qh.x), (float)(y - (double)qh.y), (float)(z - (double)qh.z), 0.f);
             dvs_count_leaves(DvsWarp{lane}, tv, leaves, nleaf, largest, inside, partial, [&](uint32_t p) {
                 const float v = f_dr2(qh, ql, ft.phi[p], ft.plo[p]);
-                if (f_hi(v) < rr32 * (1.f - kRel)) return true;
-                if (f_lo(v) > rr32 * (1.f + kRel)) return false;
+                if (f_hi(v, ft.tol) < rr32 * (1.f - kRel)) return true;
+                if (f_lo(v, ft.tol) > rr32 * (1.f + kRel)) return false;
                 return point_within(tv.t.pos + p, x, y, z, rr);
             });
         };
@@ -240,7 +239,7 @@ int density_vs_scale(Context &c, const plan_params &p, double time, std::vector<
         for (const std::vector<double> *v : {&xs, &ys, &zs})
             if (!v->empty()) coord = std::fmax(coord, std::fmax(std::fabs(v->front()), std::fabs(v->back())) + g.sub1[0] + g.sub1[1] + g.sub1[2]);
         const DvsGeomF gf = dvs_geom_f(g, coord);
-        const FTree ft{tr.phi, tr.plo, tr.nhi, tr.nlo};
+        const FTree ft = ftree_of(tr);
         const DevTreeView tv{ktree_of(tr)};
         const uint64_t ncentre = (uint64_t)g.nx * g.ny * g.nz * g.nlev;
         int sms = 152;

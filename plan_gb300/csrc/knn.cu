@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(32 * kWkWarps) k_density_w(KTree t, FTree f, u
     const double4_32a p = t.pos[i];
     WkQuery q{p.x, p.y, p.z, f.phi[i], f.plo[i]};
     uint32_t m, visited, tau;
-    bool ok = wk_collect(t, f, q, wk_first_radius(t, q, t.leaf_of[i], k, err), k, s, m, visited, tau, err) && visited >= k && wk_kset(s, k, m, tau);
+    bool ok = wk_collect(t, f, q, wk_first_radius(t, q, t.leaf_of[i], k, err), k, s, m, visited, tau, err) && visited >= k && wk_kset(s, k, m, tau, f.tol);
     uint32_t last = 0, c = 0;
     if (ok) {
         __syncwarp();
@@ -147,13 +147,13 @@ __global__ void __launch_bounds__(32 * kWkWarps) k_density_w(KTree t, FTree f, u
         for (uint32_t j = lane; j < k; j += 32)
             if (s.key[j] <= T) med = max(med, s.key[j]);
         med = __reduce_max_sync(full, med);
-        const float lo4 = 4.f * f_lo(__uint_as_float(med)), hi4 = 4.f * f_hi(__uint_as_float(med));
+        const float lo4 = 4.f * f_lo(__uint_as_float(med), f.tol), hi4 = 4.f * f_hi(__uint_as_float(med), f.tol);
         uint32_t far = 0, second = 0;
         bool clear = true;
         for (uint32_t j = lane; j < k; j += 32) {
             const float v = __uint_as_float(s.key[j]);
-            const bool in = f_hi(v) <= lo4;
-            clear = clear && (in || f_lo(v) > hi4);
+            const bool in = f_hi(v, f.tol) <= lo4;
+            clear = clear && (in || f_lo(v, f.tol) > hi4);
             if (in) {
                 ++c;
                 second = max(second, min(far, s.key[j]));
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(32 * kWkWarps) k_density_w(KTree t, FTree f, u
         const unsigned holders = __ballot_sync(full, far == top);
         // the last point: no other as far, within the error bound
         second = __reduce_max_sync(full, (far == top && lane == (uint32_t)(__ffs(holders) - 1)) ? second : far);
-        ok = __all_sync(full, clear) && c > 0 && f_hi(__uint_as_float(second)) < f_lo(__uint_as_float(top));
+        ok = __all_sync(full, clear) && c > 0 && f_hi(__uint_as_float(second), f.tol) < f_lo(__uint_as_float(top), f.tol);
         if (c == 1) ok = __all_sync(full, clear);
         for (uint32_t j = lane; j < k; j += 32)
             if (s.key[j] == top) last = s.ix[j];
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(32 * kWkWarps) k_density_w(KTree t, FTree f, u
                     for (uint32_t o = 0; o < k; ++o) {
                         const uint32_t u = s.key[o];
                         rank += u < v ? 1u : 0u;
-                        order = order && (o == j || u > top || f_hi(__uint_as_float(min(u, v))) < f_lo(__uint_as_float(max(u, v))));
+                        order = order && (o == j || u > top || f_hi(__uint_as_float(min(u, v)), f.tol) < f_lo(__uint_as_float(max(u, v)), f.tol));
                     }
                     ms[rank] = t.pos[s.ix[j]].w;
                 }
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(32 * kWkWarps) k_densest_w(KTree t, FTree f, u
     const double4_32a p = t.pos[i];
     WkQuery q{p.x, p.y, p.z, f.phi[i], f.plo[i]};
     uint32_t m, visited, tau;
-    if (wk_collect(t, f, q, wk_first_radius(t, q, t.leaf_of[i], k, err), k, s, m, visited, tau, err) && visited >= k && wk_kset(s, k, m, tau)) {
+    if (wk_collect(t, f, q, wk_first_radius(t, q, t.leaf_of[i], k, err), k, s, m, visited, tau, err) && visited >= k && wk_kset(s, k, m, tau, f.tol)) {
         __syncwarp();
         wk_densest(s.ix, k, i, di, dens, densest);
     } else if (lane == 0) {
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(32 * kWkWarps) k_exact_w(KTree t, FTree f, con
             if (lane == 0) out.dens[i] = 0.0;
             continue;
         }
-        ok = ok && visited >= k && wk_sorted(t, q, s, k, m, tau);
+        ok = ok && visited >= k && wk_sorted(t, q, s, k, m, tau, f.tol);
         if (!ok) {
             if (lane == 0) out.redo[atomicAdd(out.nredo, 1u)] = i;
             continue;
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(kBkThreads) k_exact_block(KTree t, FTree f, co
             unsigned m = __ballot_sync(full, v[j] <= tau);
             if (!m) continue;
             if (n + __popc(m) > kBkPart) {
-                wk_compact(key, ix, k, n, tau);
+                wk_compact(key, ix, k, n, tau, f.tol);
                 if (lane == 0) atomicMin(&sh.tau, tau);
                 m = __ballot_sync(full, v[j] <= tau);
                 if (n + __popc(m) > kBkPart) {
@@ -510,7 +510,7 @@ __global__ void __launch_bounds__(kBkThreads) k_exact_block(KTree t, FTree f, co
             __syncwarp();
         }
     }
-    wk_compact(key, ix, k, n, tau);
+    wk_compact(key, ix, k, n, tau, f.tol);
     if (lane == 0) atomicMin(&sh.tau, tau);
     __syncthreads();
     tau = sh.tau;
@@ -529,7 +529,7 @@ __global__ void __launch_bounds__(kBkThreads) k_exact_block(KTree t, FTree f, co
     __syncthreads();
     if (w != 0) return;
     const uint32_t all = sh.nmerged;
-    if (!sh.over && wk_sorted(t, q, sh.merged, k, all, tau)) wk_finish<OP>(t, sh.merged, p, true, i, k, fpo3, sc, out);
+    if (!sh.over && wk_sorted(t, q, sh.merged, k, all, tau, f.tol)) wk_finish<OP>(t, sh.merged, p, true, i, k, fpo3, sc, out);
     else if (lane == 0) out.redo[atomicAdd(out.nredo, 1u)] = i;
 }
 
@@ -567,7 +567,7 @@ int launch_density(Context &c, const plan_params &p, uint32_t k, cudaStream_t s)
     if (k > 64) return kErrUnsupported;
     KTree t = ktree_of(c.tree);
     const double fpo3 = 3.14159265358979323846 * 4. / 3.;
-    FTree f{c.tree.phi, c.tree.plo, c.tree.nhi, c.tree.nlo};
+    const FTree f = ftree_of(c.tree);
     const uint32_t n = c.tree.Tu;
     const size_t mark = c.scratch.used;
     RedoLists redo;
@@ -615,7 +615,7 @@ int launch_density(Context &c, const plan_params &p, uint32_t k, cudaStream_t s)
 int launch_densest(Context &c, const plan_params &p, uint32_t k, double threshold, uint32_t *densest, cudaStream_t s) {
     if (k > 64) return kErrUnsupported;
     KTree t = ktree_of(c.tree);
-    FTree f{c.tree.phi, c.tree.plo, c.tree.nhi, c.tree.nlo};
+    const FTree f = ftree_of(c.tree);
     const uint32_t n = c.tree.Tu;
     const size_t mark = c.scratch.used;
     RedoLists redo;
@@ -653,7 +653,7 @@ int launch_density_at(Context &c, const double *d_q3, const double *d_est, uint3
     KTree t = ktree_of(c.tree);
     const double fpo3 = 3.14159265358979323846 * 4. / 3.;
     const bool spl = !c.fs.median_kernel;
-    FTree f{c.tree.phi, c.tree.plo, c.tree.nhi, c.tree.nlo};
+    const FTree f = ftree_of(c.tree);
     const size_t mark = c.scratch.used;
     uint32_t *heap = c.scratch.get<uint32_t>(nq + 1), *warp = c.scratch.get<uint32_t>(nq + 1), *nheap = c.scratch.get<uint32_t>(4);
     if (!heap || !warp || !nheap) {
@@ -708,7 +708,7 @@ int knn_positions(Context &c, const double *pos3, uint32_t nq, uint32_t k, doubl
     PLAN_CUDA(cudaMemsetAsync(d_redo.p, 0, 4, s));
     PLAN_CUDA(cudaMemcpyAsync(d_q.p, pos3, (size_t)nq * 3 * 8, cudaMemcpyHostToDevice, s));
     KTree t = ktree_of(c.tree);
-    FTree f{c.tree.phi, c.tree.plo, c.tree.nhi, c.tree.nlo};
+    const FTree f = ftree_of(c.tree);
     int rc = launch_by_k(k, [&](auto km, int threads) {
         constexpr int KM = decltype(km)::value;
         k_exact_w<kOpKnn><<<(nq + kWkWarps - 1) / kWkWarps, 32 * kWkWarps, 0, s>>>(t, f, d_q.p, nullptr, est, nullptr, nullptr, nq, k, 0.0,

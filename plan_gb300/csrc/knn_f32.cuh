@@ -8,9 +8,10 @@
 // decided in FP32 when the FP32 value is outside a proven error bound of the threshold.
 // The bound used is relative 2^-17 plus a small absolute term, against a worst-case FP32
 // error near 2^-20 relative, so a decided comparison always agrees with the FP64 one.
-// Coordinates that are not float sums (ghost images shifted by the shear at t != 0) are held
-// to 2^-48 relative, an absolute error below 1e-15 per difference for |x| < 0.25; squared
-// distances then err by at most 2*sqrt(3)*d*1e-15, which 2^-17*d^2 + 1e-24 covers for every d.
+// Coordinates that are not float sums (ghost images shifted by the shear at t != 0, clump centres,
+// a program's own positions) are held to 2^-48 relative, an absolute error below 1e-15 per
+// difference for |x| < 0.25; squared distances then err by at most 2*sqrt(3)*d*1e-15, which
+// 2^-17*d^2 + 1e-24 covers for every d. Larger coordinates scale the absolute terms (Tol).
 // When a comparison falls inside its bound the query is redone on the exact FP64 path, and
 // exact FP64 distances are computed for every candidate that could belong to the k
 // nearest; a tie at the k-boundary also sends the query to the exact heap path.
@@ -18,9 +19,23 @@
 
 namespace plan {
 
+// The absolute error terms of a squared distance and of a difference.
+struct Tol {
+    float sq, len;
+};
+
+// reach: the largest magnitude of a coordinate in the root box. Positions up to twice as far out
+// are held as well as 2 reach; for one beyond, the distance to any point of the box is at least
+// half its own magnitude, and the relative bound alone covers it.
+inline Tol tol_of(double reach) {
+    const double k = 8.0 * reach > 1.0 ? 8.0 * reach : 1.0;
+    return Tol{(float)(1e-24 * k * k), (float)(1e-14 * k)};
+}
+
 struct FTree {
     const float4 *phi, *plo;  // points: x, y, z (hi / lo)
     const float4 *nhi, *nlo;  // nodes: cx, cy, cz, hw (hi / lo)
+    Tol tol;
 };
 
 constexpr float kRel = 7.62939453125e-06f;  // 2^-17
@@ -39,24 +54,24 @@ __device__ __forceinline__ int f_less(float a, float b, float abs_a = kAbs) {
 __device__ __forceinline__ float f_diff(float ah, float al, float bh, float bl) { return (ah - bh) + (al - bl); }
 
 // SphereContainNode in FP32: 1 contained, 0 not, -1 unsure
-__device__ __forceinline__ int f_contained(const float4 nh, const float4 nl, const float4 qh, const float4 ql, float r) {
+__device__ __forceinline__ int f_contained(const float4 nh, const float4 nl, const float4 qh, const float4 ql, float r, Tol tol) {
     float t = nh.w * kSqrt3f;
     float a = fabsf(f_diff(nh.x, nl.x, qh.x, ql.x)) + t;
     float b = fabsf(f_diff(nh.y, nl.y, qh.y, ql.y)) + t;
     float c = fabsf(f_diff(nh.z, nl.z, qh.z, ql.z)) + t;
     float s = a * a + b * b + c * c;
-    return f_less(s, r * r, 1e-24f);
+    return f_less(s, r * r, tol.sq);
 }
 
 // SphereNodeIntersect in FP32: 1 intersects, 0 not, -1 unsure
-__device__ __forceinline__ int f_intersects(const float4 nh, const float4 nl, const float4 qh, const float4 ql, float r) {
+__device__ __forceinline__ int f_intersects(const float4 nh, const float4 nl, const float4 qh, const float4 ql, float r, Tol tol) {
     float dx = f_diff(nh.x, nl.x, qh.x, ql.x), dy = f_diff(nh.y, nl.y, qh.y, ql.y), dz = f_diff(nh.z, nl.z, qh.z, ql.z);
     float c2c = dx * dx + dy * dy + dz * dz;
     float t = nh.w * kSqrt3f + r;
-    int outside = f_less(t * t, c2c, 1e-24f);  // c2c > t^2
+    int outside = f_less(t * t, c2c, tol.sq);  // c2c > t^2
     if (outside == 1) return 0;
     if (outside == -1) return -1;
-    int a = f_less(c2c, r, 1e-24f), b = f_less(c2c, nh.w, 1e-24f);
+    int a = f_less(c2c, r, tol.sq), b = f_less(c2c, nh.w, tol.sq);
     if (a == 1 || b == 1) return 1;
     if (a == -1 || b == -1) return -1;
     // exact box distance: q below, inside or above each face (differences q - c vs +-hw). What is
@@ -66,12 +81,12 @@ __device__ __forceinline__ int f_intersects(const float4 nh, const float4 nl, co
     float d3[3] = {-dx, -dy, -dz};  // q - c
     for (int k = 0; k < 3; ++k) {
         float u = d3[k];
-        int below = f_less(u, -nh.w, 1e-14f), above = f_less(nh.w, u, 1e-14f);
+        int below = f_less(u, -nh.w, tol.len), above = f_less(nh.w, u, tol.len);
         if (below == -1 || above == -1) return -1;
         if (below == 1) { float e = u + nh.w; m2 += e * e; beyond -= e; }
         else if (above == 1) { float e = u - nh.w; m2 += e * e; beyond += e; }
     }
-    int in = f_less(r * r, m2, 1e-24f + nh.w * beyond * 9.5367431640625e-07f);  // m2 > r^2 means no intersection
+    int in = f_less(r * r, m2, tol.sq + nh.w * beyond * 9.5367431640625e-07f);  // m2 > r^2 means no intersection
     if (in == -1) return -1;
     return in == 1 ? 0 : 1;
 }
@@ -82,7 +97,7 @@ __device__ __forceinline__ float f_dr2(const float4 qh, const float4 ql, const f
 }
 
 // Upper/lower bounds of the FP64 distance given the FP32 one.
-__device__ __forceinline__ float f_hi(float v) { return v * (1.f + kRel) + 1e-24f; }
-__device__ __forceinline__ float f_lo(float v) { return v * (1.f - kRel) - 1e-24f; }
+__device__ __forceinline__ float f_hi(float v, Tol tol) { return v * (1.f + kRel) + tol.sq; }
+__device__ __forceinline__ float f_lo(float v, Tol tol) { return v * (1.f - kRel) - tol.sq; }
 
 }  // namespace plan

@@ -17,7 +17,6 @@
 #pragma once
 
 #include "exact64.cuh"
-#include "knn_f32.cuh"
 #include "tree_walk.cuh"
 
 namespace plan {
@@ -76,9 +75,9 @@ __device__ __forceinline__ double wk_first_radius(const KTree &t, const WkQuery 
 // 1 contained, 2 met, 0 neither
 __device__ __forceinline__ int wk_class(const KTree &t, const FTree &f, uint32_t node, const WkQuery &q, double r, float rf) {
     const float4 nh = f.nhi[node], nl = f.nlo[node];
-    const int c = f_contained(nh, nl, q.h, q.l, rf);
+    const int c = f_contained(nh, nl, q.h, q.l, rf, f.tol);
     if (c > 0) return 1;
-    const int m = f_intersects(nh, nl, q.h, q.l, rf);
+    const int m = f_intersects(nh, nl, q.h, q.l, rf, f.tol);
     if (c < 0 || m < 0) return node_class(t.ncf + node, q.x, q.y, q.z, r);
     return m ? 2 : 0;
 }
@@ -131,12 +130,12 @@ __device__ __forceinline__ uint32_t wk_filter(uint32_t *key, uint32_t *ix, uint3
 
 // Drops the candidates that cannot be among the k nearest: tau becomes a key that no member of
 // the exact k-set exceeds.
-__device__ __forceinline__ void wk_compact(uint32_t *key, uint32_t *ix, uint32_t k, uint32_t &n, uint32_t &tau) {
+__device__ __forceinline__ void wk_compact(uint32_t *key, uint32_t *ix, uint32_t k, uint32_t &n, uint32_t &tau, Tol tol) {
     __syncwarp();
     if (n < k) return;
     uint32_t count;
-    const float thr = f_hi(__uint_as_float(wk_select(key, n, k, count)));
-    tau = min(tau, __float_as_uint((thr + 2e-24f) * (1.f + 4.f * kRel)));
+    const float thr = f_hi(__uint_as_float(wk_select(key, n, k, count)), tol);
+    tau = min(tau, __float_as_uint((thr + 2.f * tol.sq) * (1.f + 4.f * kRel)));
     n = wk_filter(key, ix, n, tau);
 }
 
@@ -158,7 +157,7 @@ __device__ inline bool wk_collect(const KTree &t, const FTree &f, const WkQuery 
             unsigned m = __ballot_sync(full, v <= tau);
             if (!m) return;
             if (n + __popc(m) > kWkPoints) {
-                wk_compact(s.key, s.ix, k, n, tau);
+                wk_compact(s.key, s.ix, k, n, tau, f.tol);
                 m = __ballot_sync(full, v <= tau);
                 if (n + __popc(m) > kWkPoints) {
                     over = true;
@@ -237,7 +236,7 @@ __device__ inline bool wk_collect(const KTree &t, const FTree &f, const WkQuery 
 
 // The exact k-set from the FP32 keys alone: the k smallest of the buffer are moved to its
 // front, unless the (k+1)-th is too close to the k-th to tell (then false).
-__device__ __forceinline__ bool wk_kset(WkBuf &s, uint32_t k, uint32_t n, uint32_t tau) {
+__device__ __forceinline__ bool wk_kset(WkBuf &s, uint32_t k, uint32_t n, uint32_t tau, Tol tol) {
     const uint32_t lane = threadIdx.x & 31;
     __syncwarp();
     if (n < k) return false;
@@ -252,7 +251,7 @@ __device__ __forceinline__ bool wk_kset(WkBuf &s, uint32_t k, uint32_t n, uint32
     }
     in = __reduce_max_sync(0xffffffffu, in);
     out = __reduce_min_sync(0xffffffffu, out);
-    if (!(f_hi(__uint_as_float(in)) < f_lo(__uint_as_float(out)))) return false;
+    if (!(f_hi(__uint_as_float(in), tol) < f_lo(__uint_as_float(out), tol))) return false;
     wk_filter(s.key, s.ix, n, T);
     return true;
 }
@@ -289,9 +288,9 @@ __device__ inline void warp_sort_pairs(unsigned long long *key, uint32_t *ix, ui
 
 // The exact k-set in ascending FP64 distance, in xkey (bits) and xix. False when two of its
 // members, or the k-th and the next, are equally far: their order is the library heap's.
-__device__ __forceinline__ bool wk_sorted(const KTree &t, const WkQuery &q, WkBuf &s, uint32_t k, uint32_t n, uint32_t tau) {
+__device__ __forceinline__ bool wk_sorted(const KTree &t, const WkQuery &q, WkBuf &s, uint32_t k, uint32_t n, uint32_t tau, Tol tol) {
     const uint32_t lane = threadIdx.x & 31;
-    wk_compact(s.key, s.ix, k, n, tau);
+    wk_compact(s.key, s.ix, k, n, tau, tol);
     if (n < k || n > kWkExact) return false;
     __syncwarp();
     for (uint32_t j = lane; j < n; j += 32) {

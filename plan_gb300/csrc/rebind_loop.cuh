@@ -203,9 +203,9 @@ __global__ void k_node_slices(uint32_t nodes, const uint32_t *nbeg, const uint32
 __device__ __forceinline__ int rb_class(const KTree &t, const FTree &f, uint2 e, uint32_t node, const BallQ &b) {
     const float4 nh = f.nhi[node], nl = f.nlo[node];
     if (e.x == e.y) return 3;
-    const int cont = f_contained(nh, nl, b.qh, b.ql, b.rf);
+    const int cont = f_contained(nh, nl, b.qh, b.ql, b.rf, f.tol);
     if (cont > 0) return 1;
-    int inter = f_intersects(nh, nl, b.qh, b.ql, b.rf);
+    int inter = f_intersects(nh, nl, b.qh, b.ql, b.rf, f.tol);
     if (cont < 0 || inter < 0) {
         const int c = node_class(t.ncf + node, b.cx, b.cy, b.cz, b.r);
         if (c == 1) return 1;
@@ -435,8 +435,8 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
         for (int j = 0; j < kIn; ++j) {
             keep[j] = have[j] && ow[j] != myrank;
             if (keep[j] && !all[j]) {
-                if (f_lo(v[j]) > ball.rr32 * (1.f + kRel)) keep[j] = false;
-                else if (!(f_hi(v[j]) < ball.rr32 * (1.f - kRel))) keep[j] = point_within(t.pos + q[j], ball.cx, ball.cy, ball.cz, ball.rr);
+                if (f_lo(v[j], a.ft.tol) > ball.rr32 * (1.f + kRel)) keep[j] = false;
+                else if (!(f_hi(v[j], a.ft.tol) < ball.rr32 * (1.f - kRel))) keep[j] = point_within(t.pos + q[j], ball.cx, ball.cy, ball.cz, ball.rr);
             }
         }
         unsigned m[kIn];

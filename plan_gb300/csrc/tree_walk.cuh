@@ -2,6 +2,7 @@
 // clump-tree kernels (src/tree.hpp:3001-3049, 3086-3102, 3275-3293).
 #pragma once
 
+#include "knn_f32.cuh"
 #include "pipeline.h"
 
 namespace plan {
@@ -32,6 +33,15 @@ inline KTree ktree_of(const DevTree &tr) {
     t.box = tr.box;
     t.nodes = tr.nodes;
     return t;
+}
+
+inline FTree ftree_of(const DevTree &tr) {
+    double reach = 0;
+    for (int d = 0; d < 3; ++d) {
+        const double c = tr.box.root_center[d] < 0 ? -tr.box.root_center[d] : tr.box.root_center[d];
+        if (c + tr.box.half_width > reach) reach = c + tr.box.half_width;
+    }
+    return FTree{tr.phi, tr.plo, tr.nhi, tr.nlo, tol_of(reach)};
 }
 
 __device__ __forceinline__ bool node_contained(const double4_32a nc, double qx, double qy, double qz, double r) {

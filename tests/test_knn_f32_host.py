@@ -4,7 +4,8 @@ f_contained and f_intersects (knn_f32.cuh) may say -1 (too close to call), never
 than the FP64 tests of src/tree.hpp:3001-3049: for nodes from the root to single points and
 spheres from far below a node's size to far above it, at random and placed at the edges of every
 comparison, among them spheres that end just before or behind the faces of a node many times
-their size. f_lo and f_hi must enclose the FP64 squared distance.
+their size, in root boxes of half widths from 0.01 to 10^6. f_lo and f_hi must enclose the FP64
+squared distance of a position as close as 10^-12 of the box to a sheared point.
 """
 from __future__ import annotations
 
@@ -56,9 +57,10 @@ int main() {
     std::mt19937_64 rng(7);
     auto u = [&](double a, double b) { return a + (b - a) * ((double)(rng() >> 11) * 0x1p-53); };
     long bad = 0, n = 0, unsure = 0, said[2][2] = {{0, 0}, {0, 0}};
-    const double boxes[] = {0.125, 0.013, 4.0, 0.7};  // half widths of the root
+    const double boxes[] = {0.125, 0.013, 4.0, 0.7, 300.0, 1e6};  // half widths of the root
     for (double X : boxes) {
-        for (int i = 0; i < 1500000; ++i) {
+        const Tol tol = tol_of(X);
+        for (int i = 0; i < 1000000; ++i) {
             // a node of the tree: the root's corners halved
             const int depth = (int)(rng() % 20);
             const double hw = std::ldexp(X, -depth);
@@ -81,7 +83,7 @@ int main() {
             if (edge == 4)  // the sphere through the containment test's corner
                 for (int d = 0; d < 3; ++d) q[d] = c[d] + side * (r / 1.7320508075688772 - hw * 1.7320508075688772) * (1.0 + jit);
             const float4 nh = hi4(c, hw), nl = lo4(c, hw), qh = hi4(q, 0), ql = lo4(q, 0);
-            const int cf = f_contained(nh, nl, qh, ql, (float)r), mf = f_intersects(nh, nl, qh, ql, (float)r);
+            const int cf = f_contained(nh, nl, qh, ql, (float)r, tol), mf = f_intersects(nh, nl, qh, ql, (float)r, tol);
             const int cd = contained(c, hw, q, r), md = intersects(c, hw, q, r);
             ++n;
             if (cf < 0 || mf < 0) ++unsure;
@@ -90,15 +92,18 @@ int main() {
             if ((cf >= 0 && cf != cd) || (mf >= 0 && mf != md)) {
                 if (bad++ < 8) printf("box %g hw %g r %g edge %d: contained %d (%d), met %d (%d)\n", X, hw, r, edge, cf, cd, mf, md);
             }
-            // a point near the query: a record's float position, moved by a shear as ghosts are
-            double p[3], s = 0;
-            const double near = X * std::pow(10.0, -(double)(rng() % 12));
-            for (int d = 0; d < 3; ++d) p[d] = (double)(float)(q[d] + u(-1.0, 1.0) * near);
-            if (rng() & 1) p[1] = p[1] + u(-0.1, 0.1) * near;
-            for (int d = 0; d < 3; ++d) s = s + (q[d] - p[d]) * (q[d] - p[d]);
-            const float v = f_dr2(qh, ql, hi4(p, 0), lo4(p, 0));
-            if (!((double)f_lo(v) <= s && s <= (double)f_hi(v))) {
-                if (bad++ < 8) printf("box %g: distance %g not in [%g, %g]\n", X, s, (double)f_lo(v), (double)f_hi(v));
+            // a point near a query: a record's float position, moved by a shear as ghosts are
+            double p[3], near[3], s = 0;
+            const double by = X * std::pow(10.0, -(double)(rng() % 13));
+            for (int d = 0; d < 3; ++d) p[d] = (double)(float)(u(-1.0, 1.0) * X);
+            if (rng() & 1) p[1] = p[1] + u(-0.5, 0.5) * X;
+            for (int d = 0; d < 3; ++d) {
+                near[d] = p[d] + u(-1.0, 1.0) * by;
+                s = s + (near[d] - p[d]) * (near[d] - p[d]);
+            }
+            const float v = f_dr2(hi4(near, 0), lo4(near, 0), hi4(p, 0), lo4(p, 0));
+            if (!((double)f_lo(v, tol) <= s && s <= (double)f_hi(v, tol))) {
+                if (bad++ < 8) printf("box %g: distance %g not in [%g, %g]\n", X, s, (double)f_lo(v, tol), (double)f_hi(v, tol));
             }
         }
     }
