@@ -52,6 +52,8 @@ int Context::ensure(Arena &a, size_t bytes) {
     return kOk;
 }
 
+uint64_t scratch_bytes_for(uint64_t T) { return T * kScratchBytesPerTreePoint + (1ull << 20); }
+
 // Device bytes for a snapshot of n input particles with the ghost count of a uniform box
 // (T = 1.5625 n); the exact count is known, and the arena grown to it, during the build.
 static void footprint(uint64_t n, uint64_t &arena, uint64_t &scratch) {

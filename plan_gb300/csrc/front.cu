@@ -897,8 +897,10 @@ int build_tree(Context &c, const plan_lis_view &v, plan_params &p, int first_fil
     c.launches++;
     if (selected) PLAN_CUDA(cudaMemcpyAsync(keep_rank, sel_rank, (size_t)N * 4, cudaMemcpyDeviceToDevice, s));
     cudaEventRecord(ev[1], s);
-    // phase A buffers are dead from here on: the scratch arena is reused
+    // phase A buffers are dead from here on: the scratch arena is reused, grown where the ghosts
+    // are more than its first size allows for
     PLAN_CUDA(cudaStreamSynchronize(s));
+    if (c.ensure(c.scratch, (size_t)scratch_bytes_for(Tmax))) return kErrOutOfMemory;
     c.scratch.used = 0;
     size_t sort_bytes = std::max(radix_sort96_scratch_bytes(Tmax), scan_u32_scratch_bytes(Tmax));
     void *scr = c.scratch.take(sort_bytes);

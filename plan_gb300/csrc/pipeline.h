@@ -124,12 +124,19 @@ int launch_densest(Context &c, const plan_params &p, uint32_t k, double threshol
 // and the scratch bytes per input particle; used for sizing and for admission.
 constexpr uint64_t kArenaBytesPerTreePoint = 512;
 constexpr uint64_t kScratchBytesPerParticle = 160;
+// Scratch bytes per tree point of the stages after the ghosts: HOP's member sort takes 53 (three
+// key words and the two record buffers of the radix sort, then two scan words), the octree 48. A
+// box narrower than its ghost zone has four tree points per particle, more than the estimate from
+// the particles covers.
+constexpr uint64_t kScratchBytesPerTreePoint = 56;
 // Room for the clump stage's member pool beyond that: a larger pool means fewer compactions
 // (and fewer relaunches) while the rebinding loop writes fresh segments. Capped so that the
 // largest snapshots still fit the device.
 constexpr uint64_t kPoolBytesPerTreePoint = 800;
 constexpr uint64_t kPoolBytesMax = 24ull << 30;
 
+// The scratch arena for T tree points.
+uint64_t scratch_bytes_for(uint64_t T);
 // The snapshot arena for T tree points.
 inline uint64_t arena_bytes_for(uint64_t T) {
     const uint64_t pool = T * kPoolBytesPerTreePoint < kPoolBytesMax ? T * kPoolBytesPerTreePoint : kPoolBytesMax;
