@@ -2751,6 +2751,7 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
         auto run_loop = [&](const std::vector<uint32_t> &list, const std::vector<std::vector<uint32_t>> *blk) -> int {
             std::vector<uint32_t> todo = list;
             int stuck = 0;
+            uint64_t steps = ~0ull;
             for (int attempt = 0; !todo.empty(); ++attempt) {
                 if (attempt > 4096 || stuck > 3) return kErrOutOfMemory;
                 std::vector<uint8_t> fin(nb, 1);
@@ -2841,7 +2842,16 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
                     if (sus[sl]) next.push_back(sl);
                 if (!next.empty()) {
                     suspensions += next.size();
-                    stuck = next.size() == todo.size() ? stuck + 1 : 0;
+                    // the calls and sorts of the pass's clumps so far: as long as they grow it goes on
+                    std::vector<uint32_t> calls;
+                    std::vector<uint8_t> pending;
+                    r = st.down(calls, d_ccall, nb);
+                    if (!r) r = st.down(pending, d_needsort, nb);
+                    if (r) return r;
+                    uint64_t now = 0;
+                    for (uint32_t sl : list) now += 2 * (uint64_t)calls[sl] - (pending[sl] ? 1 : 0);
+                    stuck = now == steps ? stuck + 1 : 0;
+                    steps = now;
                     r = st.maybe_compact(true);
                     if (r) return r;
                 }

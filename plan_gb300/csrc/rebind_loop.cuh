@@ -78,14 +78,7 @@ __host__ __device__ inline bool ck_after(uint32_t j) {
     return j % 3 == 0 && ((j / 3) & (j / 3 - 1)) == 0;
 }
 
-// A clump's room in the member pool besides its members: the capacity of its present segment
-// (0 where the host packed it), the segment it left last and the sort buffers. Calls go back and
-// forth between two segments that grow by half, so a launch needs a few times the members
-// instead of a segment per call, and the pool does not fill up: a launch that stops for a
-// compaction costs the blocks that wait for one another their order.
-struct RbSeg {
-    uint32_t cap, spare, spare_cap, buf, buf_cap;
-};
+#include "rebind_pool.cuh"
 
 struct RbArgs {
     const uint32_t *list;  // clumps of this launch, in key-rank order
@@ -227,37 +220,6 @@ struct RbShared {
     float *sf;           // acceptance state for every thread: hi[6], lo[6], Mf
     double *sd;          // acceptance state in FP64: x y z vx vy vz M
 };
-
-// room for n entries, half as many on top where the pool has them (cap: what was taken)
-__device__ __forceinline__ uint32_t rb_alloc(const Pool &P, uint32_t n, uint32_t &cap) {
-    cap = n + n / 2;
-    uint32_t o = cap > n ? pool_try_alloc(P, cap) : kNone;
-    if (o == kNone) {
-        cap = n;
-        o = pool_try_alloc(P, n);
-    }
-    return o;
-}
-
-// the segment a clump left last, or a new one in its place, with room for n entries
-__device__ __forceinline__ uint32_t rb_spare(const Pool &P, RbSeg &g, uint32_t n) {
-    if (g.spare_cap >= n) return g.spare;
-    uint32_t cap;
-    const uint32_t o = rb_alloc(P, n, cap);
-    if (o != kNone) {
-        g.spare = o;
-        g.spare_cap = cap;
-    }
-    return o;
-}
-
-// the members moved from the present segment at o to the spare one
-__device__ __forceinline__ void rb_switch(RbSeg &g, uint32_t o) {
-    const uint32_t cap = g.cap;
-    g.cap = g.spare_cap;
-    g.spare = o;
-    g.spare_cap = cap;
-}
 
 // ------------------------------------------------------------------ one SearchBound call
 // Returns the number of accepted particles, or kNone when the member pool is full (nothing
@@ -1124,17 +1086,7 @@ __device__ bool rb_sort_particles(const RbArgs &a, uint32_t slot, RbShared &sh, 
         // half of the pool), the sorted pairs in its spare segment
         if (tid == 0) {
             RbSeg &g = a.seg[slot];
-            s_r = rb_spare(a.P, g, m);
-            if (s_r != kNone && g.buf_cap < 2 * m + 1) {
-                uint32_t cap;
-                const uint32_t x = rb_alloc(a.P, 2 * m + 1, cap);
-                if (x == kNone) {
-                    s_r = kNone;
-                } else {
-                    g.buf = x;
-                    g.buf_cap = cap;
-                }
-            }
+            s_r = rb_sort_room(a.P, g, m) ? g.spare : kNone;
             s_x = g.buf;
         }
         __syncthreads();
