@@ -267,6 +267,10 @@ static void energy_tiles(int w[kEnergyClasses]) {
         for (int j = 0; j < kEnergyClasses; ++j) w[j] = v[j];
 }
 
+// A batch's workspace up to this size stays in the context. An allocation costs a batch of 16 small
+// groups some of its 110 us, one of this size (a million particles) far less of its own time.
+constexpr size_t kEnergyKept = 64u << 20;
+
 int group_energies(Context &c, const float *pos3, const float *vel3, const float *mass, const uint64_t *offsets, uint32_t ngroups, double G,
                    double shear_y, double *e_kin, double *e_pot, uint64_t *zero_pairs, cudaStream_t s) {
     if (ngroups == 0) return kOk;
@@ -292,7 +296,7 @@ int group_energies(Context &c, const float *pos3, const float *vel3, const float
         cbase[k + 1] = cbase[k] + iofs[k][glist[k].size()];
     }
     const uint64_t nitems = cbase[kEnergyClasses];
-    // One workspace, the context's scratch: the tables (and a small batch's particles) go up in one
+    // One workspace: the tables (and a small batch's particles) go up in one
     // copy, the results come back in one. Fifteen stream-ordered allocations and eight copies cost
     // a batch of 16 small groups two thirds of its 189 us.
     struct Layout {
@@ -310,8 +314,17 @@ int group_energies(Context &c, const float *pos3, const float *vel3, const float
     const size_t o_p3 = lay.take(12 * n), o_v3 = lay.take(12 * n), o_m = lay.take(4 * n), particles = lay.at;
     const size_t o_pm = lay.take(16 * n), o_v = lay.take(16 * n), o_part = lay.take(8 * nitems), o_com = lay.take(32ull * ngroups);
     const size_t o_ek = lay.take(8ull * ngroups), o_sum = lay.take(8ull * ngroups), o_zeros = lay.take(8), results = lay.at - o_ek;
-    if (c.ensure(c.scratch, lay.at)) return kErrOutOfMemory;
-    char *d = c.scratch.base;
+    // the context's scratch, which stays with it, for small batches and wherever it is large enough
+    // already; a larger batch gives its memory back
+    StreamBuf<char> own(s);
+    char *d;
+    if (lay.at <= std::max(kEnergyKept, c.scratch.cap)) {
+        if (c.ensure(c.scratch, lay.at)) return kErrOutOfMemory;
+        d = c.scratch.base;
+    } else {
+        PLAN_CUDA(own.alloc(lay.at));
+        d = own.p;
+    }
     const bool together = particles - tables <= (1u << 20);
     std::vector<char> up(together ? particles : tables, 0);
     std::memcpy(up.data() + o_off, offsets, (ngroups + 1) * 8ull);
