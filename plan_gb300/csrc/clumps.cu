@@ -559,13 +559,14 @@ __global__ void k_ball_clumps(int pass, uint32_t C, CT ct, KTree t, bool hill_mo
 }
 
 // The same search with a warp per clump over all nct clump points (in tree order, which is the
-// traversal's), for clump sets where that is the smaller work: a thread's FP64 walk of the clump
-// tree took 0.1 ms for 100 clumps, this 6 us (0.03 ms for 1,600, growing with the square of the
-// number; the walk's time grows with its logarithm). The ball holds the points within it, decided in FP32 unless too
-// close to its surface; there the point takes the walk's own way, the FP64 tests of the nodes
-// above it. (A point inside the ball by more than the rounding of its key lies in nodes that all
-// meet the ball, one outside by as much in none that it contains.)
-constexpr uint32_t kBruteClumps = 8192;
+// traversal's), for clump sets where that is the smaller work: it grows with the square of the
+// number, a thread's FP64 walk of the clump tree a little faster than the number itself. Measured,
+// brute force against the walk: 964 clumps 0.014 and 0.16 ms, 3,605 0.070 and 0.30, 7,914 0.24 and
+// 0.66, 18,919 1.15 and 1.2 to 1.5 ms; the line lies before they meet. The ball holds the points
+// within it, decided in FP32 unless too close to its surface; there the point takes the walk's own
+// way, the FP64 tests of the nodes above it. (A point inside the ball by more than the rounding of
+// its key lies in nodes that all meet the ball, one outside by as much in none that it contains.)
+constexpr uint32_t kBruteClumps = 16384;
 
 static __device__ __noinline__ bool ball_takes(const KTree &t, uint32_t q, double x, double y, double z, double r) {
     uint32_t n = t.leaf_of[q];
@@ -2153,6 +2154,13 @@ static double wall_ms() {
 
 // PLAN_TRACE=1 in the environment prints the progress of FindPlanetesimals to stderr (the
 // stream is synchronised at every mark, so traced runs are slower; off by default).
+// The largest clump set that a merge sweep searches by brute force: the measured limit, or
+// PLAN_BRUTE_CLUMPS.
+static uint32_t brute_clumps() {
+    const char *e = std::getenv("PLAN_BRUTE_CLUMPS");
+    return e && *e ? (uint32_t)std::strtoul(e, nullptr, 10) : kBruteClumps;
+}
+
 struct Trace {
     bool on = false, fine_on = false;  // PLAN_TRACE=1: stages; 2: also the steps inside a merge sweep
     cudaStream_t s = nullptr;
@@ -2185,6 +2193,7 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
     for (auto &e : ev) cudaEventCreate(&e);
     cudaEventRecord(ev[0], s);
     Trace trace(s);
+    const uint32_t max_brute = brute_clumps();
     c.counters[27] = 0;  // saddle queries of the merge sweeps left to the exact heap path (ties)
     const DevTree &tr = c.tree;
     const uint32_t Tu = tr.Tu, N = c.n_input;
@@ -2383,7 +2392,7 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
             // candidates
             uint32_t ncand = 0;
             if (nct) {
-                if (nct <= kBruteClumps)
+                if (nct <= max_brute)
                     k_ball_brute<<<(C + 3) / 4, 128, 0, s>>>(0, C, ct, kct, ftree_of(ctree), ctree.Tu, hill_mode, hillf,
                                                              max_radius, d_cnt, nullptr, nullptr);
                 else
@@ -2408,7 +2417,7 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
             PLAN_CUDA(cudaMemsetAsync(d_nrl, 0, 4, s));
             uint32_t nsaddle = 0;
             if (ncand) {
-                if (nct <= kBruteClumps)
+                if (nct <= max_brute)
                     k_ball_brute<<<(C + 3) / 4, 128, 0, s>>>(1, C, ct, kct, ftree_of(ctree), ctree.Tu, hill_mode, hillf,
                                                              max_radius, d_cnt, d_off, d_cand);
                 else
