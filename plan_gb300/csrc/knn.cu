@@ -359,8 +359,8 @@ __global__ void __launch_bounds__(32 * kWkWarps) k_exact_w(KTree t, FTree f, con
     }
 }
 
-// The same for a few queries that may visit 10^5 points (the Hill sweeps' saddles: tens of queries
-// from a Hill radius): a block per query. Its threads walk the tree a level at a time, listing the
+// The same for queries that may visit 10^5 points (the Hill sweeps' saddles: tens of queries from a
+// Hill radius): a block per query. Its threads walk the tree a level at a time, listing the
 // visited ranges; the points are shared out evenly over all warps, each with a buffer of its own
 // and the smallest bound any of them has found, and warp 0 merges what is left. Measured on 48 to
 // 72 such queries of 262,144 particles: 1.6 -> 0.15 ms per sweep against a warp per query. Queries
@@ -368,7 +368,10 @@ __global__ void __launch_bounds__(32 * kWkWarps) k_exact_w(KTree t, FTree f, con
 constexpr int kBkThreads = 256, kBkWarps = kBkThreads / 32;
 constexpr uint32_t kBkNodes = 4096, kBkRanges = 4096, kBkPart = 256;
 constexpr uint32_t kBkMaxK = 48;       // eight warps' bounds must fit the merged buffer
-constexpr uint32_t kBkQueries = 600;   // from here on the warps of the queries fill the GPU
+// Queries of one call from which on a warp takes each. Measured, a block and a warp per query: 236
+// queries 0.04 and 0.10 ms, 1,292 0.16 and 0.21, 5,460 0.64 and 0.76, 10,018 1.29 and 1.74, 15,634
+// 1.95 and 1.82 ms.
+constexpr uint32_t kBkQueries = 12000;
 
 struct BkShared {
     WkBuf merged;
