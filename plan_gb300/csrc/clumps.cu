@@ -36,6 +36,7 @@
 #include "sort.h"
 #include "ordered_sum.cuh"
 #include "tree_walk.cuh"
+#include "bound_f32.cuh"
 #include "unbind_f32.cuh"
 
 namespace plan {
@@ -917,8 +918,8 @@ __device__ __forceinline__ double div_by_rcp(double num, double den, double y) {
 constexpr int kFront = 2048;
 constexpr int kRebindThreads = 256;
 constexpr int kCopyTasks = 512;  // queued copies of contained runs in the fill step
-constexpr int kTile = 192;  // candidates staged per step of the acceptance: 64 + 52 + 4 + 1 B each
-static_assert(kTile * (64 + 52 + 4 + 1) <= kFront * (3 * 4 + 2), "the candidate tile must fit in the frontier space");
+constexpr int kTile = 192;  // candidates staged per step of the acceptance: position and velocity, CandF, index, flag
+static_assert(kTile * (64 + sizeof(CandF) + 4 + 1) <= kFront * (3 * 4 + 2), "the candidate tile must fit in the frontier space");
 
 __global__ void k_elig_flags(uint32_t Tu, const uint8_t *in_clump, const double *dens, double thr, uint32_t *flag) {
     uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1046,57 +1047,6 @@ __device__ __forceinline__ bool bound_fp64(const double4_32a p, const double4_32
     const double ex = (vx - 0.0 * dx) - v.x, ey = (vy - cp.shear * dx) - v.y, ez = (vz - 0.0 * dx) - v.z;
     const double e = +0.5 / M * norm2_3(ex, ey, ez) - cp.G / norm3(dx, y - p.y, z - p.z);
     return e < 0;
-}
-
-// The boundness test entirely in FP32 from hi/lo pairs of the state (sh, sl: x, y, z, vx,
-// vy, vz) and of the candidate: 1 bound, 0 not, -1 too close to call (then bound_fp64).
-// Differences of hi/lo pairs carry a relative error below 2^-23 (plus 2^-48 of the
-// coordinates from the splits); the y velocity term, a difference of two such values, carries
-// an absolute error below 2^-21 (|T1| + |T2|). With at most ten further FP32 roundings per
-// term, |A - A_exact| <= A 2^-20 + |ey| err_y / M and |B - B_exact| <= B 2^-20, inside the
-// margin below; the reference's own FP64 rounding is far smaller.
-__device__ __forceinline__ int bound_hilo(const CandF &c, float Mf, const float sh[6], const float sl[6], float G, float shear) {
-    const float dx = (sh[0] - c.ph[0]) + (sl[0] - c.pl[0]);
-    const float dy = (sh[1] - c.ph[1]) + (sl[1] - c.pl[1]);
-    const float dz = (sh[2] - c.ph[2]) + (sl[2] - c.pl[2]);
-    const float ex = (sh[3] - c.vh[0]) + (sl[3] - c.vl[0]);
-    const float t1 = (sh[4] - c.vh[1]) + (sl[4] - c.vl[1]), t2 = shear * dx;
-    const float ey = t1 - t2;
-    const float ez = (sh[5] - c.vh[2]) + (sl[5] - c.vl[2]);
-    const float K = ex * ex + ey * ey + ez * ez, D2 = dx * dx + dy * dy + dz * dz;
-    const float M = Mf + c.w;
-    if (!(K > 1e-30f && D2 > 1e-30f && K < 1e30f && D2 < 1e30f && M > 1e-30f && M < 1e30f)) return -1;
-    const float A = 0.5f / M * K, B = G / sqrtf(D2);
-    const float e = A - B;
-    const float margin = (fabsf(A) + fabsf(B)) * 3.814697265625e-06f                             // 2^-18
-                         + fabsf(ey) * (fabsf(t1) + fabsf(t2)) * 9.5367431640625e-07f / M;    // 2^-20 / M
-    if (e > margin) return 0;
-    if (e < -margin) return 1;
-    return -1;
-}
-
-// The same test with the FP32 quotient and square root taken by the fast intrinsics
-// (__fdividef, rsqrtf: at most 2 ulp each for the argument ranges admitted above). With
-// them A and B still carry a relative error below 2^-20, inside the margin.
-__device__ __forceinline__ int bound_hilo_fast(const CandF &c, float Mf, const float sh[6], const float sl[6], float G, float shear) {
-    const float dx = (sh[0] - c.ph[0]) + (sl[0] - c.pl[0]);
-    const float dy = (sh[1] - c.ph[1]) + (sl[1] - c.pl[1]);
-    const float dz = (sh[2] - c.ph[2]) + (sl[2] - c.pl[2]);
-    const float ex = (sh[3] - c.vh[0]) + (sl[3] - c.vl[0]);
-    const float t1 = (sh[4] - c.vh[1]) + (sl[4] - c.vl[1]), t2 = shear * dx;
-    const float ey = t1 - t2;
-    const float ez = (sh[5] - c.vh[2]) + (sl[5] - c.vl[2]);
-    const float K = ex * ex + ey * ey + ez * ez, D2 = dx * dx + dy * dy + dz * dz;
-    const float M = Mf + c.w;
-    if (!(K > 1e-30f && D2 > 1e-30f && K < 1e30f && D2 < 1e30f && M > 1e-30f && M < 1e30f)) return -1;
-    const float rM = __fdividef(1.0f, M);
-    const float A = 0.5f * rM * K, B = G * rsqrtf(D2);
-    const float e = A - B;
-    const float margin = (fabsf(A) + fabsf(B)) * 3.814697265625e-06f              // 2^-18
-                         + fabsf(ey) * (fabsf(t1) + fabsf(t2)) * 9.5367431640625e-07f * rM;  // 2^-20 / M
-    if (e > margin) return 0;
-    if (e < -margin) return 1;
-    return -1;
 }
 
 __device__ __forceinline__ void split_f(double d, float &hi, float &lo) {
@@ -1368,6 +1318,7 @@ __global__ void __launch_bounds__(kRebindThreads) k_rebind_round(const uint32_t 
             split_f(vv.y, cf.vh[1], cf.vl[1]);
             split_f(vv.z, cf.vh[2], cf.vl[2]);
             cf.w = (float)pp.w;
+            cand_limits(cf, shear32);
             tf[i] = cf;
         }
         __syncthreads();

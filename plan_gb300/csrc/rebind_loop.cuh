@@ -670,6 +670,7 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
             split_any(nv.z, cf.vh[2], cf.vl[2]);
             float wl;
             split_any(np.w, cf.w, wl);
+            cand_limits(cf, shear32);
         }
         uint32_t place;  // the candidates left, side by side in the tile
         const uint32_t tlen = rb_block_rank(!taken, place, sh.warp_tot);

@@ -23,7 +23,7 @@ struct UbShared {
     double upd[32 * 9];   // a window's removals: m x .. m vz, the masses before and after, 1 / after
     double hist[33 * 8];  // its states: x y z vx vy vz M, before it and after each removal
     double sd[8];         // the state
-    float sf[16];         // as float pairs: hi[6], lo[6]; M; the largest centre and velocity component squared
+    float sf[13];         // as float pairs: hi[6], lo[6]; M
     uint32_t first[kUb / 32];
     uint32_t at;
 };
@@ -43,17 +43,10 @@ __device__ __forceinline__ bool ub_exact(const double4_32a p, const double4_32a 
 }
 
 __device__ __forceinline__ void ub_floats(const double *S, float *sf) {
-    float big = 0.f, fast = 0.f;
 #pragma unroll
-    for (int c = 0; c < 6; ++c) {
-        split_any(S[c], sf[c], sf[6 + c]);
-        if (c < 3) big = fmaxf(big, fabsf(sf[c]));
-        else fast = fmaxf(fast, fabsf(sf[c]));
-    }
+    for (int c = 0; c < 6; ++c) split_any(S[c], sf[c], sf[6 + c]);
     float l;
     split_any(S[6], sf[12], l);
-    sf[13] = big * big;
-    sf[14] = fast * fast;
 }
 
 __global__ void __launch_bounds__(kUb) k_unbind(const uint32_t *list, CT ct, Pool P, const double4_32a *pos, const double4_32a *vel, FTree ft,
@@ -92,6 +85,7 @@ __global__ void __launch_bounds__(kUb) k_unbind(const uint32_t *list, CT ct, Poo
             split_any(v.z, cf.vh[2], cf.vl[2]);
             float l;
             split_any(p.w, cf.w, l);
+            cand_limits(cf, shear32);
             sh.pos[tid] = p;
             sh.vel[tid] = v;
             sh.f[tid] = cf;
@@ -184,7 +178,7 @@ __global__ void __launch_bounds__(kUb) k_unbind(const uint32_t *list, CT ct, Poo
                     bool unb = false;
                     const double *S = sh.hist + 8 * rank;
                     if (has && (uint32_t)lane < lim) {
-                        float sf[15];
+                        float sf[13];
                         ub_floats(S, sf);
                         const int r = ub_test(c, sf, G32, shear32);
                         unb = r < 0 ? ub_exact(sh.pos[k], sh.vel[k], S, cp) : r == 1;

@@ -71,19 +71,13 @@ int main() {
         const double ex = (c[3] - 0.0 * ddx) - v[0], ey = (c[4] - shear * ddx) - v[1], ez = (c[5] - 0.0 * ddx) - v[2];
         const double E = 0.5 / M * (ex * ex + ey * ey + ez * ez) -
                          G / std::sqrt(ddx * ddx + (c[1] - p[1]) * (c[1] - p[1]) + (c[2] - p[2]) * (c[2] - p[2]));
-        float sf[15], l;
-        float big = 0, fast = 0;
-        for (int k = 0; k < 6; ++k) {
-            split(S[k], sf[k], sf[6 + k]);
-            if (k < 3) big = std::fmax(big, std::fabs(sf[k]));
-            else fast = std::fmax(fast, std::fabs(sf[k]));
-        }
+        float sf[13], l;
+        for (int k = 0; k < 6; ++k) split(S[k], sf[k], sf[6 + k]);
         split(S[6], sf[12], l);
-        sf[13] = big * big;
-        sf[14] = fast * fast;
         CandF f;
         for (int d = 0; d < 3; ++d) { split(p[d], f.ph[d], f.pl[d]); split(v[d], f.vh[d], f.vl[d]); }
         split(m, f.w, l);
+        cand_limits(f, (float)shear);
         const int got = ub_test(f, sf, (float)G, (float)shear);
         ++n;
         light += left > 0.9;
