@@ -1,8 +1,8 @@
-// --Density_Vs_Scale on the GPU: every (cell centre, radius, sub-centre) query of
-// BasicAnalysesWithTree is one thread walking the particle tree with the reference's sheared
-// node tests (dvs.cuh, the same code the CPU tests run on the oracle's tree); the largest
-// count per radius is an atomic maximum, and queries that cannot reach it stop early. The host sets up the grid with the reference's own
-// arithmetic and turns the counts into densities.
+// --Density_Vs_Scale on the GPU: a warp takes a (cell centre, radius, sub-centre) query of
+// BasicAnalysesWithTree at a time and walks the particle tree with the reference's sheared node
+// tests in FP32, in FP64 where that cannot tell (dvs.cuh, the same code the CPU tests run); the
+// largest count per radius is an atomic maximum, and queries that cannot exceed it stop early. The
+// host sets up the grid with the reference's own arithmetic and turns the counts into densities.
 #include <algorithm>
 #include <cmath>
 #include <cstring>

@@ -49,8 +49,8 @@ struct DvsParams {
 // accumulated x += cell as its loops do). zlo, zhi: extreme z of the tree points. 0; -1 when
 // the grid gives more radii than kDvsMaxLevels; -2 when an axis would need more than 2^24
 // centres (coordinates far outside any box the parameters describe, where the reference's
-// loops would run for ever); -3 when the queries (one device thread each) would need more
-// than 2^31 - 1 blocks of 128.
+// loops would run for ever); -3 when there are more than (2^31 - 1) x 128 queries (3 x 10^11: hours
+// of device time).
 inline int dvs_setup(const DvsParams &p, double time, double zlo, double zhi, DvsGeom &g, std::vector<double> &xs, std::vector<double> &ys,
                      std::vector<double> &zs) {
     g = DvsGeom{};

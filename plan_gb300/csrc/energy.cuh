@@ -16,7 +16,7 @@
 
 namespace plan {
 
-constexpr int kPairTile = 128;  // the default tile width (and the widest but one)
+constexpr int kPairTile = 128;  // the tile width of the CPU replay
 
 // the size class of a group of n particles (host)
 inline int energy_class(uint64_t n) {
@@ -28,11 +28,12 @@ inline int energy_class(uint64_t n) {
 // a tile width the pass is built for
 inline bool energy_tile_ok(int w) { return w == 32 || w == 64 || w == 128 || w == 256; }
 
-// Tile (ti, tj), tj >= ti, of the upper triangle of a T x T tiling, with tiles numbered row
-// by row: row ti starts at ti T - ti (ti - 1) / 2.
+// The upper triangle one tile at a time, as the CPU tests replay a group against an FP64 sum (the
+// GPU pass takes strips of tiles, below): tile (ti, tj), tj >= ti, of a T x T tiling, with tiles
+// numbered row by row; row ti starts at ti T - ti (ti - 1) / 2.
 PLAN_EN_HD inline uint64_t tri_row_start(uint64_t T, uint64_t k) { return k * T - k * (k - 1) / 2; }
 
-// The tile queue over all groups: item_off[g] is the first queue item of group g, whose
+// The same over all groups: item_off[g] is the first queue item of group g, whose
 // n_g = offsets[g+1] - offsets[g] particles make T (T + 1) / 2 tiles of the upper triangle
 // (T = ceil(n_g / tile)); item_off[ngroups] is the number of items. -1 when the offsets
 // decrease.

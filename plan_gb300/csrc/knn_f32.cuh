@@ -12,9 +12,9 @@
 // a program's own positions) are held to 2^-48 relative, an absolute error below 1e-15 per
 // difference for |x| < 0.25; squared distances then err by at most 2*sqrt(3)*d*1e-15, which
 // 2^-17*d^2 + 1e-24 covers for every d. Larger coordinates scale the absolute terms (Tol).
-// When a comparison falls inside its bound the query is redone on the exact FP64 path, and
-// exact FP64 distances are computed for every candidate that could belong to the k
-// nearest; a tie at the k-boundary also sends the query to the exact heap path.
+// A node test inside its bound is decided in FP64. Where the order of two points matters and their
+// distances are too close, the FP64 distances of the candidates are sorted; a tie among the k
+// nearest or at their boundary sends the query to the exact heap path.
 #pragma once
 
 namespace plan {
