@@ -434,7 +434,7 @@ def run_gpu(args) -> None:
                 "roofline": roof, "roofline_density": roof_dens, "cpu_baseline": cpu, "clocks": clk, "gpu_launches": launches,
                 "snapshots_per_s": world * args.steps / (total / 1e3),
                 "latency_ms": {"p50": float(np.percentile(per, 50)), "p99": float(np.percentile(per, 99))},
-                "stage_ms": {"ingest_ghosts_keys": stage[0], "sort": stage[1], "sinks_tree": stage[2], "tree_tail": stage[3],
+                "stage_ms": {"ingest": stage[0], "ghosts": stage[1], "box_keys_sort": stage[2], "sinks_octree": stage[3],
                              "density": stage[4], "densest": stage[5], "hop": stage[6], "clump_stage": stage[7],
                              "catalogue": stage[8], "density_kernel": stage[20], "densest_kernel": stage[21],
                              "rebinding": stage[12], "rebinding_kernel": stage[19]},
