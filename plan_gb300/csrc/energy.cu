@@ -267,9 +267,10 @@ static void energy_tiles(int w[kEnergyClasses]) {
         for (int j = 0; j < kEnergyClasses; ++j) w[j] = v[j];
 }
 
-// A batch's workspace up to this size stays in the context. An allocation costs a batch of 16 small
-// groups some of its 110 us, one of this size (a million particles) far less of its own time.
-constexpr size_t kEnergyKept = 64u << 20;
+// A batch's workspace up to this size (17 million particles) stays in the context. An allocation of
+// its own makes the first pass of a batch of 15 million 0.6 ms longer (43.8 -> 44.4 ms; 4 ms where it
+// is the process's first) and the others no longer.
+constexpr size_t kEnergyKept = 1u << 30;
 
 int group_energies(Context &c, const float *pos3, const float *vel3, const float *mass, const uint64_t *offsets, uint32_t ngroups, double G,
                    double shear_y, double *e_kin, double *e_pot, uint64_t *zero_pairs, cudaStream_t s) {

@@ -1,7 +1,7 @@
 """What a batch of group energies leaves behind on the device.
 
-The workspace of a small batch stays with the context; a large batch gives its memory back when the
-call returns, with or without a tree in the context.
+The workspace of a batch of up to 1 GiB stays with the context; a larger one gives its memory back
+when the call returns.
 """
 from __future__ import annotations
 
@@ -26,11 +26,11 @@ def test_large_batch_gives_its_memory_back(built):
     p = built.params()
     built.lib().plan_params_derive(C.byref(p))
     f = built.Finder(0)
-    small, large = _batch(16, 100), _batch(40000, 200)
+    small, large = _batch(16, 100), _batch(130000, 200)
     want = f.group_energies(*small, p)
     torch.cuda.synchronize()
     free = torch.cuda.mem_get_info()[0]
-    first = f.group_energies(*large, p)  # 8 million particles: some 500 MB
+    first = f.group_energies(*large, p)  # 26 million particles: 1.6 GB
     torch.cuda.synchronize()
     assert torch.cuda.mem_get_info()[0] >= free - (64 << 20)
     for a, b in zip(f.group_energies(*large, p), first):
