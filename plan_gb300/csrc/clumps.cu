@@ -1318,7 +1318,6 @@ __global__ void __launch_bounds__(kRebindThreads) k_rebind_round(const uint32_t 
             split_f(vv.y, cf.vh[1], cf.vl[1]);
             split_f(vv.z, cf.vh[2], cf.vl[2]);
             cf.w = (float)pp.w;
-            cand_limits(cf, shear32);
             tf[i] = cf;
         }
         __syncthreads();
@@ -1341,7 +1340,7 @@ __global__ void __launch_bounds__(kRebindThreads) k_rebind_round(const uint32_t 
                 const bool tk = valid && ttaken[k - base] != 0;
                 bool tent = false;
                 if (valid && !tk) {
-                    const int r = bound_hilo(tf[k - base], Mf, sh, sl, G32, shear32);
+                    const int r = bound_hilo(tf[k - base], Mf, sh, sl, G32, shear32, bound_limits(tf[k - base], shear32));
                     tent = r >= 0 ? r == 1 : bound_fp64(tpos[k - base], tvel[k - base], M_, x_, y_, z_, vx_, vy_, vz_, cp);
                 }
                 const unsigned B = __ballot_sync(full, tent), V = __ballot_sync(full, valid);
@@ -1391,7 +1390,7 @@ __global__ void __launch_bounds__(kRebindThreads) k_rebind_round(const uint32_t 
                     float h[6], l[6];
                     split_f(s0, h[0], l[0]); split_f(s1, h[1], l[1]); split_f(s2, h[2], l[2]);
                     split_f(s3, h[3], l[3]); split_f(s4, h[4], l[4]); split_f(s5, h[5], l[5]);
-                    const int r = bound_hilo(tf[k - base], (float)Ms, h, l, G32, shear32);
+                    const int r = bound_hilo(tf[k - base], (float)Ms, h, l, G32, shear32, bound_limits(tf[k - base], shear32));
                     ver = r >= 0 ? r == 1 : bound_fp64(tpos[k - base], tvel[k - base], Ms, s0, s1, s2, s3, s4, s5, cp);
                 }
                 const unsigned Vb = __ballot_sync(full, ver);
@@ -1453,7 +1452,7 @@ __global__ void __launch_bounds__(kRebindThreads) k_rebind_round(const uint32_t 
                 double yk = 0;  // kSpec == 2: 1 / (M + m_k), taken while the lanes test
                 if (k < tend && !ttaken[k - base]) {
                     if (kSpec == 2) yk = 1.0 / (M_ + tpos[k - base].w);
-                    const int r = bound_hilo(tf[k - base], Mf, sh, sl, G32, shear32);
+                    const int r = bound_hilo(tf[k - base], Mf, sh, sl, G32, shear32, bound_limits(tf[k - base], shear32));
                     bound = r >= 0 ? r == 1 : bound_fp64(tpos[k - base], tvel[k - base], M_, x_, y_, z_, vx_, vy_, vz_, cp);
                 }
                 const unsigned b = __ballot_sync(0xffffffffu, bound);
@@ -2648,7 +2647,8 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
         if (!use_rounds) {
             k_node_slices<<<grid_for(kt.nodes, 256), 256, 0, s>>>(kt.nodes, kt.nbeg, kt.nend, epos, enode);
             c.launches++;
-            k_member_terms<<<grid_for(Tu, 256), 256, 0, s>>>(Tu, tr.pos, tr.vel, tm0, tm1);
+            PLAN_CUDA(cudaMemsetAsync(d_head + 1, 0, 4, s));
+            k_member_terms<<<grid_for(Tu, 256), 256, 0, s>>>(Tu, tr.pos, tr.vel, tm0, tm1, d_head + 1);
             c.launches++;
             PLAN_CUDA(cudaMemsetAsync(d_needsort, 0, nb, s));
             PLAN_CUDA(cudaMemsetAsync(d_distsq, 0, nb, s));
@@ -2758,6 +2758,8 @@ int find_planetesimals(Context &c, plan_params &p, cudaStream_t s, plan_catalogu
                 ra.E = E;
                 ra.enode = enode;
                 ra.seg = d_seg;
+                ra.xtop = (float)box_reach(tr.box) * 1.000001f;
+                ra.vtop = d_head + 1;
                 ra.owner = owner;
                 ra.rank_of = rank_of;
                 ra.slot_of_rank = slot_of_rank;

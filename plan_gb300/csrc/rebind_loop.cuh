@@ -111,16 +111,31 @@ struct RbArgs {
     uint32_t *dcall, *dfirst;  // per deferral record / per slot: the earliest call that made it
     Ckpt ck;               // ck.n null: no checkpoints
     RbSeg *seg;            // per slot, zero at the start of a launch
+    float xtop;            // the largest magnitude of a coordinate in the root box
+    const uint32_t *vtop;  // of a velocity component: its upper 32 bits
 };
 
 // per-point products for the member sums (src/tree.hpp:4436-4440: mass, pos * mass,
 // vel * mass, each component rounded once)
-__global__ void k_member_terms(uint32_t Tu, const double4_32a *pos, const double4_32a *vel, double4_32a *tm0, double4_32a *tm1) {
+// *vtop (zero before): the upper 32 bits of the largest velocity component's magnitude.
+__global__ void __launch_bounds__(256) k_member_terms(uint32_t Tu, const double4_32a *pos, const double4_32a *vel, double4_32a *tm0, double4_32a *tm1,
+                                                      uint32_t *vtop) {
+    __shared__ uint32_t s_top;
+    if (threadIdx.x == 0) s_top = 0;
+    __syncthreads();
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= Tu) return;
-    const double4_32a p = pos[q], v = vel[q];
-    tm0[q] = make_double4_32a(p.w, p.x * p.w, p.y * p.w, p.z * p.w);
-    tm1[q] = make_double4_32a(v.x * p.w, v.y * p.w, v.z * p.w, 0.0);
+    uint32_t top = 0;
+    if (q < Tu) {
+        const double4_32a p = pos[q], v = vel[q];
+        tm0[q] = make_double4_32a(p.w, p.x * p.w, p.y * p.w, p.z * p.w);
+        tm1[q] = make_double4_32a(v.x * p.w, v.y * p.w, v.z * p.w, 0.0);
+        top = max(max((uint32_t)(dbits(v.x) >> 32) & 0x7fffffffu, (uint32_t)(dbits(v.y) >> 32) & 0x7fffffffu),
+                  (uint32_t)(dbits(v.z) >> 32) & 0x7fffffffu);
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_top, top);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_top > *(volatile uint32_t *)vtop) atomicMax(vtop, s_top);
 }
 
 // (calls, so that no FP64 instruction is run under a predicate where it is not needed)
@@ -444,6 +459,8 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
     CandF *tf = reinterpret_cast<CandF *>(tq + kRB);
     uint32_t &s_pos = sh.u[8];
     const float G32 = (float)a.cp.G, shear32 = (float)a.cp.shear;
+    // no candidate's limits are beyond those of the largest coordinate and velocity
+    const BoundLimits limits = bound_limits(a.xtop, (float)dfrom((uint64_t)(*a.vtop + 1u) << 32), shear32);
     double comp = 0.0;      // warp 0, lane c < 6: component c of the state (x y z vx vy vz)
     double M = sh.st[0];    // warp 0: the mass
     uint32_t nacc = 0, rounds = 0;
@@ -473,7 +490,7 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
         }
     }
     // warp 0: candidate k against the state in FP32
-    auto test = [&](const CandF &cf) { return bound_hilo_fast(cf, sh.sf[12], sh.sf, sh.sf + 6, G32, shear32); };
+    auto test = [&](const CandF &cf) { return bound_hilo_fast(cf, sh.sf[12], sh.sf, sh.sf + 6, G32, shear32, limits); };
     // warp 0 takes the window of the tile's candidates from at on; returns where the next one
     // starts, and whether any candidate was bound (or too close to call) on entry
     auto window = [&](uint32_t at, uint32_t tlen, bool &any) -> uint32_t {
@@ -572,12 +589,12 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
             int r;
             if (few) {
                 const float *f = sh.histf + 14 * rank;
-                r = bound_hilo_fast(cf, f[6], f, f + 7, G32, shear32);
+                r = bound_hilo_fast(cf, f[6], f, f + 7, G32, shear32, limits);
             } else {
                 float h[6], l[6], mh, ml;
                 for (int c = 0; c < 6; ++c) split_any(S[c], h[c], l[c]);
                 split_any(S[6], mh, ml);
-                r = bound_hilo_fast(cf, mh, h, l, G32, shear32);
+                r = bound_hilo_fast(cf, mh, h, l, G32, shear32, limits);
             }
             bound = r == 1;
             unsure = r < 0;
@@ -670,7 +687,6 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
             split_any(nv.z, cf.vh[2], cf.vl[2]);
             float wl;
             split_any(np.w, cf.w, wl);
-            cand_limits(cf, shear32);
         }
         uint32_t place;  // the candidates left, side by side in the tile
         const uint32_t tlen = rb_block_rank(!taken, place, sh.warp_tot);
@@ -698,7 +714,7 @@ __device__ uint32_t rb_call(const RbArgs &a, uint32_t slot, uint32_t myrank, RbS
             ++rounds;
             bool bound = false, unsure = false;
             if ((uint32_t)tid < tlen && (uint32_t)tid >= pos) {
-                const int r = bound_hilo_fast(cf, sh.sf[12], sh.sf, sh.sf + 6, G32, shear32);
+                const int r = bound_hilo_fast(cf, sh.sf[12], sh.sf, sh.sf + 6, G32, shear32, limits);
                 if (r >= 0) bound = r == 1;
                 else unsure = true;
             }

@@ -35,14 +35,17 @@ inline KTree ktree_of(const DevTree &tr) {
     return t;
 }
 
-inline FTree ftree_of(const DevTree &tr) {
+// the largest magnitude of a coordinate in the box
+inline double box_reach(const TreeBox &b) {
     double reach = 0;
-    for (int d = 0; d < 3; ++d) {
-        const double c = tr.box.root_center[d] < 0 ? -tr.box.root_center[d] : tr.box.root_center[d];
-        if (c + tr.box.half_width > reach) reach = c + tr.box.half_width;
+    for (double c : b.root_center) {
+        const double r = (c < 0 ? -c : c) + b.half_width;
+        if (r > reach) reach = r;
     }
-    return FTree{tr.phi, tr.plo, tr.nhi, tr.nlo, tol_of(reach)};
+    return reach;
 }
+
+inline FTree ftree_of(const DevTree &tr) { return FTree{tr.phi, tr.plo, tr.nhi, tr.nlo, tol_of(box_reach(tr.box))}; }
 
 __device__ __forceinline__ bool node_contained(const double4_32a nc, double qx, double qy, double qz, double r) {
     double t = nc.w * kSqrt3;

@@ -18,7 +18,7 @@ constexpr int kUb = 256;
 
 struct UbShared {
     double4_32a pos[kUb], vel[kUb];  // pos.w: the mass
-    CandF f[kUb];
+    UbCand f[kUb];
     uint32_t idx[kUb];
     double upd[32 * 9];   // a window's removals: m x .. m vz, the masses before and after, 1 / after
     double hist[33 * 8];  // its states: x y z vx vy vz M, before it and after each removal
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(kUb) k_unbind(const uint32_t *list, CT ct, Poo
     // member i - k is the tile's entry k; member 0 is never tested
     for (int i = (int)m0 - 1; i >= 1; i -= kUb) {
         const int tlen = min(kUb, i);
-        CandF cf;
+        UbCand cf;
         if (tid < tlen) {
             const uint32_t q = P.idx[o + i - tid];
             const double4_32a p = pos[q], v = vel[q];
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kUb) k_unbind(const uint32_t *list, CT ct, Poo
             split_any(v.z, cf.vh[2], cf.vl[2]);
             float l;
             split_any(p.w, cf.w, l);
-            cand_limits(cf, shear32);
+            cf.lim = bound_limits(cf, shear32);
             sh.pos[tid] = p;
             sh.vel[tid] = v;
             sh.f[tid] = cf;
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(kUb) k_unbind(const uint32_t *list, CT ct, Poo
                 for (bool any = true; any && at < (uint32_t)tlen;) {
                     const uint32_t k = at + lane;
                     const bool has = k < (uint32_t)tlen;
-                    const CandF c = sh.f[has ? k : at];
+                    const UbCand c = sh.f[has ? k : at];
                     const unsigned U = __ballot_sync(full, has && ub_test(c, sh.sf, G32, shear32) != 0);
                     any = U != 0;
                     if (!any) {

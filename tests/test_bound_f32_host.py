@@ -74,9 +74,11 @@ int main() {
             split(v[d], f.vh[d], f.vl[d]);
         }
         split(m, f.w, l);
-        cand_limits(f, (float)shear);
-        for (int fast = 0; fast < 2; ++fast) {
-            const int got = fast ? bound_hilo_fast(f, Mf, sh, sl, (float)G, (float)shear) : bound_hilo(f, Mf, sh, sl, (float)G, (float)shear);
+        for (int way = 0; way < 3; ++way) {
+            // the candidate's own limits, and those of the whole box
+            const BoundLimits own = bound_limits(f, (float)shear), all = bound_limits((float)(1.4 * X), 2e-2f, (float)shear);
+            const int got = way == 0 ? bound_hilo(f, Mf, sh, sl, (float)G, (float)shear, own)
+                                     : bound_hilo_fast(f, Mf, sh, sl, (float)G, (float)shear, way == 1 ? own : all);
             ++n;
             if (got < 0) ++unsure;
             else if (got == (E < 0)) ++said[got];

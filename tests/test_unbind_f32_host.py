@@ -74,10 +74,10 @@ int main() {
         float sf[13], l;
         for (int k = 0; k < 6; ++k) split(S[k], sf[k], sf[6 + k]);
         split(S[6], sf[12], l);
-        CandF f;
+        UbCand f;
         for (int d = 0; d < 3; ++d) { split(p[d], f.ph[d], f.pl[d]); split(v[d], f.vh[d], f.vl[d]); }
         split(m, f.w, l);
-        cand_limits(f, (float)shear);
+        f.lim = bound_limits(f, (float)shear);
         const int got = ub_test(f, sf, (float)G, (float)shear);
         ++n;
         light += left > 0.9;
